@@ -239,8 +239,10 @@ def forward_helpers(src):
     qs = function(src, "__device__ __forceinline__ double qsat_qs(double t, double p,")
     qs = rep(qs, "double qsat_qs(", "double qsat_qs_f(")
     qs = rep(qs, "estblf(", "estblf_f(")
-    cd = function(src, "__device__ __noinline__ int conden(double p,")
-    cd = rep(cd, "int conden(", "int conden_f(")
+    cd = function(src, "__device__ __forceinline__ int conden(double p,")
+    cd = rep(cd, "__device__ __forceinline__ int conden(", "__device__ __noinline__ int conden_f(")
+    cd = rep(cd, "double& rv0, ", "")
+    cd = rep(cd, "    rv0 = rvls;\n", "")
     cd = rep(cd, "const double* __restrict__ tbl)\n{", "const double* __restrict__ tbl, double& t_sat)\n{")
     cd = rep(cd, "qsat_qs(", "qsat_qs_f(", 2)
     cd = rep(cd, "        th = temps / ex;\n", "        th = temps / ex;\n        t_sat = temps;\n")
@@ -254,7 +256,7 @@ def main():
     s = src[src.index("#pragma once"):]
     # the column code only: the FP64 kernels are replaced by the adjoint kernels
     s = s[: s.index("// ---- kernels ------")].rstrip() + "\n"
-    s = rep(s, '#include "uw_math.h"', '#include "uw_math.h"\n#include "uw_adj.h"')
+    s = rep(s, '#include "uw_math.h"', '#define UW_MATH_INLINE 1\n#include "uw_math.h"\n#include "uw_adj.h"\n\n#define UW_TAPE_ORDER 1')
     s = rep(s, '#include "uwshcu_common.cuh"', '#include "uwshcu_common.cuh"\n#include "uwshcu.h"')
     s = re.sub(r"\bdouble\b", "Ad", s)
     # tables and constants stay double
@@ -262,8 +264,15 @@ def main():
     s = s.replace("const Ad* __restrict__ tbl", "const double* __restrict__ tbl")
     s = s.replace("__shared__ Ad tbl[UW_TBL];", "__shared__ double tbl[UW_TBL];")
     # conden: the taped version with the implicit derivative, after the FP64 helpers
-    old = function(s, "__device__ __noinline__ int conden(Ad p,")
+    old = function(s, "__device__ __forceinline__ int conden(Ad p,")
     s = rep(s, old, forward_helpers(src) + CONDEN)
+    # called as it is: the fast mode's and the by-value wrappers are not used here
+    i0 = s.index("// The column code's saturation adjustment: one call")
+    s = s[:i0] + s[s.index("// roots (uwshcu.F90:4787-4829)", i0):]
+    i0 = s.index("// conden for the fast-FP64 precision mode")
+    s = s[:i0] + s[s.index("// roots (uwshcu.F90:4787-4829)", i0):]
+    s = rep(s, "#define CONDEN(...) conden_call<FAST>(__VA_ARGS__)",
+            "#define CONDEN(p, ex, thl, qt, th, qv, ql, qi, rv, tbl) conden(p, ex, thl, qt, th, qv, ql, qi, tbl)")
     # launch arguments of the adjoint kernels and the output-index table
     fields = "\n".join("#define UW_AO_%s %d" % (f, j) for j, f in enumerate(ADJ_OUT))
     s = s.replace("namespace {\n", "namespace {\n\n"

@@ -16,13 +16,10 @@ D = os.path.dirname(os.path.abspath(__file__)) + '/'
 marker = '// ------------------------------------------------------------------------------------------------\n// The column kernel.'
 cur = open(D + 'uwshcu_mixed_kernel.cuh').read()
 head = cur[:cur.index(marker)]
-# helper head fixes: warp-uniform early stop in the mixed conden, not inlined
+# helper head fix: warp-uniform early stop in the mixed conden
 old = '''        if (fabs(dT) < 1.e-9) break;'''
 if old in head:
     head = head.replace(old, '''        if (__all_sync(__activemask(), fabs(dT) < 1.e-9)) break;''')
-head = head.replace('__device__ __forceinline__ int conden(R p, R ex, R thl, R qt, R& th, R& qv, R& ql, R& qi,',
-                    '__device__ __noinline__ int conden(R p, R ex, R thl, R qt, R& th, R& qv, R& ql, R& qi,')
-
 src = open(D + 'uwshcu_fp64_kernel.cuh').read()
 b = src[src.index(marker):]
 # keep uw_column and the plain kernel only
@@ -33,7 +30,11 @@ b = b.replace('uwshcu_fp64_kernel', 'uwshcu_mixed_kernel')
 b = b.replace('uw_column<KP, NC, MODE, 0, ZW>(A, tbl, i, active, wl, wl_count);',
               'uw_column<KP, NC, MODE, 0>(A, tbl, i, active, wl, wl_count);')
 b = b.replace('template <int KP, int NC, int MODE, int ZW = 0>\n__global__', 'template <int KP, int NC, int MODE>\n__global__')
-b = b.replace('#define CONDEN(...) (FAST ? conden_fast(__VA_ARGS__) : conden(__VA_ARGS__))', '#define CONDEN(...) conden(__VA_ARGS__)')
+old = '#define CONDEN(...) conden_call<FAST>(__VA_ARGS__)'
+assert b.count(old) == 1
+# this kernel's conden has no FP32 saturation lookup to hand out (rv)
+b = b.replace('#define UW_QSAT_OF_CONDEN(t, p) rvj', '#define UW_QSAT_OF_CONDEN(t, p) qsat_qs(t, p, tbld, tblf)')
+b = b.replace(old, '#define CONDEN(p, ex, thl, qt, th, qv, ql, qi, rv, td, tf) conden_call(p, ex, thl, qt, th, qv, ql, qi, td, tf)')
 b = re.sub(r'\bdouble\b', 'R', b)
 lit = re.compile(r'(?<![\w.])((?:\d+\.\d*|\.\d+)(?:[eE][-+]?\d+)?|\d+[eE][-+]?\d+)(?![\w.f])')
 b = lit.sub(lambda m: m.group(1) + 'f', b)

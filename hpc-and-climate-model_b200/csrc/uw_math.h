@@ -21,8 +21,21 @@
 
 #if defined(__CUDACC__)
 #define UW_HD __host__ __device__ __forceinline__
+#define UW_HD_SLOW static __host__ __device__ __noinline__
 #else
 #define UW_HD static inline
+#define UW_HD_SLOW static
+#endif
+// exp, log, pow and erfc are calls on the device: inlined at each of their ~25 uses they made up 110 kB
+// of the 510 to 620 kB worklist kernels, which wait for their instructions (the step at 1,048,576
+// columns: 150 ms with calls against 158 ms inlined, loops not unrolled in both).
+// The adjoint's kernels (UW_MATH_INLINE) run few warps and wait on each one's chain: they keep them inlined.
+#if !defined(__CUDACC__)
+#define UW_HD_CALL static inline
+#elif defined(UW_MATH_INLINE)
+#define UW_HD_CALL UW_HD
+#else
+#define UW_HD_CALL UW_HD_SLOW
 #endif
 
 // Multiplications and additions that no compiler contracts into an fma: __dmul_rn/__dadd_rn on
@@ -73,11 +86,8 @@ UW_HD double uw_div_by(double a, double b, double y)
 // memory, 3.2 KB per block, they changed the FP64 kernels' time by under 1 % and slowed the adjoint's
 // one-warp blocks by 14 %, whose shared-memory carveout then leaves less L1 for their stacks.)
 #if defined(__CUDACC__)
-#define UW_HD_SLOW static __host__ __device__ __noinline__
 static __device__ const double uw_cr_expt_d[128] = UW_CR_EXPT_INIT;
 static __device__ const double uw_cr_logt_d[276] = UW_CR_LOGT_INIT;
-#else
-#define UW_HD_SLOW static
 #endif
 static const double uw_cr_expt_h[128] = UW_CR_EXPT_INIT;
 static const double uw_cr_logt_h[276] = UW_CR_LOGT_INIT;
@@ -229,7 +239,7 @@ UW_HD int uw_exp_fast(double xh, double xl, double err_rel, double* y)
     return 1;
 }
 
-UW_HD double uw_exp(double x)
+UW_HD_CALL double uw_exp(double x)
 {
     if (x != x) return x;
     if (x > 709.8) return HUGE_VAL;
@@ -339,7 +349,7 @@ UW_HD void uw_log_fast(double x, double* H, double* L)
     uw_fast_two_sum(s3, lo, H, L);
 }
 
-UW_HD double uw_log(double x)
+UW_HD_CALL double uw_log(double x)
 {
     if (!(x > 0.0)) {
         if (x == 0.0) return -HUGE_VAL;
@@ -362,7 +372,7 @@ UW_HD_SLOW double uw_pow_accurate(double x, double y)
 }
 
 // pow(x, y) for x >= 0: exp(y log x) with log and the product in double-double.
-UW_HD double uw_pow(double x, double y)
+UW_HD_CALL double uw_pow(double x, double y)
 {
     if (x != x || y != y) return x + y;
     if (y == 0.0) return 1.0;
@@ -388,7 +398,7 @@ UW_HD double uw_pow(double x, double y)
 #endif
 
 // erfc(x), Cody's CALERF with jint = 1.
-UW_HD double uw_erfc(double x)
+UW_HD_CALL double uw_erfc(double x)
 {
     const double A[5] = {3.16112374387056560e00, 1.13864154151050156e02, 3.77485237685302021e02,
                          3.20937758913846947e03, 1.85777706184603153e-1};

@@ -103,6 +103,7 @@ struct UwConst {
     double tmin, tmax, ttrice, epsqs, rgasv, hlatf, hlatv, cpws, tmelt;
     double pcf[6];
     double omeps, trinv;   // 1 - epsqs and 1/ttrice, as vqsatd computes them on every call
+    double findsp_c3;      // rair (7.5 log 10) / cpws of findsp (uwshcu.F90:5164-5454)
     int icephs;
     // constituents
     int ncnst, ixnumliq, ixnumice;

@@ -992,6 +992,7 @@ int uwshcu_init(double xlv, double cp, double xlf, double zvir, double r, double
     k.pcf[5] = 0.0;
     k.omeps = 1.0 - k.epsqs;
     k.trinv = (ttrice != 0.0) ? 1.0 / ttrice : 0.0;
+    k.findsp_c3 = 287.04 * (7.5 * uw_log(10.0)) / k.cpws;
     k.ncnst = ncnst;
     k.ixnumliq = ixnumliq;
     k.ixnumice = ixnumice;

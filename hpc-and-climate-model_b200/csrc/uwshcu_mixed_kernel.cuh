@@ -28,6 +28,8 @@ __constant__ double c_estbl[UW_TBL];
 
 typedef float R;
 
+#define UW_TAPE_ORDER 0   // the adjoint kernel's order of operations (the FP64 kernel's header)
+
 #define MX(a, b) ((a) > (b) ? (a) : (b))
 #define MN(a, b) ((a) < (b) ? (a) : (b))
 
@@ -117,7 +119,7 @@ __device__ __forceinline__ void qsat3_d(double t, double p, double& es, double& 
 __device__ __forceinline__ float exnf(float p) { return powf(p / (float)c.p00, (float)c.rovcp); }
 
 // conden (uwshcu.F90:4718-4785): FP64 saturation adjustment from FP32 (p, exner, thl, qt).
-__device__ __noinline__ int conden(R p, R ex, R thl, R qt, R& th, R& qv, R& ql, R& qi,
+__device__ __forceinline__ int conden(R p, R ex, R thl, R qt, R& th, R& qv, R& ql, R& qi,
                                       const double* __restrict__ tbld, const float* __restrict__ tblf)
 {
     (void)tblf;
@@ -158,6 +160,28 @@ __device__ __noinline__ int conden(R p, R ex, R thl, R qt, R& th, R& qv, R& ql, 
     qi = (R)(nu * qc);
     th = (R)(temps / (double)ex);
     return (fabs((temps - (leff / c.cp) * qc) - tc) >= 1.0) ? 1 : 0;
+}
+
+// One call for the column code's ~20 sites, results by value in registers.
+struct CondenOut {
+    R th, qv, ql, qi;
+    int id;
+};
+__device__ __noinline__ CondenOut conden_out(R p, R ex, R thl, R qt, const double* __restrict__ tbld, const float* __restrict__ tblf)
+{
+    CondenOut r;
+    r.id = conden(p, ex, thl, qt, r.th, r.qv, r.ql, r.qi, tbld, tblf);
+    return r;
+}
+__device__ __forceinline__ int conden_call(R p, R ex, R thl, R qt, R& th, R& qv, R& ql, R& qi,
+                                           const double* __restrict__ tbld, const float* __restrict__ tblf)
+{
+    const CondenOut r = conden_out(p, ex, thl, qt, tbld, tblf);
+    th = r.th;
+    qv = r.qv;
+    ql = r.ql;
+    qi = r.qi;
+    return r.id;
 }
 
 // roots (uwshcu.F90:4787-4829), FP64.
@@ -454,7 +478,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                                           const bool active, int* __restrict__ wl, int* __restrict__ wl_count)
 {
     const int i = (MODE == UW_MODE_RESUME && active) ? A.hand->col[i_in] : i_in;
-#define CONDEN(...) conden(__VA_ARGS__)
+    // Code size bounds the worklist passes: with the loops unrolled by the compiler and exp, log and pow
+    // inlined at each use their kernels were 833 kB (LIST1) and 631 kB (RESUME), far beyond the
+    // instruction caches that 16 warps at different places share, and at full occupancy a warp waited 4.4f
+    // to 6.5f cycles per instruction for its next one.  So no loop here is unrolled and the
+    // transcendentals are calls.
+#define CONDEN(p, ex, thl, qt, th, qv, ql, qi, rv, td, tf) conden_call(p, ex, thl, qt, th, qv, ql, qi, td, tf)
+// qsat_qs(t, p) right after a CONDEN call at that temperature and pressure: its first lookup
+#define UW_QSAT_OF_CONDEN(t, p) qsat_qs(t, p, tbld, tblf)
     bool cand = false;
     // lanes of this warp that run a column; UW_SYNC() joins them where every one of them arrives
     const unsigned live = __ballot_sync(0xffffffffu, active);
@@ -486,7 +517,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 // (uwshcu.F90:1945-1990 and :4383-4433)
 #define PUT_DIAG_LEVEL()                                                                                  \
     if (A.diag_level) {                                                                                   \
-        for (int k = 0; k <= mkx; k++) {                                                                  \
+        _Pragma("unroll 1") for (int k = 0; k <= mkx; k++) {                                              \
             DLV(UW_DL_UFRC, k) = ufrc[k];                                                                 \
             DLV(UW_DL_QTU, k) = qtu[k];                                                                   \
             DLV(UW_DL_THLU, k) = thlu[k];                                                                 \
@@ -497,8 +528,8 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             DLV(UW_DL_FLXRAIN, k) = flxrain[k];                                                           \
             DLV(UW_DL_FLXSNOW, k) = flxsnow[k];                                                           \
         }                                                                                                 \
-        for (int j = UW_DL_FER; j < UW_NDL; j++) DLV(j, 0) = 0.0f;                                         \
-        for (int k = 1; k <= mkx; k++) {                                                                  \
+        _Pragma("unroll 1") for (int j = UW_DL_FER; j < UW_NDL; j++) DLV(j, 0) = 0.0f;                     \
+        _Pragma("unroll 1") for (int k = 1; k <= mkx; k++) {                                              \
             DLV(UW_DL_FER, k) = fer[k];                                                                   \
             DLV(UW_DL_FDR, k) = fdr[k];                                                                   \
             DLV(UW_DL_DWTEN, k) = dwten[k];                                                               \
@@ -521,6 +552,9 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     R qlten[KP], qiten[KP], qvten[KP], sten[KP], qc[KP], qc_l[KP], qc_i[KP], evapc[KP];
     R flxrain[KP], flxsnow[KP], cufrc[KP], qcu[KP], qlu[KP], qiu[KP], trten[NC][KP];
     R qw0[KP], trflx_d[KP], trflx_u[KP];
+#if !UW_TAPE_ORDER
+    R qltop[KP], qitop[KP];
+#endif
     R trsrc[NC], tre[NC];
 
     unsigned int errbits = 0;
@@ -545,7 +579,8 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     R thlu_top = 0, qtu_top = 0, exntop = 1.0f, drage = 0, bogbot = 0, bogtop = 0, rho0j = 0,
            wtwb = 0, wtw = 0;
     double xs1 = 0, xs2 = 0, xc1 = 0, xc2 = 0;
-    R thj = 0, qvj = 0, qlj = 0, qij = 0;
+    R thj = 0, qvj = 0, qlj = 0, qij = 0, rvj = 0;
+    (void)rvj;
     Kahan rainflx, snowflx;
     (void)kinv_o_d;
     const R pblh = __ldg(&A.pblh[i]);
@@ -556,6 +591,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 
     // ---- output initialisation (uwshcu.F90:1087-1124) ------------------------------------------
     if (MODE != UW_MODE_TRIGGER) {
+#pragma unroll 1
     for (int k = 0; k <= mkx; k++) {
         OI(umf, k) = 0.0f;
         OI(slflx, k) = 0.0f;
@@ -564,11 +600,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         OI(flxsnow1, k) = 0.0f;
         OI(wu, k) = 0.0f;
     }
+#pragma unroll 1
     for (int k = 1; k <= mkx; k++) {
         OL(qvten, k) = 0.0f; OL(qlten, k) = 0.0f; OL(qiten, k) = 0.0f; OL(sten, k) = 0.0f;
         OL(uten, k) = 0.0f; OL(vten, k) = 0.0f; OL(qrten, k) = 0.0f; OL(qsten, k) = 0.0f;
         OL(evapc, k) = 0.0f; OL(cufrc, k) = 0.0f; OL(qcu, k) = 0.0f; OL(qlu, k) = 0.0f;
         OL(qiu, k) = 0.0f; OL(qc, k) = 0.0f;
+#pragma unroll 1
         for (int m = 1; m <= ncnst; m++) OT(m, k) = 0.0f;
     }
     A.precip[i] = 0.0f;
@@ -586,12 +624,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     // only that status bit (no findsp at or above the bad level, no conden).  The values are checked
     // as they are loaded; z0 and tke, which the scheme reads later and only at some levels, once here.
     bool nonfinite = !uw_isfinite(pblh) || !uw_isfinite(A.cush[i]);
+#pragma unroll 1
     for (int k = 0; k <= mkx; k++) {
         ps0[k] = GI(ps0, k);
         zs0[k] = GI(zs0, k);
         nonfinite |= !uw_isfinite(ps0[k]) || !uw_isfinite(zs0[k]) || !uw_isfinite(GI(tke, k));
         exns0[k] = powf(ps0[k] / p00, rovcp);
     }
+#pragma unroll 1
     for (int k = 1; k <= mkx; k++) {
         p0[k] = GL(p0, k);
         dp0[k] = GL(dp0, k);
@@ -612,17 +652,21 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         R tmpf[KP];
         slope<KP>(mkx, thl0, p0, ssthl0);
         slope<KP>(mkx, qt0, p0, ssqt0);
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             tmpf[k] = GL(u0, k);
             nonfinite |= !uw_isfinite(tmpf[k]);
         }
         slope<KP>(mkx, tmpf, p0, ssu0);
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             tmpf[k] = GL(v0, k);
             nonfinite |= !uw_isfinite(tmpf[k]);
         }
         slope<KP>(mkx, tmpf, p0, ssv0);
+#pragma unroll 1
         for (int m = 1; m <= ncnst; m++) {
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {
                 tmpf[k] = GT(m, k);
                 nonfinite |= !uw_isfinite(tmpf[k]);
@@ -637,10 +681,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         stop = true;
     }
     // thv0 at layer bottom/top (:1275-1299)
+#pragma unroll 1
     for (int k = 1; k <= mkx && !nonfinite; k++) {
         R thl0bot = thl0[k] + ssthl0[k] * (ps0[k - 1] - p0[k]);
         R qt0bot = qt0[k] + ssqt0[k] * (ps0[k - 1] - p0[k]);
-        if (CONDEN(ps0[k - 1], exns0[k - 1], thl0bot, qt0bot, thj, qvj, qlj, qij, tbld, tblf)) {
+        if (CONDEN(ps0[k - 1], exns0[k - 1], thl0bot, qt0bot, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
             xflags |= UW_X_CONDEN;
             id_exit = true;
             stop = true;
@@ -650,7 +695,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         thvl0bot[k] = thl0bot * (1.0f + zvir * qt0bot);
         R thl0top = thl0[k] + ssthl0[k] * (ps0[k] - p0[k]);
         R qt0top = qt0[k] + ssqt0[k] * (ps0[k] - p0[k]);
-        if (CONDEN(ps0[k], exns0[k], thl0top, qt0top, thj, qvj, qlj, qij, tbld, tblf)) {
+        if (CONDEN(ps0[k], exns0[k], thl0top, qt0top, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
             xflags |= UW_X_CONDEN;
             id_exit = true;
             stop = true;
@@ -665,16 +710,19 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     }
     if (!stop) {
     // per-column initialisation (:1333-1408)
+#pragma unroll 1
     for (int k = 0; k <= mkx; k++) {
         umf[k] = 0.0f; emf[k] = 0.0f; slflx[k] = 0.0f; qtflx[k] = 0.0f; uflx[k] = 0.0f; vflx[k] = 0.0f;
         ufrc[k] = 0.0f; thlu[k] = 0.0f; qtu[k] = 0.0f; uu[k] = 0.0f; vu[k] = 0.0f; wu[k] = 0.0f;
         thvu[k] = 0.0f; thlu_emf[k] = 0.0f; qtu_emf[k] = 0.0f; uu_emf[k] = 0.0f; vu_emf[k] = 0.0f;
+#pragma unroll 1
         for (int m = 0; m < ncnst; m++) {
             trflx[m][k] = 0.0f;
             tru[m][k] = 0.0f;
             tru_emf[m][k] = 0.0f;
         }
     }
+#pragma unroll 1
     for (int k = 1; k <= mkx; k++) {
         qvten[k] = 0.0f; qlten[k] = 0.0f; qiten[k] = 0.0f; sten[k] = 0.0f; uten[k] = 0.0f; vten[k] = 0.0f;
         qrten[k] = 0.0f; qsten[k] = 0.0f; dwten[k] = 0.0f; diten[k] = 0.0f; evapc[k] = 0.0f;
@@ -682,6 +730,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         qc[k] = 0.0f; qc_l[k] = 0.0f; qc_i[k] = 0.0f; qtten[k] = 0.0f; slten[k] = 0.0f;
         qlten_sink[k] = 0.0f; qiten_sink[k] = 0.0f; nlten_sink[k] = 0.0f; niten_sink[k] = 0.0f;
         rei[k] = 0.0f; uf[k] = 0.0f; vf[k] = 0.0f;
+#pragma unroll 1
         for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0f;
     }
     cnt = (R)mkx;
@@ -692,25 +741,32 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         // and the arrays that the set-up and that branch's restore build from the inputs, rebuilt
         // with the same operations
         UW_LOAD_STATE(A.hand->state + i_in, (size_t)A.hand->cap, tscaleh_r);
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             ps0[k] = GI(ps0, k);
             zs0[k] = GI(zs0, k);
         }
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             p0[k] = GL(p0, k);
             dp0[k] = GL(dp0, k);
         }
         {
             R tmpf[KP];
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) tmpf[k] = GL(u0, k);
             slope<KP>(mkx, tmpf, p0, ssu0);
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) tmpf[k] = GL(v0, k);
             slope<KP>(mkx, tmpf, p0, ssv0);
+#pragma unroll 1
             for (int m = 1; m <= ncnst; m++) {
+#pragma unroll 1
                 for (int k = 1; k <= mkx; k++) tmpf[k] = GT(m, k);
                 slope<KP>(mkx, tmpf, p0, sstr0[m - 1]);
             }
         }
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             qv0[k] = GL(qv0, k);
             ql0[k] = GL(ql0, k);
@@ -726,23 +782,27 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         }
         slope<KP>(mkx, thl0, p0, ssthl0);
         slope<KP>(mkx, qt0, p0, ssqt0);
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             umf[k] = 0.0f; emf[k] = 0.0f; slflx[k] = 0.0f; qtflx[k] = 0.0f; uflx[k] = 0.0f;
             vflx[k] = 0.0f; ufrc[k] = 0.0f; thlu[k] = 0.0f; qtu[k] = 0.0f; uu[k] = 0.0f;
             vu[k] = 0.0f; wu[k] = 0.0f; thvu[k] = 0.0f; thlu_emf[k] = 0.0f; qtu_emf[k] = 0.0f;
             uu_emf[k] = 0.0f; vu_emf[k] = 0.0f;
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++) {
                 trflx[m][k] = 0.0f;
                 tru[m][k] = 0.0f;
                 tru_emf[m][k] = 0.0f;
             }
         }
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             qvten[k] = 0.0f; qlten[k] = 0.0f; qiten[k] = 0.0f; sten[k] = 0.0f; uten[k] = 0.0f;
             vten[k] = 0.0f; qrten[k] = 0.0f; qsten[k] = 0.0f; dwten[k] = 0.0f; diten[k] = 0.0f;
             evapc[k] = 0.0f; cufrc[k] = 0.0f; qcu[k] = 0.0f; qlu[k] = 0.0f; qiu[k] = 0.0f;
             fer[k] = 0.0f; fdr[k] = 0.0f; qc[k] = 0.0f; qc_l[k] = 0.0f; qc_i[k] = 0.0f;
             qtten[k] = 0.0f; slten[k] = 0.0f;
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0f;
         }
     }
@@ -757,6 +817,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     // sections.  (Lanes that leave a loop at different iterations otherwise run apart for the rest
     // of the column: the worklist kernel ran with 1.9f of 32 lanes active.)  Loops marked `uniform`
     // have the same trip count on every live lane; UW_SYNC() appears only directly inside them.
+#pragma unroll 1
     for (int iter = (MODE == UW_MODE_RESUME ? 2 : 1); iter <= (MODE == UW_MODE_TRIGGER ? 1 : 2); iter++) {   // uniform
         R tscaleh = tscaleh_r;
         if constexpr (MODE != UW_MODE_RESUME) {   // uniform
@@ -768,6 +829,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         kinv = 1;
         {
             bool found = false;
+#pragma unroll 1
             for (int k = mkx - 1; k >= 1; k--) {
                 if (!found && (pblh + 5.0f - zs0[k]) * (pblh + 5.0f - zs0[k + 1]) < 0.0f) {
                     kinv = k + 1;
@@ -785,6 +847,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         {
             Kahan dpsum, tksum;
             thvlmin = 1000.0f;
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 if (k > kinv - 1) continue;
                 R dpi;
@@ -803,6 +866,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         thlsrc = thvlsrc / (1.0f + zvir * qtsrc);
         usrc = GL(u0, kinv - 1) + ssu0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
         vsrc = GL(v0, kinv - 1) + ssv0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
+#pragma unroll 1
         for (int m = 1; m <= ncnst; m++) trsrc[m - 1] = GT(m, 1);
         } while (0);
         UW_SYNC();
@@ -812,6 +876,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         klcl = mkx;
         {
             bool found = false;
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 if (!found && ps0[k] < plcl) {
                     klcl = k;
@@ -830,7 +895,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         {
             R thl0lcl = thl0[klcl] + ssthl0[klcl] * (plcl - p0[klcl]);
             R qt0lcl = qt0[klcl] + ssqt0[klcl] * (plcl - p0[klcl]);
-            if (CONDEN(plcl, exlcl, thl0lcl, qt0lcl, thj, qvj, qlj, qij, tbld, tblf)) {
+            if (CONDEN(plcl, exlcl, thl0lcl, qt0lcl, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                 xflags |= UW_X_CONDEN;
                 id_exit = true;
                 stop = true;
@@ -855,6 +920,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             const bool lcl_above = (klcl >= kinv);
             R thvubot = 0.0f, thvutop = 0.0f;
             bool ldone = stop;
+#pragma unroll 1
             for (int k = 2; k <= mkx - 1; k++) {   // uniform (kinv >= 2)
                 if (!ldone && k >= kinv) do {
                     if (lcl_above && k < klcl) {
@@ -864,7 +930,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                         break;
                     }
                     if (!lcl_above && k == kinv) {
-                        if (CONDEN(ps0[k - 1], exns0[k - 1], thlsrc, qtsrc, thj, qvj, qlj, qij, tbld, tblf)) {
+                        if (CONDEN(ps0[k - 1], exns0[k - 1], thlsrc, qtsrc, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                             xflags |= UW_X_CONDEN;
                             id_exit = true;
                             stop = true;
@@ -884,7 +950,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     } else {
                         thvubot = thvutop;
                     }
-                    if (CONDEN(ps0[k], exns0[k], thlsrc, qtsrc, thj, qvj, qlj, qij, tbld, tblf)) {
+                    if (CONDEN(ps0[k], exns0[k], thlsrc, qtsrc, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                         xflags |= UW_X_CONDEN;
                         id_exit = true;
                         stop = true;
@@ -920,6 +986,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             kinv_o = kinv; klcl_o = klcl; klfc_o = klfc; plcl_o = plcl; plfc_o = plfc;
             tkeavg_o = tkeavg; thvlmin_o = thvlmin; qtsrc_o = qtsrc; thvlsrc_o = thvlsrc;
             thlsrc_o = thlsrc; usrc_o = usrc; vsrc_o = vsrc; thv0lcl_o = thv0lcl;
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++) trsrc_o[m] = trsrc[m];
         } else {
             double del_CIN = cin - cin_i;
@@ -931,8 +998,10 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 kinv = kinv_o; klcl = klcl_o; klfc = klfc_o; plcl = plcl_o; plfc = plfc_o;
                 tkeavg = tkeavg_o; thvlmin = thvlmin_o; qtsrc = qtsrc_o; thvlsrc = thvlsrc_o;
                 thlsrc = thlsrc_o; usrc = usrc_o; vsrc = vsrc_o; thv0lcl = thv0lcl_o;
+#pragma unroll 1
                 for (int m = 0; m < ncnst; m++) trsrc[m] = trsrc_o[m];
                 exlcl = exnf(plcl);
+#pragma unroll 1
                 for (int k = 1; k <= mkx; k++) {
                     qv0[k] = GL(qv0, k);
                     ql0[k] = GL(ql0, k);
@@ -948,23 +1017,27 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 }
                 slope<KP>(mkx, thl0, p0, ssthl0);
                 slope<KP>(mkx, qt0, p0, ssqt0);
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) {
                     umf[k] = 0.0f; emf[k] = 0.0f; slflx[k] = 0.0f; qtflx[k] = 0.0f; uflx[k] = 0.0f;
                     vflx[k] = 0.0f; ufrc[k] = 0.0f; thlu[k] = 0.0f; qtu[k] = 0.0f; uu[k] = 0.0f;
                     vu[k] = 0.0f; wu[k] = 0.0f; thvu[k] = 0.0f; thlu_emf[k] = 0.0f; qtu_emf[k] = 0.0f;
                     uu_emf[k] = 0.0f; vu_emf[k] = 0.0f;
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++) {
                         trflx[m][k] = 0.0f;
                         tru[m][k] = 0.0f;
                         tru_emf[m][k] = 0.0f;
                     }
                 }
+#pragma unroll 1
                 for (int k = 1; k <= mkx; k++) {
                     qvten[k] = 0.0f; qlten[k] = 0.0f; qiten[k] = 0.0f; sten[k] = 0.0f; uten[k] = 0.0f;
                     vten[k] = 0.0f; qrten[k] = 0.0f; qsten[k] = 0.0f; dwten[k] = 0.0f; diten[k] = 0.0f;
                     evapc[k] = 0.0f; cufrc[k] = 0.0f; qcu[k] = 0.0f; qlu[k] = 0.0f; qiu[k] = 0.0f;
                     fer[k] = 0.0f; fdr[k] = 0.0f; qc[k] = 0.0f; qc_l[k] = 0.0f; qc_i[k] = 0.0f;
                     qtten[k] = 0.0f; slten[k] = 0.0f;
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0f;
                 }
                 precip = 0.0f; snow = 0.0f; rliq.reset(); cbmf = 0.0f;
@@ -973,6 +1046,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 // explicit CIN: the iteration-1 outputs already sit in the output slots (:1891-2011);
                 // flxprc1/flxsnow1 keep their initial zeros on this path, wu_out gets wu.
                 lflags |= UW_L_DELCIN;
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) OI(wu, k) = wu[k];
                 if (A.diag_real) {
                     A.diag_real[UW_DR_CIN * (size_t)mix + i] = cin_s;
@@ -1084,6 +1158,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             break;
             }
             ufrc[krel - 1] = ufrclcl;
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 if (k < kinv - 1 || k > krel - 1) continue;
                 umf[k] = cbmf;
@@ -1100,6 +1175,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         }
         UW_SYNC();
         if (MODE != UW_MODE_TRIGGER) {   // uniform
+#if !UW_TAPE_ORDER
+        // Condensate of the final updraft at the release level, at the interfaces above it (qltop, qitop)
+        // and at the cumulus top; id_top: the adjustment at the top did not close.  The tendencies and
+        // the in-cloud diagnostics need it again; the Fortran repeats the conden calls there, with the
+        // same arguments.
+        R ql_rel = 0.0f, qi_rel = 0.0f, ql_top = 0.0f, qi_top = 0.0f;
+        bool id_top = false;
+#endif
         // updraft at the release level (:2205-2236)
         if (!stop) do {
         emf[krel - 1] = 0.0f;
@@ -1107,19 +1190,24 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         wu[krel - 1] = wlcl;
         thlu[krel - 1] = thlsrc;
         qtu[krel - 1] = qtsrc;
-        if (CONDEN(prel, exprel, thlsrc, qtsrc, thj, qvj, qlj, qij, tbld, tblf)) {
+        if (CONDEN(prel, exprel, thlsrc, qtsrc, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
             xflags |= UW_X_CONDEN;
             id_exit = true;
             stop = true;
             break;
         }
         thvu[krel - 1] = thj * (1.0f + zvir * qvj - qlj - qij);
+#if !UW_TAPE_ORDER
+        ql_rel = qlj;
+        qi_rel = qij;
+#endif
         {
             R uplus = 0.0f, vplus = 0.0f;
             if (krel == kinv) {
                 uplus = PGFc * ssu0[kinv] * (prel - ps0[kinv - 1]);
                 vplus = PGFc * ssv0[kinv] * (prel - ps0[kinv - 1]);
             } else {
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) {
                     if (k < kinv || k > MX(krel - 1, kinv)) continue;
                     uplus = uplus + PGFc * ssu0[k] * (ps0[k] - ps0[k - 1]);
@@ -1131,6 +1219,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             uu[krel - 1] = usrc + uplus;
             vu[krel - 1] = vsrc + vplus;
         }
+#pragma unroll 1
         for (int m = 0; m < ncnst; m++) tru[m][krel - 1] = trsrc[m];
         } while (0);
         UW_SYNC();
@@ -1139,8 +1228,18 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             R scaleh = tscaleh;
             if (tscaleh < 0.0f) scaleh = 1000.0f;
             // ---- buoyancy-sorting updraft, iter_scaleh loop (:2306-2952) ----------------------
+#pragma unroll 1
             for (int iter_scaleh = 1; iter_scaleh <= 3; iter_scaleh++) {   // uniform
                 R pe = 0.0f, dpe = 0.0f, exne = 1.0f, thvebot = 0.0f, thle = 0.0f, qte = 0.0f, ue = 0.0f, ve = 0.0f;
+#if !UW_TAPE_ORDER
+                // The first two passes only find the scale height: the winds and tracers of the updraft feed
+                // nothing back into it, and of the level profiles only wu (an output at every level) and
+                // fer outlive the pass, so the last pass alone computes and stores the rest.  (The
+                // per-level diagnostics also show what an earlier, deeper pass left above the cloud top.)
+                const bool full = iter_scaleh == 3 || A.diag_level != nullptr;
+                // the updraft at the level below
+                R thlu_b = 0.0f, qtu_b = 0.0f, thvu_b = 0.0f, umf_b = 0.0f;
+#endif
                 if (!stop) {
                     kbup = krel;
                     kpen = krel;
@@ -1151,13 +1250,26 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     thvebot = thv0rel;
                     thle = thl0[krel] + ssthl0[krel] * (pe - p0[krel]);
                     qte = qt0[krel] + ssqt0[krel] * (pe - p0[krel]);
+#if !UW_TAPE_ORDER
+                    thlu_b = thlu[krel - 1];
+                    qtu_b = qtu[krel - 1];
+                    thvu_b = thvu[krel - 1];
+                    umf_b = umf[krel - 1];
+                    if (full) {   // uniform
+#endif
                     ue = GL(u0, krel) + ssu0[krel] * (pe - p0[krel]);
                     ve = GL(v0, krel) + ssv0[krel] * (pe - p0[krel]);
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, krel) + sstr0[m][krel] * (pe - p0[krel]);
+#if !UW_TAPE_ORDER
+                    }
+#endif
                 }
 
+#if UW_TAPE_ORDER
                 // levels k = krel .. mkx-1, taken by every lane as k = krel + j
                 bool ldone = stop;
+#pragma unroll 1
                 for (int j = 0; j <= mkx - 2; j++) {   // uniform
                     const int k = krel + j;
                     if (k > mkx - 1) ldone = true;
@@ -1171,11 +1283,12 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     // environment at the layer midpoint: the same in both iter_xc passes, so the
                     // second pass reuses the first one's conden and qsat results (same bits)
                     R thv0j = 0.0f, excess0 = 0.0f;
+#pragma unroll 1
                     for (int iter_xc = 1; iter_xc <= 2; iter_xc++) {
                         if (!xdone && !stop) do {
                         wtw = wu[km1] * wu[km1];
                         if (iter_xc == 1) {
-                            if (CONDEN(pe, exne, thle, qte, thj, qvj, qlj, qij, tbld, tblf)) {
+                            if (CONDEN(pe, exne, thle, qte, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                                 xflags |= UW_X_CONDEN;
                                 id_exit = true;
                                 stop = true;
@@ -1185,7 +1298,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             excess0 = qte - qsat_qs(thle * exne, pe, tbld, tblf);
                         }
                         rho0j = pe / (r * thv0j * exne);
-                        if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, tbld, tblf)) {
+                        if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                             xflags |= UW_X_CONDEN;
                             id_exit = true;
                             stop = true;
@@ -1198,7 +1311,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             R exqi = ((qlj + qij) - criqc) * qij / (qlj + qij);
                             qtue = qtue - exql - exqi;
                             thlue = thlue + (xlv / cp / exne) * exql + (xls / cp / exne) * exqi;
-                            if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, tbld, tblf)) {
+                            if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                                 xflags |= UW_X_CONDEN;
                                 id_exit = true;
                                 stop = true;
@@ -1215,7 +1328,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             R xsat = excessu / (excessu - excess0);
                             R thlxsat = thlue + xsat * (thle - thlue);
                             R qtxsat = qtue + xsat * (qte - qtue);
-                            if (CONDEN(pe, exne, thlxsat, qtxsat, thj, qvj, qlj, qij, tbld, tblf)) {
+                            if (CONDEN(pe, exne, thlxsat, qtxsat, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                                 xflags |= UW_X_CONDEN;
                                 id_exit = true;
                                 stop = true;
@@ -1223,6 +1336,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             }
                             R thvxsat = thj * (1.0f + zvir * qvj - qlj - qij);
                             R x_cu = 0.0f, x_en = 0.0f;
+#pragma unroll 1
                             for (int kk = 1; kk <= 2; kk++) {
                                 R thv_x0, thv_x1;
                                 if (kk == 1) {
@@ -1275,6 +1389,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             qtu[k] = qtu[km1] + (qte + ssqt0[k] * dpe / 2.0f - qtu[km1]) * fer[k] * dpe;
                             uu[k] = uu[km1] + (ue + ssu0[k] * dpe / 2.0f - uu[km1]) * fer[k] * dpe - PGFc * ssu0[k] * dpe;
                             vu[k] = vu[km1] + (ve + ssv0[k] * dpe / 2.0f - vu[km1]) * fer[k] * dpe - PGFc * ssv0[k] * dpe;
+#pragma unroll 1
                             for (int m = 0; m < ncnst; m++)
                                 tru[m][k] = tru[m][km1] + (tre[m] + sstr0[m][k] * dpe / 2.0f - tru[m][km1]) * fer[k] * dpe;
                         } else {
@@ -1287,11 +1402,12 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                                     (ue + ssu0[k] * dpe / 2.0f - uu[km1] + (1.0f - PGFc) * ssu0[k] / fer[k]) * ef;
                             vu[k] = (ve + (1.0f - PGFc) * ssv0[k] / fer[k] - ssv0[k] * dpe / 2.0f) -
                                     (ve + ssv0[k] * dpe / 2.0f - vu[km1] + (1.0f - PGFc) * ssv0[k] / fer[k]) * ef;
+#pragma unroll 1
                             for (int m = 0; m < ncnst; m++)
                                 tru[m][k] = (tre[m] + sstr0[m][k] / fer[k] - sstr0[m][k] * dpe / 2.0f) -
                                             (tre[m] + sstr0[m][k] * dpe / 2.0f - tru[m][km1] + sstr0[m][k] / fer[k]) * ef;
                         }
-                        if (CONDEN(ps0[k], exns0[k], thlu[k], qtu[k], thj, qvj, qlj, qij, tbld, tblf)) {
+                        if (CONDEN(ps0[k], exns0[k], thlu[k], qtu[k], thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                             xflags |= UW_X_CONDEN;
                             id_exit = true;
                             stop = true;
@@ -1304,7 +1420,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             thlu[k] = thlu[k] + (xlv / cp / exns0[k]) * exql + (xls / cp / exns0[k]) * exqi;
                             dwten[k] = exql;
                             diten[k] = exqi;
-                            if (CONDEN(ps0[k], exns0[k], thlu[k], qtu[k], thj, qvj, qlj, qij, tbld, tblf)) {
+                            if (CONDEN(ps0[k], exns0[k], thlu[k], qtu[k], thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                                 xflags |= UW_X_CONDEN;
                                 id_exit = true;
                                 stop = true;
@@ -1369,14 +1485,286 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     qte = qt0[k + 1];
                     ue = GL(u0, k + 1);
                     ve = GL(v0, k + 1);
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, k + 1);
                     } while (0);
                     if (stop) ldone = true;
                     UW_SYNC();
                 }
+#else
+                // levels k = krel .. mkx-1, taken by every lane as k = krel + j
+                bool ldone = stop;
+#pragma unroll 1
+                for (int j = 0; j <= mkx - 2; j++) {   // uniform
+                    const int k = krel + j;
+                    if (k > mkx - 1) ldone = true;
+                    if (!ldone) do {
+                    const R wu_b = wu[k - 1];   // (carried like the others, the FMA-contracted modes would round
+                                                     // wu_b * wu_b with what follows it)
+                    R thlue = thlu_b;
+                    R qtue = qtu_b;
+                    R wue = wu_b;
+                    wtwb = wtw;
+                    bool xdone = false;
+                    // environment at the layer midpoint: the same in both iter_xc passes, so the
+                    // second pass reuses the first one's results (same bits)
+                    R thv0j = 0.0f, excess0 = 0.0f, reib = 0.0f;
+                    R thlu_k = 0.0f, qtu_k = 0.0f, thvu_k = 0.0f, fer_k = 0.0f, fdr_k = 0.0f, rei_k = 0.0f, ef_k = 0.0f,
+                           dmf_k = 0.0f, dw_k = 0.0f, di_k = 0.0f;
+                    const R cridis = rle * scaleh;
+#pragma unroll 1
+                    for (int iter_xc = 1; iter_xc <= 2; iter_xc++) {
+                        if (!xdone && !stop) do {
+                        wtw = wu_b * wu_b;
+                        if (iter_xc == 1) {
+                            if (CONDEN(pe, exne, thle, qte, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
+                                xflags |= UW_X_CONDEN;
+                                id_exit = true;
+                                stop = true;
+                                break;
+                            }
+                            thv0j = thj * (1.0f + zvir * qvj - qlj - qij);
+                            excess0 = qte - UW_QSAT_OF_CONDEN(thle * exne, pe);
+                            rho0j = pe / (r * thv0j * exne);
+                            reib = (0.5f * rkm / GL(z0, k) / g / rho0j);
+                        }
+                        if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
+                            xflags |= UW_X_CONDEN;
+                            id_exit = true;
+                            stop = true;
+                            break;
+                        }
+                        // condensate above criqc leaves the updraft; without it the Fortran's
+                        // second conden call repeats the first one's arguments and results
+                        if ((qlj + qij) > criqc) {
+                            R exql = ((qlj + qij) - criqc) * qlj / (qlj + qij);
+                            R exqi = ((qlj + qij) - criqc) * qij / (qlj + qij);
+                            qtue = qtue - exql - exqi;
+                            thlue = thlue + (xlv / cp / exne) * exql + (xls / cp / exne) * exqi;
+                            if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
+                                xflags |= UW_X_CONDEN;
+                                id_exit = true;
+                                stop = true;
+                                break;
+                            }
+                        }
+                        R thvj = thj * (1.0f + zvir * qvj - qlj - qij);
+                        R excessu = qtue - UW_QSAT_OF_CONDEN(thlue * exne, pe);
+                        R xc;
+                        if ((excessu <= 0.0f && excess0 <= 0.0f) || (excessu >= 0.0f && excess0 >= 0.0f)) {
+                            xc = MN(1.0f, MX(0.0f, 1.0f - 2.0f * rbuoy * g * cridis / (wue * wue) * (1.0f - thvj / thv0j)));
+                        } else {
+                            R xsat = excessu / (excessu - excess0);
+                            R thlxsat = thlue + xsat * (thle - thlue);
+                            R qtxsat = qtue + xsat * (qte - qtue);
+                            if (CONDEN(pe, exne, thlxsat, qtxsat, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
+                                xflags |= UW_X_CONDEN;
+                                id_exit = true;
+                                stop = true;
+                                break;
+                            }
+                            R thvxsat = thj * (1.0f + zvir * qvj - qlj - qij);
+                            R x_cu = 0.0f, x_en = 0.0f;
+#pragma unroll 1
+                            for (int kk = 1; kk <= 2; kk++) {
+                                R thv_x0, thv_x1;
+                                if (kk == 1) {
+                                    thv_x0 = thvj;
+                                    thv_x1 = (1.0f - 1.0f / xsat) * thvj + (1.0f / xsat) * thvxsat;
+                                } else {
+                                    thv_x1 = thv0j;
+                                    thv_x0 = (xsat / (xsat - 1.0f)) * thv0j + (1.0f / (1.0f - xsat)) * thvxsat;
+                                }
+                                R aquad = wue * wue;
+                                R bquad = 2.0f * rbuoy * g * cridis * (thv_x1 - thv_x0) / thv0j - 2.0f * (wue * wue);
+                                R cquad = 2.0f * rbuoy * g * cridis * (thv_x0 - thv0j) / thv0j + (wue * wue);
+                                if (kk == 1) {
+                                    if ((bquad * bquad - 4.0f * aquad * cquad) >= 0.0f) {
+                                        roots(aquad, bquad, cquad, xs1, xs2);
+                                        x_cu = MN(1.0f, MX(0.0f, MN(xsat, MN(xs1, xs2))));
+                                    } else {
+                                        x_cu = xsat;
+                                    }
+                                } else {
+                                    if ((bquad * bquad - 4.0f * aquad * cquad) >= 0.0f) {
+                                        roots(aquad, bquad, cquad, xs1, xs2);
+                                        x_en = MN(1.0f, MX(0.0f, MX(xsat, MN(xs1, xs2))));
+                                    } else {
+                                        x_en = 1.0f;
+                                    }
+                                }
+                            }
+                            if (x_cu == xsat) xc = MX(x_cu, x_en);
+                            else xc = x_cu;
+                        }
+                        R ee2 = xc * xc;
+                        R ud2 = 1.0f - 2.0f * xc + xc * xc;
+                        rei_k = reib;
+                        if (xc > 0.5f) rei_k = MN(rei_k, 0.9f * logf(dp0[k] / g / dt / umf_b + 1.0f) / dpe / (2.0f * xc - 1.0f));
+                        fer_k = rei_k * ee2;
+                        fdr_k = rei_k * ud2;
+                        // compute_zwshcu's entrainment option (zwshcu.F90:2818-2844)
+                        if (ZW && c.zw_ent) {
+                            bogbot = rbuoy * (thvu_b / thvebot - 1.0f) * g;
+                            fer_k = c.zw_ent0 * bogbot / MX(wue * wue, 1.0e-4f);
+                            R fer_min = 0.0f;
+                            if (bogbot > 1.e-4f) fer_min = 1.e-4f;
+                            fer_k = MN(MX(fer_k, fer_min), 3.0e-2f);
+                        }
+                        dmf_k = dpe * (fer_k - fdr_k);
+                        if (fer_k * dpe < 1.e-4f) {
+                            thlu_k = thlu_b + (thle + ssthl0[k] * dpe / 2.0f - thlu_b) * fer_k * dpe;
+                            qtu_k = qtu_b + (qte + ssqt0[k] * dpe / 2.0f - qtu_b) * fer_k * dpe;
+                        } else {
+                            ef_k = expf(-fer_k * dpe);
+                            thlu_k = (thle + ssthl0[k] / fer_k - ssthl0[k] * dpe / 2.0f) -
+                                     (thle + ssthl0[k] * dpe / 2.0f - thlu_b + ssthl0[k] / fer_k) * ef_k;
+                            qtu_k = (qte + ssqt0[k] / fer_k - ssqt0[k] * dpe / 2.0f) -
+                                    (qte + ssqt0[k] * dpe / 2.0f - qtu_b + ssqt0[k] / fer_k) * ef_k;
+                        }
+                        if (CONDEN(ps0[k], exns0[k], thlu_k, qtu_k, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
+                            xflags |= UW_X_CONDEN;
+                            id_exit = true;
+                            stop = true;
+                            break;
+                        }
+                        if ((qlj + qij) > criqc) {
+                            R exql = ((qlj + qij) - criqc) * qlj / (qlj + qij);
+                            R exqi = ((qlj + qij) - criqc) * qij / (qlj + qij);
+                            qtu_k = qtu_k - exql - exqi;
+                            thlu_k = thlu_k + (xlv / cp / exns0[k]) * exql + (xls / cp / exns0[k]) * exqi;
+                            dw_k = exql;
+                            di_k = exqi;
+                            if (CONDEN(ps0[k], exns0[k], thlu_k, qtu_k, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
+                                xflags |= UW_X_CONDEN;
+                                id_exit = true;
+                                stop = true;
+                                break;
+                            }
+                        } else {
+                            // nothing removed: the Fortran's second conden call repeats the first
+                            dw_k = 0.0f;
+                            di_k = 0.0f;
+                        }
+                        thvu_k = thj * (1.0f + zvir * qvj - qlj - qij);
+                        bogbot = rbuoy * (thvu_b / thvebot - 1.0f);
+                        bogtop = rbuoy * (thvu_k / thv0top[k] - 1.0f);
+                        R delbog = bogtop - bogbot;
+                        drage = fer_k * (1.0f + rdrag);
+                        R expfac = expf(-2.0f * drage * dpe);
+                        wtwb = wtw;
+                        if (drage * dpe > 1.e-3f)
+                            wtw = wtw * expfac + (delbog + (1.0f - expfac) * (bogbot + delbog / (-2.0f * drage * dpe))) / (rho0j * drage);
+                        else
+                            wtw = wtw + dpe * (bogbot + bogtop) / rho0j;
+                        if (wtw > 0.0f) {
+                            thlue = 0.5f * (thlu_b + thlu_k);
+                            qtue = 0.5f * (qtu_b + qtu_k);
+                            wue = 0.5f * sqrtf(MX(wtwb + wtw, 0.0f));
+                        } else {
+                            xdone = true;   // go to 111
+                        }
+                        } while (0);
+                    }
+                    if (stop) break;
+                    fer[k] = fer_k;
+                    // the mass flux and, in the last pass, the level's profiles with the final fer and fdr
+                    // (the Fortran evaluates them in each iter_xc pass)
+                    R umf_k = umf_b * expf(dmf_k);
+                    if (full) {
+                        const int km1 = k - 1;
+                        rei[k] = rei_k;
+                        thlu[k] = thlu_k;
+                        qtu[k] = qtu_k;
+                        thvu[k] = thvu_k;
+                        dwten[k] = dw_k;
+                        diten[k] = di_k;
+                        qltop[k] = qlj;
+                        qitop[k] = qij;
+                        if (fer_k * dpe < 1.e-4f) {
+                            uu[k] = uu[km1] + (ue + ssu0[k] * dpe / 2.0f - uu[km1]) * fer_k * dpe - PGFc * ssu0[k] * dpe;
+                            vu[k] = vu[km1] + (ve + ssv0[k] * dpe / 2.0f - vu[km1]) * fer_k * dpe - PGFc * ssv0[k] * dpe;
+#pragma unroll 1
+                            for (int m = 0; m < ncnst; m++)
+                                tru[m][k] = tru[m][km1] + (tre[m] + sstr0[m][k] * dpe / 2.0f - tru[m][km1]) * fer_k * dpe;
+                        } else {
+                            uu[k] = (ue + (1.0f - PGFc) * ssu0[k] / fer_k - ssu0[k] * dpe / 2.0f) -
+                                    (ue + ssu0[k] * dpe / 2.0f - uu[km1] + (1.0f - PGFc) * ssu0[k] / fer_k) * ef_k;
+                            vu[k] = (ve + (1.0f - PGFc) * ssv0[k] / fer_k - ssv0[k] * dpe / 2.0f) -
+                                    (ve + ssv0[k] * dpe / 2.0f - vu[km1] + (1.0f - PGFc) * ssv0[k] / fer_k) * ef_k;
+#pragma unroll 1
+                            for (int m = 0; m < ncnst; m++)
+                                tru[m][k] = (tre[m] + sstr0[m][k] / fer_k - sstr0[m][k] * dpe / 2.0f) -
+                                            (tre[m] + sstr0[m][k] * dpe / 2.0f - tru[m][km1] + sstr0[m][k] / fer_k) * ef_k;
+                        }
+                    }
+                    // (label 111, :2726-2793)
+                    if (umf_k == 0.0f) wtw = -1.0f;
+                    if (bogtop > 0.0f && wtw > 0.0f) kbup = k;
+                    if (wtw <= 0.0f) {
+                        kpen = k;
+                        ldone = true;
+                        if (full) {
+                            umf[k] = umf_k;
+                            fdr[k] = fdr_k;
+                        }
+                        break;   // go to 45
+                    }
+                    wu[k] = sqrtf(wtw);
+                    if (wu[k] > 100.0f) {
+                        xflags |= UW_X_WU;
+                        id_exit = true;
+                        stop = true;
+                        break;
+                    }
+                    {
+                        R rhos0j = ps0[k] / (r * 0.5f * (thv0bot[k + 1] + thv0top[k]) * exns0[k]);
+                        R ufrc_k = umf_k / (rhos0j * wu[k]);
+                        if (ufrc_k > rmaxfrac) {
+                            lflags |= UW_L_UFRC;
+                            ufrc_k = rmaxfrac;
+                            umf_k = rmaxfrac * rhos0j * wu[k];
+                            fdr_k = fer_k - logf(umf_k / umf_b) / dpe;
+                        }
+                        if (full) {
+                            ufrc[k] = ufrc_k;
+                            umf[k] = umf_k;
+                            fdr[k] = fdr_k;
+                        }
+                    }
+                    thlu_b = thlu_k;
+                    qtu_b = qtu_k;
+                    thvu_b = thvu_k;
+                    umf_b = umf_k;
+                    pe = p0[k + 1];
+                    dpe = dp0[k + 1];
+                    exne = exn0[k + 1];
+                    thvebot = thv0bot[k + 1];
+                    thle = thl0[k + 1];
+                    qte = qt0[k + 1];
+                    if (full) {
+                        ue = GL(u0, k + 1);
+                        ve = GL(v0, k + 1);
+#pragma unroll 1
+                        for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, k + 1);
+                    }
+                    } while (0);
+                    if (stop) ldone = true;
+                    UW_SYNC();
+                }
+#endif
                 UW_SYNC();
                 // (label 45) penetration depth (:2884-2907)
                 if (!stop) do {
+#if UW_TAPE_ORDER
+                const R thlu_b = thlu[kpen - 1], qtu_b = qtu[kpen - 1];
+#else
+                // the updraft at kpen - 1 (the release level's when no level stopped it: kpen = krel)
+                if (kpen == krel) {
+                    thlu_b = thlu[krel - 1];
+                    qtu_b = qtu[krel - 1];
+                }
+#endif
                 if (drage == 0.0f) {
                     R aquad = (bogtop - bogbot) / (ps0[kpen] - ps0[kpen - 1]);
                     R bquad = 2.0f * bogbot;
@@ -1401,22 +1789,23 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 if (ppen == -dp0[kpen] || ppen == 0.0f) lflags |= UW_L_PPEN;
                 // condensate at the cumulus top (:2917-2942)
                 if (fer[kpen] * (-ppen) < 1.e-4f) {
-                    thlu_top = thlu[kpen - 1] + (thl0[kpen] + ssthl0[kpen] * (-ppen) / 2.0f - thlu[kpen - 1]) * fer[kpen] * (-ppen);
-                    qtu_top = qtu[kpen - 1] + (qt0[kpen] + ssqt0[kpen] * (-ppen) / 2.0f - qtu[kpen - 1]) * fer[kpen] * (-ppen);
+                    thlu_top = thlu_b + (thl0[kpen] + ssthl0[kpen] * (-ppen) / 2.0f - thlu_b) * fer[kpen] * (-ppen);
+                    qtu_top = qtu_b + (qt0[kpen] + ssqt0[kpen] * (-ppen) / 2.0f - qtu_b) * fer[kpen] * (-ppen);
                 } else {
                     const R ef = expf(-fer[kpen] * (-ppen));
                     thlu_top = (thl0[kpen] + ssthl0[kpen] / fer[kpen] - ssthl0[kpen] * (-ppen) / 2.0f) -
-                               (thl0[kpen] + ssthl0[kpen] * (-ppen) / 2.0f - thlu[kpen - 1] + ssthl0[kpen] / fer[kpen]) * ef;
+                               (thl0[kpen] + ssthl0[kpen] * (-ppen) / 2.0f - thlu_b + ssthl0[kpen] / fer[kpen]) * ef;
                     qtu_top = (qt0[kpen] + ssqt0[kpen] / fer[kpen] - ssqt0[kpen] * (-ppen) / 2.0f) -
-                              (qt0[kpen] + ssqt0[kpen] * (-ppen) / 2.0f - qtu[kpen - 1] + ssqt0[kpen] / fer[kpen]) * ef;
+                              (qt0[kpen] + ssqt0[kpen] * (-ppen) / 2.0f - qtu_b + ssqt0[kpen] / fer[kpen]) * ef;
                 }
                 exntop = powf((ps0[kpen - 1] + ppen) / p00, rovcp);
-                if (CONDEN(ps0[kpen - 1] + ppen, exntop, thlu_top, qtu_top, thj, qvj, qlj, qij, tbld, tblf)) {
+                if (CONDEN(ps0[kpen - 1] + ppen, exntop, thlu_top, qtu_top, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                     xflags |= UW_X_CONDEN;
                     id_exit = true;
                     stop = true;
             break;
                 }
+#if UW_TAPE_ORDER
                 if ((qlj + qij) > criqc) {
                     dwten[kpen] = ((qlj + qij) - criqc) * qlj / (qlj + qij);
                     diten[kpen] = ((qlj + qij) - criqc) * qij / (qlj + qij);
@@ -1426,6 +1815,23 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     dwten[kpen] = 0.0f;
                     diten[kpen] = 0.0f;
                 }
+#else
+                if (full) {
+                    if ((qlj + qij) > criqc) {
+                        dwten[kpen] = ((qlj + qij) - criqc) * qlj / (qlj + qij);
+                        diten[kpen] = ((qlj + qij) - criqc) * qij / (qlj + qij);
+                        qtu_top = qtu_top - dwten[kpen] - diten[kpen];
+                        thlu_top = thlu_top + (xlv / cp / exntop) * dwten[kpen] + (xls / cp / exntop) * diten[kpen];
+                        id_top = CONDEN(ps0[kpen - 1] + ppen, exntop, thlu_top, qtu_top, thj, qvj, qlj, qij, rvj, tbld, tblf) != 0;
+                    } else {
+                        dwten[kpen] = 0.0f;
+                        diten[kpen] = 0.0f;
+                        id_top = false;
+                    }
+                    ql_top = qlj;
+                    qi_top = qij;
+                }
+#endif
                 {
                     R rhos0j = ps0[kpen - 1] / (r * 0.5f * (thv0bot[kpen] + thv0top[kpen - 1]) * exns0[kpen - 1]);
                     cush = zs0[kpen - 1] - ppen / rhos0j / g;
@@ -1445,12 +1851,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             break;
         }
         lflags &= ~UW_L_SHCU;
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             if (k < kpen) continue;
             umf[k] = 0.0f;
             emf[k] = 0.0f;
             ufrc[k] = 0.0f;
         }
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             if (k < kpen + 1) continue;
             dwten[k] = 0.0f;
@@ -1459,13 +1867,16 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             fdr[k] = 0.0f;
         }
         // penetrative entrainment (:3055-3183)
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             thlu_emf[k] = thlu[k];
             qtu_emf[k] = qtu[k];
             uu_emf[k] = uu[k];
             vu_emf[k] = vu[k];
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++) tru_emf[m][k] = tru[m][k];
         }
+#pragma unroll 1
         for (int k = mkx; k >= 0; k--) {
             if (k > kpen - 1 || k < kbup) continue;
             R rhos0j = ps0[k] / (r * 0.5f * (thv0bot[k + 1] + thv0top[k]) * exns0[k]);
@@ -1477,6 +1888,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 qtu_emf[k] = qt0[kpen] + ssqt0[kpen] * (ps0[k] - p0[kpen]);
                 uu_emf[k] = GL(u0, kpen) + ssu0[kpen] * (ps0[k] - p0[kpen]);
                 vu_emf[k] = GL(v0, kpen) + ssv0[kpen] * (ps0[k] - p0[kpen]);
+#pragma unroll 1
                 for (int m = 0; m < ncnst; m++) tru_emf[m][k] = GT(m + 1, kpen) + sstr0[m][kpen] * (ps0[k] - p0[kpen]);
             } else {
                 if ((emf[k + 1] - umf[k] * dp0[k + 1] * rei[k + 1] * rpen) < -0.1f * rhos0j) lflags |= UW_L_EMF;
@@ -1487,6 +1899,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     qtu_emf[k] = (qtu_emf[k + 1] * emf[k + 1] + qt0[k + 1] * (emf[k] - emf[k + 1])) / emf[k];
                     uu_emf[k] = (uu_emf[k + 1] * emf[k + 1] + GL(u0, k + 1) * (emf[k] - emf[k + 1])) / emf[k];
                     vu_emf[k] = (vu_emf[k + 1] * emf[k + 1] + GL(v0, k + 1) * (emf[k] - emf[k + 1])) / emf[k];
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++)
                         tru_emf[m][k] = (tru_emf[m][k + 1] * emf[k + 1] + GT(m + 1, k + 1) * (emf[k] - emf[k + 1])) / emf[k];
                 } else {
@@ -1494,6 +1907,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     qtu_emf[k] = qt0[k + 1];
                     uu_emf[k] = GL(u0, k + 1);
                     vu_emf[k] = GL(v0, k + 1);
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++) tru_emf[m][k] = GT(m + 1, k + 1);
                 }
             }
@@ -1504,37 +1918,44 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             R xtop = qt0[kinv + 1] + ssqt0[kinv + 1] * (ps0[kinv] - p0[kinv + 1]);
             R xbot = qt0[kinv - 1] + ssqt0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
             fluxbelowinv(cbmf, ps0, kinv, dt, xsrc, xmean, xtop, xbot, xflx);
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) if (k <= kinv - 1) qtflx[k] = xflx[k];
             xsrc = thlsrc;
             xmean = thl0[kinv];
             xtop = thl0[kinv + 1] + ssthl0[kinv + 1] * (ps0[kinv] - p0[kinv + 1]);
             xbot = thl0[kinv - 1] + ssthl0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
             fluxbelowinv(cbmf, ps0, kinv, dt, xsrc, xmean, xtop, xbot, xflx);
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) if (k <= kinv - 1) slflx[k] = cp * exns0[k] * xflx[k];
             xsrc = usrc;
             xmean = GL(u0, kinv);
             xtop = GL(u0, kinv + 1) + ssu0[kinv + 1] * (ps0[kinv] - p0[kinv + 1]);
             xbot = GL(u0, kinv - 1) + ssu0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
             fluxbelowinv(cbmf, ps0, kinv, dt, xsrc, xmean, xtop, xbot, xflx);
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) if (k <= kinv - 1) uflx[k] = xflx[k];
             xsrc = vsrc;
             xmean = GL(v0, kinv);
             xtop = GL(v0, kinv + 1) + ssv0[kinv + 1] * (ps0[kinv] - p0[kinv + 1]);
             xbot = GL(v0, kinv - 1) + ssv0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
             fluxbelowinv(cbmf, ps0, kinv, dt, xsrc, xmean, xtop, xbot, xflx);
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) if (k <= kinv - 1) vflx[k] = xflx[k];
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++) {
                 xsrc = trsrc[m];
                 xmean = GT(m + 1, kinv);
                 xtop = GT(m + 1, kinv + 1) + sstr0[m][kinv + 1] * (ps0[kinv] - p0[kinv + 1]);
                 xbot = GT(m + 1, kinv - 1) + sstr0[m][kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
                 fluxbelowinv(cbmf, ps0, kinv, dt, xsrc, xmean, xtop, xbot, xflx);
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) if (k <= kinv - 1) trflx[m][k] = xflx[k];
             }
         }
         // 2.f non-buoyancy-sorting fluxes (:3300-3313)
         {
             R uplus = 0.0f, vplus = 0.0f;
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 if (k < kinv || k > krel - 1) continue;
                 const int kp1 = k + 1;
@@ -1544,11 +1965,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 vplus = vplus + PGFc * ssv0[k] * (ps0[k] - ps0[k - 1]);
                 uflx[k] = cbmf * (usrc + uplus - (GL(u0, kp1) + ssu0[kp1] * (ps0[k] - p0[kp1])));
                 vflx[k] = cbmf * (vsrc + vplus - (GL(v0, kp1) + ssv0[kp1] * (ps0[k] - p0[kp1])));
+#pragma unroll 1
                 for (int m = 0; m < ncnst; m++)
                     trflx[m][k] = cbmf * (trsrc[m] - (GT(m + 1, kp1) + sstr0[m][kp1] * (ps0[k] - p0[kp1])));
             }
         }
         // 3.f buoyancy-sorting fluxes (:3322-3331)
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             if (k < krel || k > kbup - 1) continue;
             const int kp1 = k + 1;
@@ -1556,16 +1979,19 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             qtflx[k] = umf[k] * (qtu[k] - (qt0[kp1] + ssqt0[kp1] * (ps0[k] - p0[kp1])));
             uflx[k] = umf[k] * (uu[k] - (GL(u0, kp1) + ssu0[kp1] * (ps0[k] - p0[kp1])));
             vflx[k] = umf[k] * (vu[k] - (GL(v0, kp1) + ssv0[kp1] * (ps0[k] - p0[kp1])));
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++)
                 trflx[m][k] = umf[k] * (tru[m][k] - (GT(m + 1, kp1) + sstr0[m][kp1] * (ps0[k] - p0[kp1])));
         }
         // 4.f penetrative-entrainment fluxes (:3392-3401)
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             if (k < kbup || k > kpen - 1) continue;
             slflx[k] = cp * exns0[k] * emf[k] * (thlu_emf[k] - (thl0[k] + ssthl0[k] * (ps0[k] - p0[k])));
             qtflx[k] = emf[k] * (qtu_emf[k] - (qt0[k] + ssqt0[k] * (ps0[k] - p0[k])));
             uflx[k] = emf[k] * (uu_emf[k] - (GL(u0, k) + ssu0[k] * (ps0[k] - p0[k])));
             vflx[k] = emf[k] * (vu_emf[k] - (GL(v0, k) + ssv0[k] * (ps0[k] - p0[k])));
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++)
                 trflx[m][k] = emf[k] * (tru_emf[m][k] - (GT(m + 1, k) + sstr0[m][k] * (ps0[k] - p0[k])));
         }
@@ -1578,6 +2004,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     ((kk) <= kinv - 2 ? cbmf * (ps0[0] - ps0[(kk)]) / (ps0[0] - ps0[kinv - 1])                             \
                       : ((kk) <= krel - 1 ? cbmf : ((kk) <= kbup - 1 ? umf[(kk)] : ((kk) <= kpen - 1 ? emf[(kk)] : 0.0f))))
             bool ldone = stop;
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {   // uniform
                 if (k > kpen) ldone = true;
                 if (!ldone) do {
@@ -1610,7 +2037,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 }
                 R thl_prog = thl0[k] + thlten_sub * dt;
                 R qt_prog = MX(qt0[k] + qtten_sub * dt, 1.e-12f);
-                if (CONDEN(p0[k], exn0[k], thl_prog, qt_prog, thj, qvj, qlj, qij, tbld, tblf)) {
+                if (CONDEN(p0[k], exn0[k], thl_prog, qt_prog, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                     id_exit = true;
                     stop = true;
             break;
@@ -1626,6 +2053,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         UW_SYNC();
         if (!stop) do {
         // momentum tendency (:3488-3501)
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             if (k > kpen) continue;
             uten[k] = (uflx[k - 1] - uflx[k]) * g / dp0[k];
@@ -1642,6 +2070,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         {
             R qlubelow = 0.0f, qiubelow = 0.0f;
             bool ldone = stop;
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {   // uniform
                 if (k > kpen) ldone = true;
                 if (!ldone) do {
@@ -1681,10 +2110,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     qlj = 0.0f;
                     qij = 0.0f;
                 } else {
-                    // one conden call site for the release level, the cloud top and the levels between
+                    // the release level, the cloud top and the levels between
                     const bool atrel = (k == krel), attop = (k != krel && k == kpen);
+#if UW_TAPE_ORDER
                     if (atrel) {
-                        if (CONDEN(prel, exprel, thlu[krel - 1], qtu[krel - 1], thj, qvj, qlj, qij, tbld, tblf)) {
+                        if (CONDEN(prel, exprel, thlu[krel - 1], qtu[krel - 1], thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                             xflags |= UW_X_CONDEN;
                             id_exit = true;
                             stop = true;
@@ -1694,12 +2124,26 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                         qiubelow = qij;
                     }
                     if (CONDEN(attop ? ps0[k - 1] + ppen : ps0[k], attop ? exntop : exns0[k], attop ? thlu_top : thlu[k],
-                               attop ? qtu_top : qtu[k], thj, qvj, qlj, qij, tbld, tblf)) {
+                               attop ? qtu_top : qtu[k], thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                         xflags |= UW_X_CONDEN;
                         id_exit = true;
                         stop = true;
                         break;
                     }
+#else
+                    if (attop && id_top) {
+                        xflags |= UW_X_CONDEN;
+                        id_exit = true;
+                        stop = true;
+                        break;
+                    }
+                    if (atrel) {
+                        qlubelow = ql_rel;
+                        qiubelow = qi_rel;
+                    }
+                    qlj = attop ? ql_top : qltop[k];
+                    qij = attop ? qi_top : qitop[k];
+#endif
                     if (atrel) {
                         qlu_mid = 0.5f * (qlubelow + qlj) * (prel - ps0[k]) / (ps0[k - 1] - ps0[k]);
                         qiu_mid = 0.5f * (qiubelow + qij) * (prel - ps0[k]) / (ps0[k - 1] - ps0[k]);
@@ -1739,7 +2183,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     nc_lm = nc_lm - g * umf[k] * trl / (ps0[k - 1] - ps0[k]);
                     nc_im = nc_im - g * umf[k] * tri / (ps0[k - 1] - ps0[k]);
                     R ql_emf_kbup, qi_emf_kbup, thjj, qvjj;
-                    if (CONDEN(p0[k], exn0[k], thlu_emf[k], qtu_emf[k], thjj, qvjj, ql_emf_kbup, qi_emf_kbup, tbld, tblf)) {
+                    if (CONDEN(p0[k], exn0[k], thlu_emf[k], qtu_emf[k], thjj, qvjj, ql_emf_kbup, qi_emf_kbup, rvj, tbld, tblf)) {
                         id_exit = true;
                         stop = true;
             break;
@@ -1768,10 +2212,12 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         if (!stop) do {
         {
             Kahan evpint_rain, evpint_snow;
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 flxrain[k] = 0.0f;
                 flxsnow[k] = 0.0f;
             }
+#pragma unroll 1
             for (int k = mkx; k >= 1; k--) {
                 R snowmlt;
                 if (t0[k] > 273.16f) snowmlt = MX(0.0f, flxsnow[k] * g / dp0[k]);
@@ -1816,6 +2262,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             snow = flxsnow[0] / 1000.0f;
         }
         // remove detrained condensate (:3966-3981)
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             if (k > kpen) continue;
             qtten[k] = qtten[k] - qc[k];
@@ -1874,25 +2321,30 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             slten[k] = sten[k] - xlv * qlten[k] - xls * qiten[k];
         }
         // tracer tendencies (:4007-4076)
+#pragma unroll 1
         for (int m = 4; m <= ncnst; m++) {
             if (m != ixnumliq && m != ixnumice) {
                 const R trmin = c.qmin[m - 1];
                 const bool wet = c.wet[m - 1] != 0;
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) {
                     trflx_d[k] = 0.0f;
                     trflx_u[k] = 0.0f;
                 }
+#pragma unroll 1
                 for (int k = 1; k <= mkx - 1; k++) {
                     R pdelx = wet ? dp0[k] : GL(dpdry0, k);
                     R dum = (GT(m, k) - trmin) * pdelx / g / dt + trflx[m - 1][k - 1] - trflx[m - 1][k] + trflx_d[k - 1];
                     trflx_d[k] = MN(0.0f, dum);
                 }
+#pragma unroll 1
                 for (int k = mkx; k >= 2; k--) {
                     R pdelx = wet ? dp0[k] : GL(dpdry0, k);
                     R dum = (GT(m, k) - trmin) * pdelx / g / dt + trflx[m - 1][k - 1] - trflx[m - 1][k] +
                                  trflx_d[k - 1] - trflx_d[k] - trflx_u[k];
                     trflx_u[k - 1] = MX(0.0f, -dum);
                 }
+#pragma unroll 1
                 for (int k = 1; k <= mkx; k++) {
                     R pdelx = wet ? dp0[k] : GL(dpdry0, k);
                     trten[m - 1][k] = (trflx[m - 1][k - 1] - trflx[m - 1][k] + trflx_d[k - 1] - trflx_d[k] +
@@ -1901,24 +2353,36 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             }
         }
         // in-cloud diagnostics (:4092-4158)
-        if (CONDEN(prel, exprel, thlu[krel - 1], qtu[krel - 1], thj, qvj, qlj, qij, tbld, tblf)) {
+#if UW_TAPE_ORDER
+        if (CONDEN(prel, exprel, thlu[krel - 1], qtu[krel - 1], thj, qvj, qlj, qij, rvj, tbld, tblf)) {
             xflags |= UW_X_CONDEN;
             id_exit = true;
             stop = true;
             break;
         }
+#else
+        qlj = ql_rel;
+        qij = qi_rel;
+#endif
         } while (0);
         UW_SYNC();
         {
             R qcubelow = qlj + qij, qlubelow = qlj, qiubelow = qij;
             bool ldone = stop;
+#pragma unroll 1
             for (int j = 0; j <= mkx; j++) {   // uniform
                 const int k = krel + j;
                 if (k > kpen) ldone = true;
                 if (!ldone) do {
                 const bool attop = (k == kpen);
+#if UW_TAPE_ORDER
                 const int idc = CONDEN(attop ? ps0[k - 1] + ppen : ps0[k], attop ? exntop : exns0[k],
-                                       attop ? thlu_top : thlu[k], attop ? qtu_top : qtu[k], thj, qvj, qlj, qij, tbld, tblf);
+                                       attop ? thlu_top : thlu[k], attop ? qtu_top : qtu[k], thj, qvj, qlj, qij, rvj, tbld, tblf);
+#else
+                const bool idc = attop && id_top;
+                qlj = attop ? ql_top : qltop[k];
+                qij = attop ? qi_top : qitop[k];
+#endif
                 if (idc) {
                     xflags |= UW_X_CONDEN;
                     id_exit = true;
@@ -1964,17 +2428,20 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 
         if (iter == 1) {
             // Save the iteration-1 outputs into the output slots (the Fortran *_s copies, :4177-4277)
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 OI(umf, k) = umf[k];
                 OI(slflx, k) = slflx[k];
                 OI(qtflx, k) = qtflx[k];
             }
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {
                 OL(qvten, k) = qvten[k]; OL(qlten, k) = qlten[k]; OL(qiten, k) = qiten[k];
                 OL(sten, k) = sten[k]; OL(uten, k) = uten[k]; OL(vten, k) = vten[k];
                 OL(qrten, k) = qrten[k]; OL(qsten, k) = qsten[k]; OL(evapc, k) = evapc[k];
                 OL(cufrc, k) = cufrc[k]; OL(qcu, k) = qcu[k]; OL(qlu, k) = qlu[k];
                 OL(qiu, k) = qiu[k]; OL(qc, k) = qc[k];
+#pragma unroll 1
                 for (int m = 1; m <= ncnst; m++) OT(m, k) = trten[m - 1][k];
             }
             A.precip[i] = precip;
@@ -1989,6 +2456,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             pbup_s = ps0[kbup]; ppen_s = ps0[kpen - 1] + ppen; tkeavg_s = tkeavg;
             kinv_s = kinv; klcl_s = klcl; klfc_s = klfc; krel_s = krel; kbup_s = kbup; kpen_s = kpen;
             // advance the state for the second CIN estimate (:4177-4184, :4285-4327)
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {
                 R qv0s = qv0[k] + qvten[k] * dt;
                 R ql0s = ql0[k] + qlten[k] * dt;
@@ -2010,11 +2478,12 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         UW_SYNC();
         if (iter == 1) {   // uniform
             bool ldone = stop;
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {   // uniform
                 if (!ldone) do {
                 R thl0bot = thl0[k] + ssthl0[k] * (ps0[k - 1] - p0[k]);
                 R qt0bot = qt0[k] + ssqt0[k] * (ps0[k - 1] - p0[k]);
-                if (CONDEN(ps0[k - 1], exns0[k - 1], thl0bot, qt0bot, thj, qvj, qlj, qij, tbld, tblf)) {
+                if (CONDEN(ps0[k - 1], exns0[k - 1], thl0bot, qt0bot, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                     xflags |= UW_X_CONDEN;
                     id_exit = true;
                     stop = true;
@@ -2024,7 +2493,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 thvl0bot[k] = thl0bot * (1.0f + zvir * qt0bot);
                 R thl0top = thl0[k] + ssthl0[k] * (ps0[k] - p0[k]);
                 R qt0top = qt0[k] + ssqt0[k] * (ps0[k] - p0[k]);
-                if (CONDEN(ps0[k], exns0[k], thl0top, qt0top, thj, qvj, qlj, qij, tbld, tblf)) {
+                if (CONDEN(ps0[k], exns0[k], thl0top, qt0top, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                     xflags |= UW_X_CONDEN;
                     id_exit = true;
                     stop = true;
@@ -2042,6 +2511,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 
     // ---- final outputs (uwshcu.F90:4337-4370) --------------------------------------------------
     if (!stop) {
+#pragma unroll 1
     for (int k = 0; k <= mkx; k++) {
         OI(umf, k) = umf[k];
         OI(wu, k) = wu[k];
@@ -2050,12 +2520,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         OI(flxprc1, k) = flxrain[k] + flxsnow[k];
         OI(flxsnow1, k) = flxsnow[k];
     }
+#pragma unroll 1
     for (int k = 1; k <= mkx; k++) {
         OL(qvten, k) = qvten[k]; OL(qlten, k) = qlten[k]; OL(qiten, k) = qiten[k];
         OL(sten, k) = sten[k]; OL(uten, k) = uten[k]; OL(vten, k) = vten[k];
         OL(qrten, k) = qrten[k]; OL(qsten, k) = qsten[k]; OL(evapc, k) = evapc[k];
         OL(cufrc, k) = cufrc[k]; OL(qcu, k) = qcu[k]; OL(qlu, k) = qlu[k];
         OL(qiu, k) = qiu[k]; OL(qc, k) = qc[k];
+#pragma unroll 1
         for (int m = 1; m <= ncnst; m++) OT(m, k) = trten[m - 1][k];
     }
     A.precip[i] = precip;
@@ -2082,6 +2554,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     if (!cand && !handed) {
     if (id_exit) {
         xflags |= UW_X_UWCU;
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             OI(umf, k) = 0.0f;
             OI(wu, k) = 0.0f;
@@ -2090,11 +2563,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             OI(flxprc1, k) = 0.0f;
             OI(flxsnow1, k) = 0.0f;
         }
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             OL(qvten, k) = 0.0f; OL(qlten, k) = 0.0f; OL(qiten, k) = 0.0f; OL(sten, k) = 0.0f;
             OL(uten, k) = 0.0f; OL(vten, k) = 0.0f; OL(qrten, k) = 0.0f; OL(qsten, k) = 0.0f;
             OL(evapc, k) = 0.0f; OL(cufrc, k) = 0.0f; OL(qcu, k) = 0.0f; OL(qlu, k) = 0.0f;
             OL(qiu, k) = 0.0f; OL(qc, k) = 0.0f;
+#pragma unroll 1
             for (int m = 1; m <= ncnst; m++) OT(m, k) = 0.0f;
         }
         A.precip[i] = 0.0f;
@@ -2107,10 +2582,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         if (A.diag_real) {
             A.diag_real[UW_DR_CIN * (size_t)mix + i] = -1.0f;
             A.diag_real[UW_DR_CINLCL * (size_t)mix + i] = -1.0f;
+#pragma unroll 1
             for (int j = UW_DR_PLCL; j < UW_NDR; j++) A.diag_real[j * (size_t)mix + i] = 0.0f;
         }
         if (A.diag_level)
+#pragma unroll 1
             for (int j = 0; j < UW_NDL; j++)
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) DLV(j, k) = 0.0f;
         kinv = klcl = klfc = krel = kbup = kpen = 0;
     }
@@ -2147,6 +2625,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     }
 #undef UW_SYNC
 #undef CONDEN
+#undef UW_QSAT_OF_CONDEN
 #undef RI
 #undef RL
 #undef CNT

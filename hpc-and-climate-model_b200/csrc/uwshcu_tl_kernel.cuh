@@ -17,6 +17,13 @@ typedef uwshcu_tangent UwTangent;
 __constant__ UwConst c;
 __constant__ double c_estbl[UW_TBL];
 
+// UW_TAPE_ORDER: the adjoint kernel's operations in the order, and with the repetitions, of the Fortran's
+// updraft.  A shorter tape would group the additions of its reverse sweep differently, and where a column
+// is ill-conditioned the gradient's last bits are large; its values are the same either way.
+#ifndef UW_TAPE_ORDER
+#define UW_TAPE_ORDER 0
+#endif
+
 #define MX(a, b) ((a) > (b) ? (a) : (b))
 #define MN(a, b) ((a) < (b) ? (a) : (b))
 
@@ -73,17 +80,17 @@ __device__ __forceinline__ Tl qsat_qs(Tl t, Tl p, const double* __restrict__ tbl
 
 __device__ __forceinline__ Tl exnf(Tl p) { return uw_pow(p / c.p00, c.rovcp); }
 
-// conden (uwshcu.F90:4718-4785) with ex = exnf(p) supplied by the caller.  Not inlined: the kernel
-// calls it from ~30 sites, and one shared copy keeps the kernel inside the instruction cache
-// (inlined, the stall on instruction fetch doubled the run time).
-__device__ __noinline__ int conden(Tl p, Tl ex, Tl thl, Tl qt, Tl& th, Tl& qv,
-                                      Tl& ql, Tl& qi, const double* __restrict__ tbl)
+// conden (uwshcu.F90:4718-4785) with ex = exnf(p) supplied by the caller.  rv0: the saturation humidity
+// at (thl ex, p), its first lookup.
+__device__ __forceinline__ int conden(Tl p, Tl ex, Tl thl, Tl qt, Tl& th, Tl& qv,
+                                      Tl& ql, Tl& qi, Tl& rv0, const double* __restrict__ tbl)
 {
     Tl tc = thl * ex;
     Tl nu = MX(MN((268.0 - tc) / 20.0, 1.0), 0.0);
     Tl leff = (1.0 - nu) * c.xlv + nu * c.xls;
     Tl temps = tc;
     Tl rvls = qsat_qs(temps, p, tbl);
+    rv0 = rvls;
     int id_check = 0;
     if (rvls >= qt) {
         qv = qt;
@@ -120,14 +127,15 @@ __device__ __noinline__ int conden(Tl p, Tl ex, Tl thl, Tl qt, Tl& th, Tl& qv,
 // iteration and fall below 1e-10 T after 5-7, so the result differs from conden by about 1e-12
 // relative.  A lane's result depends only on its own column; the warp leaves the loop when every
 // lane is done (__all_sync over the lanes active at the call), so the lanes stay together.
-__device__ __noinline__ int conden_fast(Tl p, Tl ex, Tl thl, Tl qt, Tl& th, Tl& qv,
-                                        Tl& ql, Tl& qi, const double* __restrict__ tbl)
+__device__ __forceinline__ int conden_fast(Tl p, Tl ex, Tl thl, Tl qt, Tl& th, Tl& qv,
+                                           Tl& ql, Tl& qi, Tl& rv0, const double* __restrict__ tbl)
 {
     Tl tc = thl * ex;
     Tl nu = MX(MN((268.0 - tc) / 20.0, 1.0), 0.0);
     Tl leff = (1.0 - nu) * c.xlv + nu * c.xls;
     Tl temps = tc;
     Tl rvls = qsat_qs(temps, p, tbl);
+    rv0 = rvls;
     int id_check = 0;
     if (rvls >= qt) {
         qv = qt;
@@ -159,6 +167,34 @@ __device__ __noinline__ int conden_fast(Tl p, Tl ex, Tl thl, Tl qt, Tl& th, Tl& 
         id_check = (fabs((temps - (leff / c.cp) * qc) - tc) >= 1.0) ? 1 : 0;
     }
     return id_check;
+}
+
+// The column code's saturation adjustment: one call for its ~20 sites (inlined at each of them, the stall
+// on instruction fetch doubled the run time), with the results by value, in registers (through
+// references they went through the stack, a store and a load each around every call).
+struct CondenOut {
+    Tl th, qv, ql, qi, rv0;
+    int id;
+};
+template <int FAST>
+__device__ __noinline__ CondenOut conden_out(Tl p, Tl ex, Tl thl, Tl qt, const double* __restrict__ tbl)
+{
+    CondenOut r;
+    if (FAST) r.id = conden_fast(p, ex, thl, qt, r.th, r.qv, r.ql, r.qi, r.rv0, tbl);
+    else r.id = conden(p, ex, thl, qt, r.th, r.qv, r.ql, r.qi, r.rv0, tbl);
+    return r;
+}
+template <int FAST>
+__device__ __forceinline__ int conden_call(Tl p, Tl ex, Tl thl, Tl qt, Tl& th, Tl& qv,
+                                           Tl& ql, Tl& qi, Tl& rv0, const double* __restrict__ tbl)
+{
+    const CondenOut r = conden_out<FAST>(p, ex, thl, qt, tbl);
+    th = r.th;
+    qv = r.qv;
+    ql = r.ql;
+    qi = r.qi;
+    rv0 = r.rv0;
+    return r.id;
 }
 
 // roots (uwshcu.F90:4787-4829); r1/r2 keep the caller's values on the failure branches.
@@ -363,8 +399,8 @@ __device__ __forceinline__ void fluxbelowinv(Tl cbmf, const Tl* ps0, int kinv, T
 // findsp (uwshcu.F90:5164-5454) for one point; returns the wet-bulb qsp and ORs error bits.
 __device__ Tl findsp_point(Tl q, Tl t, Tl p, unsigned int& errbits, const double* __restrict__ tbl)
 {
-    const Tl omeps = 1.0 - c.epsqs, trinv = 1.0 / c.ttrice, a1 = 7.5 * uw_log(10.0), rair = 287.04;
-    const Tl c3 = rair * a1 / c.cpws, dttol = 1.e-4, dqtol = 1.e-4, tt0 = 273.15;
+    const Tl omeps = 1.0 - c.epsqs, trinv = 1.0 / c.ttrice;
+    const Tl c3 = c.findsp_c3, dttol = 1.e-4, dqtol = 1.e-4, tt0 = 273.15;
     Tl dtt = 0.0, dq = 0.0, enin, enout = 1.0, tsp, qsp, hltalt = 0.0;
     int doit = 0;
     Tl tlim = MN(MX(t, 173.0), 373.0);
@@ -468,7 +504,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                                           const UwTangent& T)
 {
     const int i = (MODE == UW_MODE_RESUME && active) ? A.hand->col[i_in] : i_in;
-#define CONDEN(...) (FAST ? conden_fast(__VA_ARGS__) : conden(__VA_ARGS__))
+    // Code size bounds the worklist passes: with the loops unrolled by the compiler and exp, log and pow
+    // inlined at each use their kernels were 833 kB (LIST1) and 631 kB (RESUME), far beyond the
+    // instruction caches that 16 warps at different places share, and at full occupancy a warp waited 4.4
+    // to 6.5 cycles per instruction for its next one.  So no loop here is unrolled and the
+    // transcendentals are calls.
+#define CONDEN(...) conden_call<FAST>(__VA_ARGS__)
+// qsat_qs(t, p) right after a CONDEN call at that temperature and pressure: its first lookup
+#define UW_QSAT_OF_CONDEN(t, p) rvj
     bool cand = false;
     // lanes of this warp that run a column; UW_SYNC() joins them where every one of them arrives
     const unsigned live = __ballot_sync(0xffffffffu, active);
@@ -505,7 +548,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 // (uwshcu.F90:1945-1990 and :4383-4433)
 #define PUT_DIAG_LEVEL()                                                                                  \
     if (A.diag_level) {                                                                                   \
-        for (int k = 0; k <= mkx; k++) {                                                                  \
+        _Pragma("unroll 1") for (int k = 0; k <= mkx; k++) {                                              \
             DLV(UW_DL_UFRC, k) = tl_val(ufrc[k]);                                                                 \
             DLV(UW_DL_QTU, k) = tl_val(qtu[k]);                                                                   \
             DLV(UW_DL_THLU, k) = tl_val(thlu[k]);                                                                 \
@@ -516,8 +559,8 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             DLV(UW_DL_FLXRAIN, k) = tl_val(flxrain[k]);                                                           \
             DLV(UW_DL_FLXSNOW, k) = tl_val(flxsnow[k]);                                                           \
         }                                                                                                 \
-        for (int j = UW_DL_FER; j < UW_NDL; j++) DLV(j, 0) = tl_val(0.0);                                         \
-        for (int k = 1; k <= mkx; k++) {                                                                  \
+        _Pragma("unroll 1") for (int j = UW_DL_FER; j < UW_NDL; j++) DLV(j, 0) = tl_val(0.0);                     \
+        _Pragma("unroll 1") for (int k = 1; k <= mkx; k++) {                                              \
             DLV(UW_DL_FER, k) = tl_val(fer[k]);                                                                   \
             DLV(UW_DL_FDR, k) = tl_val(fdr[k]);                                                                   \
             DLV(UW_DL_DWTEN, k) = tl_val(dwten[k]);                                                               \
@@ -540,6 +583,9 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     Tl qlten[KP], qiten[KP], qvten[KP], sten[KP], qc[KP], qc_l[KP], qc_i[KP], evapc[KP];
     Tl flxrain[KP], flxsnow[KP], cufrc[KP], qcu[KP], qlu[KP], qiu[KP], trten[NC][KP];
     Tl qw0[KP], trflx_d[KP], trflx_u[KP];
+#if !UW_TAPE_ORDER
+    Tl qltop[KP], qitop[KP];
+#endif
     Tl trsrc[NC], tre[NC];
 
     unsigned int errbits = 0;
@@ -560,7 +606,8 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     Tl cbmf = 0, wlcl = 0, ufrclcl = 0, ppen = 0, precip = 0, snow = 0, rliq = 0, cush, cnt, cnb;
     Tl thlu_top = 0, qtu_top = 0, exntop = 1.0, drage = 0, bogbot = 0, bogtop = 0, rho0j = 0,
            wtwb = 0, wtw = 0, xs1 = 0, xs2 = 0, xc1 = 0, xc2 = 0;
-    Tl thj = 0, qvj = 0, qlj = 0, qij = 0;
+    Tl thj = 0, qvj = 0, qlj = 0, qij = 0, rvj = 0;
+    (void)rvj;
     Tl rainflx = 0, snowflx = 0;
     (void)kinv_o_d;
     const Tl pblh = Tl(__ldg(&A.pblh[i]), T.dpblh ? __ldg(&T.dpblh[i]) : 0.0);
@@ -571,6 +618,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 
     // ---- output initialisation (uwshcu.F90:1087-1124) ------------------------------------------
     if (MODE != UW_MODE_TRIGGER) {
+#pragma unroll 1
     for (int k = 0; k <= mkx; k++) {
         { const Tl v_ = (0.0); OI(umf, k) = tl_val(v_); TOI(umf, k) = tl_der(v_); }
         { const Tl v_ = (0.0); OI(slflx, k) = tl_val(v_); TOI(slflx, k) = tl_der(v_); }
@@ -579,11 +627,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         { const Tl v_ = (0.0); OI(flxsnow1, k) = tl_val(v_); TOI(flxsnow1, k) = tl_der(v_); }
         { const Tl v_ = (0.0); OI(wu, k) = tl_val(v_); TOI(wu, k) = tl_der(v_); }
     }
+#pragma unroll 1
     for (int k = 1; k <= mkx; k++) {
         { const Tl v_ = (0.0); OL(qvten, k) = tl_val(v_); TOL(qvten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qlten, k) = tl_val(v_); TOL(qlten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qiten, k) = tl_val(v_); TOL(qiten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(sten, k) = tl_val(v_); TOL(sten, k) = tl_der(v_); }
         { const Tl v_ = (0.0); OL(uten, k) = tl_val(v_); TOL(uten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(vten, k) = tl_val(v_); TOL(vten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qrten, k) = tl_val(v_); TOL(qrten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qsten, k) = tl_val(v_); TOL(qsten, k) = tl_der(v_); }
         { const Tl v_ = (0.0); OL(evapc, k) = tl_val(v_); TOL(evapc, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(cufrc, k) = tl_val(v_); TOL(cufrc, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qcu, k) = tl_val(v_); TOL(qcu, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qlu, k) = tl_val(v_); TOL(qlu, k) = tl_der(v_); }
         { const Tl v_ = (0.0); OL(qiu, k) = tl_val(v_); TOL(qiu, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qc, k) = tl_val(v_); TOL(qc, k) = tl_der(v_); }
+#pragma unroll 1
         for (int m = 1; m <= ncnst; m++) { const Tl v_ = (0.0); OT(m, k) = tl_val(v_); TOT(m, k) = tl_der(v_); }
     }
     { const Tl v_ = (0.0); A.precip[i] = tl_val(v_); T.precip[i] = tl_der(v_); }
@@ -601,12 +651,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     // only that status bit (no findsp at or above the bad level, no conden).  The values are checked
     // as they are loaded; z0 and tke, which the scheme reads later and only at some levels, once here.
     bool nonfinite = !uw_isfinite(pblh) || !uw_isfinite(A.cush[i]);
+#pragma unroll 1
     for (int k = 0; k <= mkx; k++) {
         ps0[k] = GI(ps0, k);
         zs0[k] = GI(zs0, k);
         nonfinite |= !uw_isfinite(ps0[k]) || !uw_isfinite(zs0[k]) || !uw_isfinite(GI(tke, k));
         exns0[k] = uw_pow(ps0[k] / p00, rovcp);
     }
+#pragma unroll 1
     for (int k = 1; k <= mkx; k++) {
         p0[k] = GL(p0, k);
         dp0[k] = GL(dp0, k);
@@ -627,17 +679,21 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         Tl tmpf[KP];
         slope<KP>(mkx, thl0, p0, ssthl0);
         slope<KP>(mkx, qt0, p0, ssqt0);
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             tmpf[k] = GL(u0, k);
             nonfinite |= !uw_isfinite(tmpf[k]);
         }
         slope<KP>(mkx, tmpf, p0, ssu0);
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             tmpf[k] = GL(v0, k);
             nonfinite |= !uw_isfinite(tmpf[k]);
         }
         slope<KP>(mkx, tmpf, p0, ssv0);
+#pragma unroll 1
         for (int m = 1; m <= ncnst; m++) {
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {
                 tmpf[k] = GT(m, k);
                 nonfinite |= !uw_isfinite(tmpf[k]);
@@ -652,10 +708,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         stop = true;
     }
     // thv0 at layer bottom/top (:1275-1299)
+#pragma unroll 1
     for (int k = 1; k <= mkx && !nonfinite; k++) {
         Tl thl0bot = thl0[k] + ssthl0[k] * (ps0[k - 1] - p0[k]);
         Tl qt0bot = qt0[k] + ssqt0[k] * (ps0[k - 1] - p0[k]);
-        if (CONDEN(ps0[k - 1], exns0[k - 1], thl0bot, qt0bot, thj, qvj, qlj, qij, tbl)) {
+        if (CONDEN(ps0[k - 1], exns0[k - 1], thl0bot, qt0bot, thj, qvj, qlj, qij, rvj, tbl)) {
             xflags |= UW_X_CONDEN;
             id_exit = true;
             stop = true;
@@ -665,7 +722,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         thvl0bot[k] = thl0bot * (1.0 + zvir * qt0bot);
         Tl thl0top = thl0[k] + ssthl0[k] * (ps0[k] - p0[k]);
         Tl qt0top = qt0[k] + ssqt0[k] * (ps0[k] - p0[k]);
-        if (CONDEN(ps0[k], exns0[k], thl0top, qt0top, thj, qvj, qlj, qij, tbl)) {
+        if (CONDEN(ps0[k], exns0[k], thl0top, qt0top, thj, qvj, qlj, qij, rvj, tbl)) {
             xflags |= UW_X_CONDEN;
             id_exit = true;
             stop = true;
@@ -680,16 +737,19 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     }
     if (!stop) {
     // per-column initialisation (:1333-1408)
+#pragma unroll 1
     for (int k = 0; k <= mkx; k++) {
         umf[k] = 0.0; emf[k] = 0.0; slflx[k] = 0.0; qtflx[k] = 0.0; uflx[k] = 0.0; vflx[k] = 0.0;
         ufrc[k] = 0.0; thlu[k] = 0.0; qtu[k] = 0.0; uu[k] = 0.0; vu[k] = 0.0; wu[k] = 0.0;
         thvu[k] = 0.0; thlu_emf[k] = 0.0; qtu_emf[k] = 0.0; uu_emf[k] = 0.0; vu_emf[k] = 0.0;
+#pragma unroll 1
         for (int m = 0; m < ncnst; m++) {
             trflx[m][k] = 0.0;
             tru[m][k] = 0.0;
             tru_emf[m][k] = 0.0;
         }
     }
+#pragma unroll 1
     for (int k = 1; k <= mkx; k++) {
         qvten[k] = 0.0; qlten[k] = 0.0; qiten[k] = 0.0; sten[k] = 0.0; uten[k] = 0.0; vten[k] = 0.0;
         qrten[k] = 0.0; qsten[k] = 0.0; dwten[k] = 0.0; diten[k] = 0.0; evapc[k] = 0.0;
@@ -697,6 +757,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         qc[k] = 0.0; qc_l[k] = 0.0; qc_i[k] = 0.0; qtten[k] = 0.0; slten[k] = 0.0;
         qlten_sink[k] = 0.0; qiten_sink[k] = 0.0; nlten_sink[k] = 0.0; niten_sink[k] = 0.0;
         rei[k] = 0.0; uf[k] = 0.0; vf[k] = 0.0;
+#pragma unroll 1
         for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0;
     }
     cnt = (Tl)mkx;
@@ -706,25 +767,32 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         // the state UW_MODE_LIST1 stored at the implicit-CIN branch of iteration 2 (uw_state.cuh),
         // and the arrays that the set-up and that branch's restore build from the inputs, rebuilt
         // with the same operations
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             ps0[k] = GI(ps0, k);
             zs0[k] = GI(zs0, k);
         }
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             p0[k] = GL(p0, k);
             dp0[k] = GL(dp0, k);
         }
         {
             Tl tmpf[KP];
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) tmpf[k] = GL(u0, k);
             slope<KP>(mkx, tmpf, p0, ssu0);
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) tmpf[k] = GL(v0, k);
             slope<KP>(mkx, tmpf, p0, ssv0);
+#pragma unroll 1
             for (int m = 1; m <= ncnst; m++) {
+#pragma unroll 1
                 for (int k = 1; k <= mkx; k++) tmpf[k] = GT(m, k);
                 slope<KP>(mkx, tmpf, p0, sstr0[m - 1]);
             }
         }
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             qv0[k] = SEEDL(qv0, dqv0, k);
             ql0[k] = GL(ql0, k);
@@ -740,23 +808,27 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         }
         slope<KP>(mkx, thl0, p0, ssthl0);
         slope<KP>(mkx, qt0, p0, ssqt0);
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             umf[k] = 0.0; emf[k] = 0.0; slflx[k] = 0.0; qtflx[k] = 0.0; uflx[k] = 0.0;
             vflx[k] = 0.0; ufrc[k] = 0.0; thlu[k] = 0.0; qtu[k] = 0.0; uu[k] = 0.0;
             vu[k] = 0.0; wu[k] = 0.0; thvu[k] = 0.0; thlu_emf[k] = 0.0; qtu_emf[k] = 0.0;
             uu_emf[k] = 0.0; vu_emf[k] = 0.0;
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++) {
                 trflx[m][k] = 0.0;
                 tru[m][k] = 0.0;
                 tru_emf[m][k] = 0.0;
             }
         }
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             qvten[k] = 0.0; qlten[k] = 0.0; qiten[k] = 0.0; sten[k] = 0.0; uten[k] = 0.0;
             vten[k] = 0.0; qrten[k] = 0.0; qsten[k] = 0.0; dwten[k] = 0.0; diten[k] = 0.0;
             evapc[k] = 0.0; cufrc[k] = 0.0; qcu[k] = 0.0; qlu[k] = 0.0; qiu[k] = 0.0;
             fer[k] = 0.0; fdr[k] = 0.0; qc[k] = 0.0; qc_l[k] = 0.0; qc_i[k] = 0.0;
             qtten[k] = 0.0; slten[k] = 0.0;
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0;
         }
     }
@@ -771,6 +843,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     // sections.  (Lanes that leave a loop at different iterations otherwise run apart for the rest
     // of the column: the worklist kernel ran with 1.9 of 32 lanes active.)  Loops marked `uniform`
     // have the same trip count on every live lane; UW_SYNC() appears only directly inside them.
+#pragma unroll 1
     for (int iter = (MODE == UW_MODE_RESUME ? 2 : 1); iter <= (MODE == UW_MODE_TRIGGER ? 1 : 2); iter++) {   // uniform
         Tl tscaleh = tscaleh_r;
         if constexpr (MODE != UW_MODE_RESUME) {   // uniform
@@ -782,6 +855,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         kinv = 1;
         {
             bool found = false;
+#pragma unroll 1
             for (int k = mkx - 1; k >= 1; k--) {
                 if (!found && (pblh + 5.0 - zs0[k]) * (pblh + 5.0 - zs0[k + 1]) < 0.0) {
                     kinv = k + 1;
@@ -800,6 +874,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             Tl dpsum = 0.0;
             tkeavg = 0.0;
             thvlmin = 1000.0;
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 if (k > kinv - 1) continue;
                 Tl dpi;
@@ -818,6 +893,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         thlsrc = thvlsrc / (1.0 + zvir * qtsrc);
         usrc = GL(u0, kinv - 1) + ssu0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
         vsrc = GL(v0, kinv - 1) + ssv0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
+#pragma unroll 1
         for (int m = 1; m <= ncnst; m++) trsrc[m - 1] = GT(m, 1);
         } while (0);
         UW_SYNC();
@@ -827,6 +903,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         klcl = mkx;
         {
             bool found = false;
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 if (!found && ps0[k] < plcl) {
                     klcl = k;
@@ -845,7 +922,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         {
             Tl thl0lcl = thl0[klcl] + ssthl0[klcl] * (plcl - p0[klcl]);
             Tl qt0lcl = qt0[klcl] + ssqt0[klcl] * (plcl - p0[klcl]);
-            if (CONDEN(plcl, exlcl, thl0lcl, qt0lcl, thj, qvj, qlj, qij, tbl)) {
+            if (CONDEN(plcl, exlcl, thl0lcl, qt0lcl, thj, qvj, qlj, qij, rvj, tbl)) {
                 xflags |= UW_X_CONDEN;
                 id_exit = true;
                 stop = true;
@@ -870,6 +947,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             const bool lcl_above = (klcl >= kinv);
             Tl thvubot = 0.0, thvutop = 0.0;
             bool ldone = stop;
+#pragma unroll 1
             for (int k = 2; k <= mkx - 1; k++) {   // uniform (kinv >= 2)
                 if (!ldone && k >= kinv) do {
                     if (lcl_above && k < klcl) {
@@ -879,7 +957,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                         break;
                     }
                     if (!lcl_above && k == kinv) {
-                        if (CONDEN(ps0[k - 1], exns0[k - 1], thlsrc, qtsrc, thj, qvj, qlj, qij, tbl)) {
+                        if (CONDEN(ps0[k - 1], exns0[k - 1], thlsrc, qtsrc, thj, qvj, qlj, qij, rvj, tbl)) {
                             xflags |= UW_X_CONDEN;
                             id_exit = true;
                             stop = true;
@@ -899,7 +977,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     } else {
                         thvubot = thvutop;
                     }
-                    if (CONDEN(ps0[k], exns0[k], thlsrc, qtsrc, thj, qvj, qlj, qij, tbl)) {
+                    if (CONDEN(ps0[k], exns0[k], thlsrc, qtsrc, thj, qvj, qlj, qij, rvj, tbl)) {
                         xflags |= UW_X_CONDEN;
                         id_exit = true;
                         stop = true;
@@ -935,6 +1013,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             kinv_o = kinv; klcl_o = klcl; klfc_o = klfc; plcl_o = plcl; plfc_o = plfc;
             tkeavg_o = tkeavg; thvlmin_o = thvlmin; qtsrc_o = qtsrc; thvlsrc_o = thvlsrc;
             thlsrc_o = thlsrc; usrc_o = usrc; vsrc_o = vsrc; thv0lcl_o = thv0lcl;
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++) trsrc_o[m] = trsrc[m];
         } else {
             Tl del_CIN = cin - cin_i;
@@ -946,8 +1025,10 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 kinv = kinv_o; klcl = klcl_o; klfc = klfc_o; plcl = plcl_o; plfc = plfc_o;
                 tkeavg = tkeavg_o; thvlmin = thvlmin_o; qtsrc = qtsrc_o; thvlsrc = thvlsrc_o;
                 thlsrc = thlsrc_o; usrc = usrc_o; vsrc = vsrc_o; thv0lcl = thv0lcl_o;
+#pragma unroll 1
                 for (int m = 0; m < ncnst; m++) trsrc[m] = trsrc_o[m];
                 exlcl = exnf(plcl);
+#pragma unroll 1
                 for (int k = 1; k <= mkx; k++) {
                     qv0[k] = SEEDL(qv0, dqv0, k);
                     ql0[k] = GL(ql0, k);
@@ -963,23 +1044,27 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 }
                 slope<KP>(mkx, thl0, p0, ssthl0);
                 slope<KP>(mkx, qt0, p0, ssqt0);
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) {
                     umf[k] = 0.0; emf[k] = 0.0; slflx[k] = 0.0; qtflx[k] = 0.0; uflx[k] = 0.0;
                     vflx[k] = 0.0; ufrc[k] = 0.0; thlu[k] = 0.0; qtu[k] = 0.0; uu[k] = 0.0;
                     vu[k] = 0.0; wu[k] = 0.0; thvu[k] = 0.0; thlu_emf[k] = 0.0; qtu_emf[k] = 0.0;
                     uu_emf[k] = 0.0; vu_emf[k] = 0.0;
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++) {
                         trflx[m][k] = 0.0;
                         tru[m][k] = 0.0;
                         tru_emf[m][k] = 0.0;
                     }
                 }
+#pragma unroll 1
                 for (int k = 1; k <= mkx; k++) {
                     qvten[k] = 0.0; qlten[k] = 0.0; qiten[k] = 0.0; sten[k] = 0.0; uten[k] = 0.0;
                     vten[k] = 0.0; qrten[k] = 0.0; qsten[k] = 0.0; dwten[k] = 0.0; diten[k] = 0.0;
                     evapc[k] = 0.0; cufrc[k] = 0.0; qcu[k] = 0.0; qlu[k] = 0.0; qiu[k] = 0.0;
                     fer[k] = 0.0; fdr[k] = 0.0; qc[k] = 0.0; qc_l[k] = 0.0; qc_i[k] = 0.0;
                     qtten[k] = 0.0; slten[k] = 0.0;
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0;
                 }
                 precip = 0.0; snow = 0.0; rliq = 0.0; cbmf = 0.0;
@@ -988,6 +1073,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 // explicit CIN: the iteration-1 outputs already sit in the output slots (:1891-2011);
                 // flxprc1/flxsnow1 keep their initial zeros on this path, wu_out gets wu.
                 lflags |= UW_L_DELCIN;
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) { const Tl v_ = (wu[k]); OI(wu, k) = tl_val(v_); TOI(wu, k) = tl_der(v_); }
                 if (A.diag_real) {
                     A.diag_real[UW_DR_CIN * (size_t)mix + i] = tl_val(cin_s);
@@ -1098,6 +1184,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             break;
             }
             ufrc[krel - 1] = ufrclcl;
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 if (k < kinv - 1 || k > krel - 1) continue;
                 umf[k] = cbmf;
@@ -1114,6 +1201,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         }
         UW_SYNC();
         if (MODE != UW_MODE_TRIGGER) {   // uniform
+#if !UW_TAPE_ORDER
+        // Condensate of the final updraft at the release level, at the interfaces above it (qltop, qitop)
+        // and at the cumulus top; id_top: the adjustment at the top did not close.  The tendencies and
+        // the in-cloud diagnostics need it again; the Fortran repeats the conden calls there, with the
+        // same arguments.
+        Tl ql_rel = 0.0, qi_rel = 0.0, ql_top = 0.0, qi_top = 0.0;
+        bool id_top = false;
+#endif
         // updraft at the release level (:2205-2236)
         if (!stop) do {
         emf[krel - 1] = 0.0;
@@ -1121,19 +1216,24 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         wu[krel - 1] = wlcl;
         thlu[krel - 1] = thlsrc;
         qtu[krel - 1] = qtsrc;
-        if (CONDEN(prel, exprel, thlsrc, qtsrc, thj, qvj, qlj, qij, tbl)) {
+        if (CONDEN(prel, exprel, thlsrc, qtsrc, thj, qvj, qlj, qij, rvj, tbl)) {
             xflags |= UW_X_CONDEN;
             id_exit = true;
             stop = true;
             break;
         }
         thvu[krel - 1] = thj * (1.0 + zvir * qvj - qlj - qij);
+#if !UW_TAPE_ORDER
+        ql_rel = qlj;
+        qi_rel = qij;
+#endif
         {
             Tl uplus = 0.0, vplus = 0.0;
             if (krel == kinv) {
                 uplus = PGFc * ssu0[kinv] * (prel - ps0[kinv - 1]);
                 vplus = PGFc * ssv0[kinv] * (prel - ps0[kinv - 1]);
             } else {
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) {
                     if (k < kinv || k > MX(krel - 1, kinv)) continue;
                     uplus = uplus + PGFc * ssu0[k] * (ps0[k] - ps0[k - 1]);
@@ -1145,6 +1245,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             uu[krel - 1] = usrc + uplus;
             vu[krel - 1] = vsrc + vplus;
         }
+#pragma unroll 1
         for (int m = 0; m < ncnst; m++) tru[m][krel - 1] = trsrc[m];
         } while (0);
         UW_SYNC();
@@ -1153,8 +1254,18 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             Tl scaleh = tscaleh;
             if (tscaleh < 0.0) scaleh = 1000.0;
             // ---- buoyancy-sorting updraft, iter_scaleh loop (:2306-2952) ----------------------
+#pragma unroll 1
             for (int iter_scaleh = 1; iter_scaleh <= 3; iter_scaleh++) {   // uniform
                 Tl pe = 0.0, dpe = 0.0, exne = 1.0, thvebot = 0.0, thle = 0.0, qte = 0.0, ue = 0.0, ve = 0.0;
+#if !UW_TAPE_ORDER
+                // The first two passes only find the scale height: the winds and tracers of the updraft feed
+                // nothing back into it, and of the level profiles only wu (an output at every level) and
+                // fer outlive the pass, so the last pass alone computes and stores the rest.  (The
+                // per-level diagnostics also show what an earlier, deeper pass left above the cloud top.)
+                const bool full = iter_scaleh == 3 || A.diag_level != nullptr;
+                // the updraft at the level below
+                Tl thlu_b = 0.0, qtu_b = 0.0, thvu_b = 0.0, umf_b = 0.0;
+#endif
                 if (!stop) {
                     kbup = krel;
                     kpen = krel;
@@ -1165,13 +1276,26 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     thvebot = thv0rel;
                     thle = thl0[krel] + ssthl0[krel] * (pe - p0[krel]);
                     qte = qt0[krel] + ssqt0[krel] * (pe - p0[krel]);
+#if !UW_TAPE_ORDER
+                    thlu_b = thlu[krel - 1];
+                    qtu_b = qtu[krel - 1];
+                    thvu_b = thvu[krel - 1];
+                    umf_b = umf[krel - 1];
+                    if (full) {   // uniform
+#endif
                     ue = GL(u0, krel) + ssu0[krel] * (pe - p0[krel]);
                     ve = GL(v0, krel) + ssv0[krel] * (pe - p0[krel]);
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, krel) + sstr0[m][krel] * (pe - p0[krel]);
+#if !UW_TAPE_ORDER
+                    }
+#endif
                 }
 
+#if UW_TAPE_ORDER
                 // levels k = krel .. mkx-1, taken by every lane as k = krel + j
                 bool ldone = stop;
+#pragma unroll 1
                 for (int j = 0; j <= mkx - 2; j++) {   // uniform
                     const int k = krel + j;
                     if (k > mkx - 1) ldone = true;
@@ -1185,11 +1309,12 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     // environment at the layer midpoint: the same in both iter_xc passes, so the
                     // second pass reuses the first one's conden and qsat results (same bits)
                     Tl thv0j = 0.0, excess0 = 0.0;
+#pragma unroll 1
                     for (int iter_xc = 1; iter_xc <= 2; iter_xc++) {
                         if (!xdone && !stop) do {
                         wtw = wu[km1] * wu[km1];
                         if (iter_xc == 1) {
-                            if (CONDEN(pe, exne, thle, qte, thj, qvj, qlj, qij, tbl)) {
+                            if (CONDEN(pe, exne, thle, qte, thj, qvj, qlj, qij, rvj, tbl)) {
                                 xflags |= UW_X_CONDEN;
                                 id_exit = true;
                                 stop = true;
@@ -1199,7 +1324,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             excess0 = qte - qsat_qs(thle * exne, pe, tbl);
                         }
                         rho0j = pe / (r * thv0j * exne);
-                        if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, tbl)) {
+                        if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, rvj, tbl)) {
                             xflags |= UW_X_CONDEN;
                             id_exit = true;
                             stop = true;
@@ -1212,7 +1337,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             Tl exqi = ((qlj + qij) - criqc) * qij / (qlj + qij);
                             qtue = qtue - exql - exqi;
                             thlue = thlue + (xlv / cp / exne) * exql + (xls / cp / exne) * exqi;
-                            if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, tbl)) {
+                            if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, rvj, tbl)) {
                                 xflags |= UW_X_CONDEN;
                                 id_exit = true;
                                 stop = true;
@@ -1229,7 +1354,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             Tl xsat = excessu / (excessu - excess0);
                             Tl thlxsat = thlue + xsat * (thle - thlue);
                             Tl qtxsat = qtue + xsat * (qte - qtue);
-                            if (CONDEN(pe, exne, thlxsat, qtxsat, thj, qvj, qlj, qij, tbl)) {
+                            if (CONDEN(pe, exne, thlxsat, qtxsat, thj, qvj, qlj, qij, rvj, tbl)) {
                                 xflags |= UW_X_CONDEN;
                                 id_exit = true;
                                 stop = true;
@@ -1237,6 +1362,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             }
                             Tl thvxsat = thj * (1.0 + zvir * qvj - qlj - qij);
                             Tl x_cu = 0.0, x_en = 0.0;
+#pragma unroll 1
                             for (int kk = 1; kk <= 2; kk++) {
                                 Tl thv_x0, thv_x1;
                                 if (kk == 1) {
@@ -1289,6 +1415,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             qtu[k] = qtu[km1] + (qte + ssqt0[k] * dpe / 2.0 - qtu[km1]) * fer[k] * dpe;
                             uu[k] = uu[km1] + (ue + ssu0[k] * dpe / 2.0 - uu[km1]) * fer[k] * dpe - PGFc * ssu0[k] * dpe;
                             vu[k] = vu[km1] + (ve + ssv0[k] * dpe / 2.0 - vu[km1]) * fer[k] * dpe - PGFc * ssv0[k] * dpe;
+#pragma unroll 1
                             for (int m = 0; m < ncnst; m++)
                                 tru[m][k] = tru[m][km1] + (tre[m] + sstr0[m][k] * dpe / 2.0 - tru[m][km1]) * fer[k] * dpe;
                         } else {
@@ -1301,11 +1428,12 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                                     (ue + ssu0[k] * dpe / 2.0 - uu[km1] + (1.0 - PGFc) * ssu0[k] / fer[k]) * ef;
                             vu[k] = (ve + (1.0 - PGFc) * ssv0[k] / fer[k] - ssv0[k] * dpe / 2.0) -
                                     (ve + ssv0[k] * dpe / 2.0 - vu[km1] + (1.0 - PGFc) * ssv0[k] / fer[k]) * ef;
+#pragma unroll 1
                             for (int m = 0; m < ncnst; m++)
                                 tru[m][k] = (tre[m] + sstr0[m][k] / fer[k] - sstr0[m][k] * dpe / 2.0) -
                                             (tre[m] + sstr0[m][k] * dpe / 2.0 - tru[m][km1] + sstr0[m][k] / fer[k]) * ef;
                         }
-                        if (CONDEN(ps0[k], exns0[k], thlu[k], qtu[k], thj, qvj, qlj, qij, tbl)) {
+                        if (CONDEN(ps0[k], exns0[k], thlu[k], qtu[k], thj, qvj, qlj, qij, rvj, tbl)) {
                             xflags |= UW_X_CONDEN;
                             id_exit = true;
                             stop = true;
@@ -1318,7 +1446,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             thlu[k] = thlu[k] + (xlv / cp / exns0[k]) * exql + (xls / cp / exns0[k]) * exqi;
                             dwten[k] = exql;
                             diten[k] = exqi;
-                            if (CONDEN(ps0[k], exns0[k], thlu[k], qtu[k], thj, qvj, qlj, qij, tbl)) {
+                            if (CONDEN(ps0[k], exns0[k], thlu[k], qtu[k], thj, qvj, qlj, qij, rvj, tbl)) {
                                 xflags |= UW_X_CONDEN;
                                 id_exit = true;
                                 stop = true;
@@ -1383,14 +1511,286 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     qte = qt0[k + 1];
                     ue = GL(u0, k + 1);
                     ve = GL(v0, k + 1);
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, k + 1);
                     } while (0);
                     if (stop) ldone = true;
                     UW_SYNC();
                 }
+#else
+                // levels k = krel .. mkx-1, taken by every lane as k = krel + j
+                bool ldone = stop;
+#pragma unroll 1
+                for (int j = 0; j <= mkx - 2; j++) {   // uniform
+                    const int k = krel + j;
+                    if (k > mkx - 1) ldone = true;
+                    if (!ldone) do {
+                    const Tl wu_b = wu[k - 1];   // (carried like the others, the FMA-contracted modes would round
+                                                     // wu_b * wu_b with what follows it)
+                    Tl thlue = thlu_b;
+                    Tl qtue = qtu_b;
+                    Tl wue = wu_b;
+                    wtwb = wtw;
+                    bool xdone = false;
+                    // environment at the layer midpoint: the same in both iter_xc passes, so the
+                    // second pass reuses the first one's results (same bits)
+                    Tl thv0j = 0.0, excess0 = 0.0, reib = 0.0;
+                    Tl thlu_k = 0.0, qtu_k = 0.0, thvu_k = 0.0, fer_k = 0.0, fdr_k = 0.0, rei_k = 0.0, ef_k = 0.0,
+                           dmf_k = 0.0, dw_k = 0.0, di_k = 0.0;
+                    const Tl cridis = rle * scaleh;
+#pragma unroll 1
+                    for (int iter_xc = 1; iter_xc <= 2; iter_xc++) {
+                        if (!xdone && !stop) do {
+                        wtw = wu_b * wu_b;
+                        if (iter_xc == 1) {
+                            if (CONDEN(pe, exne, thle, qte, thj, qvj, qlj, qij, rvj, tbl)) {
+                                xflags |= UW_X_CONDEN;
+                                id_exit = true;
+                                stop = true;
+                                break;
+                            }
+                            thv0j = thj * (1.0 + zvir * qvj - qlj - qij);
+                            excess0 = qte - UW_QSAT_OF_CONDEN(thle * exne, pe);
+                            rho0j = pe / (r * thv0j * exne);
+                            reib = (0.5 * rkm / GL(z0, k) / g / rho0j);
+                        }
+                        if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, rvj, tbl)) {
+                            xflags |= UW_X_CONDEN;
+                            id_exit = true;
+                            stop = true;
+                            break;
+                        }
+                        // condensate above criqc leaves the updraft; without it the Fortran's
+                        // second conden call repeats the first one's arguments and results
+                        if ((qlj + qij) > criqc) {
+                            Tl exql = ((qlj + qij) - criqc) * qlj / (qlj + qij);
+                            Tl exqi = ((qlj + qij) - criqc) * qij / (qlj + qij);
+                            qtue = qtue - exql - exqi;
+                            thlue = thlue + (xlv / cp / exne) * exql + (xls / cp / exne) * exqi;
+                            if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, rvj, tbl)) {
+                                xflags |= UW_X_CONDEN;
+                                id_exit = true;
+                                stop = true;
+                                break;
+                            }
+                        }
+                        Tl thvj = thj * (1.0 + zvir * qvj - qlj - qij);
+                        Tl excessu = qtue - UW_QSAT_OF_CONDEN(thlue * exne, pe);
+                        Tl xc;
+                        if ((excessu <= 0.0 && excess0 <= 0.0) || (excessu >= 0.0 && excess0 >= 0.0)) {
+                            xc = MN(1.0, MX(0.0, 1.0 - 2.0 * rbuoy * g * cridis / (wue * wue) * (1.0 - thvj / thv0j)));
+                        } else {
+                            Tl xsat = excessu / (excessu - excess0);
+                            Tl thlxsat = thlue + xsat * (thle - thlue);
+                            Tl qtxsat = qtue + xsat * (qte - qtue);
+                            if (CONDEN(pe, exne, thlxsat, qtxsat, thj, qvj, qlj, qij, rvj, tbl)) {
+                                xflags |= UW_X_CONDEN;
+                                id_exit = true;
+                                stop = true;
+                                break;
+                            }
+                            Tl thvxsat = thj * (1.0 + zvir * qvj - qlj - qij);
+                            Tl x_cu = 0.0, x_en = 0.0;
+#pragma unroll 1
+                            for (int kk = 1; kk <= 2; kk++) {
+                                Tl thv_x0, thv_x1;
+                                if (kk == 1) {
+                                    thv_x0 = thvj;
+                                    thv_x1 = (1.0 - 1.0 / xsat) * thvj + (1.0 / xsat) * thvxsat;
+                                } else {
+                                    thv_x1 = thv0j;
+                                    thv_x0 = (xsat / (xsat - 1.0)) * thv0j + (1.0 / (1.0 - xsat)) * thvxsat;
+                                }
+                                Tl aquad = wue * wue;
+                                Tl bquad = 2.0 * rbuoy * g * cridis * (thv_x1 - thv_x0) / thv0j - 2.0 * (wue * wue);
+                                Tl cquad = 2.0 * rbuoy * g * cridis * (thv_x0 - thv0j) / thv0j + (wue * wue);
+                                if (kk == 1) {
+                                    if ((bquad * bquad - 4.0 * aquad * cquad) >= 0.0) {
+                                        roots(aquad, bquad, cquad, xs1, xs2);
+                                        x_cu = MN(1.0, MX(0.0, MN(xsat, MN(xs1, xs2))));
+                                    } else {
+                                        x_cu = xsat;
+                                    }
+                                } else {
+                                    if ((bquad * bquad - 4.0 * aquad * cquad) >= 0.0) {
+                                        roots(aquad, bquad, cquad, xs1, xs2);
+                                        x_en = MN(1.0, MX(0.0, MX(xsat, MN(xs1, xs2))));
+                                    } else {
+                                        x_en = 1.0;
+                                    }
+                                }
+                            }
+                            if (x_cu == xsat) xc = MX(x_cu, x_en);
+                            else xc = x_cu;
+                        }
+                        Tl ee2 = xc * xc;
+                        Tl ud2 = 1.0 - 2.0 * xc + xc * xc;
+                        rei_k = reib;
+                        if (xc > 0.5) rei_k = MN(rei_k, 0.9 * uw_log(dp0[k] / g / dt / umf_b + 1.0) / dpe / (2.0 * xc - 1.0));
+                        fer_k = rei_k * ee2;
+                        fdr_k = rei_k * ud2;
+                        // compute_zwshcu's entrainment option (zwshcu.F90:2818-2844)
+                        if (ZW && c.zw_ent) {
+                            bogbot = rbuoy * (thvu_b / thvebot - 1.0) * g;
+                            fer_k = c.zw_ent0 * bogbot / MX(wue * wue, 1.0e-4);
+                            Tl fer_min = 0.0;
+                            if (bogbot > 1.e-4) fer_min = 1.e-4;
+                            fer_k = MN(MX(fer_k, fer_min), 3.0e-2);
+                        }
+                        dmf_k = dpe * (fer_k - fdr_k);
+                        if (fer_k * dpe < 1.e-4) {
+                            thlu_k = thlu_b + (thle + ssthl0[k] * dpe / 2.0 - thlu_b) * fer_k * dpe;
+                            qtu_k = qtu_b + (qte + ssqt0[k] * dpe / 2.0 - qtu_b) * fer_k * dpe;
+                        } else {
+                            ef_k = uw_exp(-fer_k * dpe);
+                            thlu_k = (thle + ssthl0[k] / fer_k - ssthl0[k] * dpe / 2.0) -
+                                     (thle + ssthl0[k] * dpe / 2.0 - thlu_b + ssthl0[k] / fer_k) * ef_k;
+                            qtu_k = (qte + ssqt0[k] / fer_k - ssqt0[k] * dpe / 2.0) -
+                                    (qte + ssqt0[k] * dpe / 2.0 - qtu_b + ssqt0[k] / fer_k) * ef_k;
+                        }
+                        if (CONDEN(ps0[k], exns0[k], thlu_k, qtu_k, thj, qvj, qlj, qij, rvj, tbl)) {
+                            xflags |= UW_X_CONDEN;
+                            id_exit = true;
+                            stop = true;
+                            break;
+                        }
+                        if ((qlj + qij) > criqc) {
+                            Tl exql = ((qlj + qij) - criqc) * qlj / (qlj + qij);
+                            Tl exqi = ((qlj + qij) - criqc) * qij / (qlj + qij);
+                            qtu_k = qtu_k - exql - exqi;
+                            thlu_k = thlu_k + (xlv / cp / exns0[k]) * exql + (xls / cp / exns0[k]) * exqi;
+                            dw_k = exql;
+                            di_k = exqi;
+                            if (CONDEN(ps0[k], exns0[k], thlu_k, qtu_k, thj, qvj, qlj, qij, rvj, tbl)) {
+                                xflags |= UW_X_CONDEN;
+                                id_exit = true;
+                                stop = true;
+                                break;
+                            }
+                        } else {
+                            // nothing removed: the Fortran's second conden call repeats the first
+                            dw_k = 0.0;
+                            di_k = 0.0;
+                        }
+                        thvu_k = thj * (1.0 + zvir * qvj - qlj - qij);
+                        bogbot = rbuoy * (thvu_b / thvebot - 1.0);
+                        bogtop = rbuoy * (thvu_k / thv0top[k] - 1.0);
+                        Tl delbog = bogtop - bogbot;
+                        drage = fer_k * (1.0 + rdrag);
+                        Tl expfac = uw_exp(-2.0 * drage * dpe);
+                        wtwb = wtw;
+                        if (drage * dpe > 1.e-3)
+                            wtw = wtw * expfac + (delbog + (1.0 - expfac) * (bogbot + delbog / (-2.0 * drage * dpe))) / (rho0j * drage);
+                        else
+                            wtw = wtw + dpe * (bogbot + bogtop) / rho0j;
+                        if (wtw > 0.0) {
+                            thlue = 0.5 * (thlu_b + thlu_k);
+                            qtue = 0.5 * (qtu_b + qtu_k);
+                            wue = 0.5 * sqrt(MX(wtwb + wtw, 0.0));
+                        } else {
+                            xdone = true;   // go to 111
+                        }
+                        } while (0);
+                    }
+                    if (stop) break;
+                    fer[k] = fer_k;
+                    // the mass flux and, in the last pass, the level's profiles with the final fer and fdr
+                    // (the Fortran evaluates them in each iter_xc pass)
+                    Tl umf_k = umf_b * uw_exp(dmf_k);
+                    if (full) {
+                        const int km1 = k - 1;
+                        rei[k] = rei_k;
+                        thlu[k] = thlu_k;
+                        qtu[k] = qtu_k;
+                        thvu[k] = thvu_k;
+                        dwten[k] = dw_k;
+                        diten[k] = di_k;
+                        qltop[k] = qlj;
+                        qitop[k] = qij;
+                        if (fer_k * dpe < 1.e-4) {
+                            uu[k] = uu[km1] + (ue + ssu0[k] * dpe / 2.0 - uu[km1]) * fer_k * dpe - PGFc * ssu0[k] * dpe;
+                            vu[k] = vu[km1] + (ve + ssv0[k] * dpe / 2.0 - vu[km1]) * fer_k * dpe - PGFc * ssv0[k] * dpe;
+#pragma unroll 1
+                            for (int m = 0; m < ncnst; m++)
+                                tru[m][k] = tru[m][km1] + (tre[m] + sstr0[m][k] * dpe / 2.0 - tru[m][km1]) * fer_k * dpe;
+                        } else {
+                            uu[k] = (ue + (1.0 - PGFc) * ssu0[k] / fer_k - ssu0[k] * dpe / 2.0) -
+                                    (ue + ssu0[k] * dpe / 2.0 - uu[km1] + (1.0 - PGFc) * ssu0[k] / fer_k) * ef_k;
+                            vu[k] = (ve + (1.0 - PGFc) * ssv0[k] / fer_k - ssv0[k] * dpe / 2.0) -
+                                    (ve + ssv0[k] * dpe / 2.0 - vu[km1] + (1.0 - PGFc) * ssv0[k] / fer_k) * ef_k;
+#pragma unroll 1
+                            for (int m = 0; m < ncnst; m++)
+                                tru[m][k] = (tre[m] + sstr0[m][k] / fer_k - sstr0[m][k] * dpe / 2.0) -
+                                            (tre[m] + sstr0[m][k] * dpe / 2.0 - tru[m][km1] + sstr0[m][k] / fer_k) * ef_k;
+                        }
+                    }
+                    // (label 111, :2726-2793)
+                    if (umf_k == 0.0) wtw = -1.0;
+                    if (bogtop > 0.0 && wtw > 0.0) kbup = k;
+                    if (wtw <= 0.0) {
+                        kpen = k;
+                        ldone = true;
+                        if (full) {
+                            umf[k] = umf_k;
+                            fdr[k] = fdr_k;
+                        }
+                        break;   // go to 45
+                    }
+                    wu[k] = sqrt(wtw);
+                    if (wu[k] > 100.0) {
+                        xflags |= UW_X_WU;
+                        id_exit = true;
+                        stop = true;
+                        break;
+                    }
+                    {
+                        Tl rhos0j = ps0[k] / (r * 0.5 * (thv0bot[k + 1] + thv0top[k]) * exns0[k]);
+                        Tl ufrc_k = umf_k / (rhos0j * wu[k]);
+                        if (ufrc_k > rmaxfrac) {
+                            lflags |= UW_L_UFRC;
+                            ufrc_k = rmaxfrac;
+                            umf_k = rmaxfrac * rhos0j * wu[k];
+                            fdr_k = fer_k - uw_log(umf_k / umf_b) / dpe;
+                        }
+                        if (full) {
+                            ufrc[k] = ufrc_k;
+                            umf[k] = umf_k;
+                            fdr[k] = fdr_k;
+                        }
+                    }
+                    thlu_b = thlu_k;
+                    qtu_b = qtu_k;
+                    thvu_b = thvu_k;
+                    umf_b = umf_k;
+                    pe = p0[k + 1];
+                    dpe = dp0[k + 1];
+                    exne = exn0[k + 1];
+                    thvebot = thv0bot[k + 1];
+                    thle = thl0[k + 1];
+                    qte = qt0[k + 1];
+                    if (full) {
+                        ue = GL(u0, k + 1);
+                        ve = GL(v0, k + 1);
+#pragma unroll 1
+                        for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, k + 1);
+                    }
+                    } while (0);
+                    if (stop) ldone = true;
+                    UW_SYNC();
+                }
+#endif
                 UW_SYNC();
                 // (label 45) penetration depth (:2884-2907)
                 if (!stop) do {
+#if UW_TAPE_ORDER
+                const Tl thlu_b = thlu[kpen - 1], qtu_b = qtu[kpen - 1];
+#else
+                // the updraft at kpen - 1 (the release level's when no level stopped it: kpen = krel)
+                if (kpen == krel) {
+                    thlu_b = thlu[krel - 1];
+                    qtu_b = qtu[krel - 1];
+                }
+#endif
                 if (drage == 0.0) {
                     Tl aquad = (bogtop - bogbot) / (ps0[kpen] - ps0[kpen - 1]);
                     Tl bquad = 2.0 * bogbot;
@@ -1415,22 +1815,23 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 if (ppen == -dp0[kpen] || ppen == 0.0) lflags |= UW_L_PPEN;
                 // condensate at the cumulus top (:2917-2942)
                 if (fer[kpen] * (-ppen) < 1.e-4) {
-                    thlu_top = thlu[kpen - 1] + (thl0[kpen] + ssthl0[kpen] * (-ppen) / 2.0 - thlu[kpen - 1]) * fer[kpen] * (-ppen);
-                    qtu_top = qtu[kpen - 1] + (qt0[kpen] + ssqt0[kpen] * (-ppen) / 2.0 - qtu[kpen - 1]) * fer[kpen] * (-ppen);
+                    thlu_top = thlu_b + (thl0[kpen] + ssthl0[kpen] * (-ppen) / 2.0 - thlu_b) * fer[kpen] * (-ppen);
+                    qtu_top = qtu_b + (qt0[kpen] + ssqt0[kpen] * (-ppen) / 2.0 - qtu_b) * fer[kpen] * (-ppen);
                 } else {
                     const Tl ef = uw_exp(-fer[kpen] * (-ppen));
                     thlu_top = (thl0[kpen] + ssthl0[kpen] / fer[kpen] - ssthl0[kpen] * (-ppen) / 2.0) -
-                               (thl0[kpen] + ssthl0[kpen] * (-ppen) / 2.0 - thlu[kpen - 1] + ssthl0[kpen] / fer[kpen]) * ef;
+                               (thl0[kpen] + ssthl0[kpen] * (-ppen) / 2.0 - thlu_b + ssthl0[kpen] / fer[kpen]) * ef;
                     qtu_top = (qt0[kpen] + ssqt0[kpen] / fer[kpen] - ssqt0[kpen] * (-ppen) / 2.0) -
-                              (qt0[kpen] + ssqt0[kpen] * (-ppen) / 2.0 - qtu[kpen - 1] + ssqt0[kpen] / fer[kpen]) * ef;
+                              (qt0[kpen] + ssqt0[kpen] * (-ppen) / 2.0 - qtu_b + ssqt0[kpen] / fer[kpen]) * ef;
                 }
                 exntop = uw_pow((ps0[kpen - 1] + ppen) / p00, rovcp);
-                if (CONDEN(ps0[kpen - 1] + ppen, exntop, thlu_top, qtu_top, thj, qvj, qlj, qij, tbl)) {
+                if (CONDEN(ps0[kpen - 1] + ppen, exntop, thlu_top, qtu_top, thj, qvj, qlj, qij, rvj, tbl)) {
                     xflags |= UW_X_CONDEN;
                     id_exit = true;
                     stop = true;
             break;
                 }
+#if UW_TAPE_ORDER
                 if ((qlj + qij) > criqc) {
                     dwten[kpen] = ((qlj + qij) - criqc) * qlj / (qlj + qij);
                     diten[kpen] = ((qlj + qij) - criqc) * qij / (qlj + qij);
@@ -1440,6 +1841,23 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     dwten[kpen] = 0.0;
                     diten[kpen] = 0.0;
                 }
+#else
+                if (full) {
+                    if ((qlj + qij) > criqc) {
+                        dwten[kpen] = ((qlj + qij) - criqc) * qlj / (qlj + qij);
+                        diten[kpen] = ((qlj + qij) - criqc) * qij / (qlj + qij);
+                        qtu_top = qtu_top - dwten[kpen] - diten[kpen];
+                        thlu_top = thlu_top + (xlv / cp / exntop) * dwten[kpen] + (xls / cp / exntop) * diten[kpen];
+                        id_top = CONDEN(ps0[kpen - 1] + ppen, exntop, thlu_top, qtu_top, thj, qvj, qlj, qij, rvj, tbl) != 0;
+                    } else {
+                        dwten[kpen] = 0.0;
+                        diten[kpen] = 0.0;
+                        id_top = false;
+                    }
+                    ql_top = qlj;
+                    qi_top = qij;
+                }
+#endif
                 {
                     Tl rhos0j = ps0[kpen - 1] / (r * 0.5 * (thv0bot[kpen] + thv0top[kpen - 1]) * exns0[kpen - 1]);
                     cush = zs0[kpen - 1] - ppen / rhos0j / g;
@@ -1459,12 +1877,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             break;
         }
         lflags &= ~UW_L_SHCU;
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             if (k < kpen) continue;
             umf[k] = 0.0;
             emf[k] = 0.0;
             ufrc[k] = 0.0;
         }
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             if (k < kpen + 1) continue;
             dwten[k] = 0.0;
@@ -1473,13 +1893,16 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             fdr[k] = 0.0;
         }
         // penetrative entrainment (:3055-3183)
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             thlu_emf[k] = thlu[k];
             qtu_emf[k] = qtu[k];
             uu_emf[k] = uu[k];
             vu_emf[k] = vu[k];
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++) tru_emf[m][k] = tru[m][k];
         }
+#pragma unroll 1
         for (int k = mkx; k >= 0; k--) {
             if (k > kpen - 1 || k < kbup) continue;
             Tl rhos0j = ps0[k] / (r * 0.5 * (thv0bot[k + 1] + thv0top[k]) * exns0[k]);
@@ -1491,6 +1914,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 qtu_emf[k] = qt0[kpen] + ssqt0[kpen] * (ps0[k] - p0[kpen]);
                 uu_emf[k] = GL(u0, kpen) + ssu0[kpen] * (ps0[k] - p0[kpen]);
                 vu_emf[k] = GL(v0, kpen) + ssv0[kpen] * (ps0[k] - p0[kpen]);
+#pragma unroll 1
                 for (int m = 0; m < ncnst; m++) tru_emf[m][k] = GT(m + 1, kpen) + sstr0[m][kpen] * (ps0[k] - p0[kpen]);
             } else {
                 if ((emf[k + 1] - umf[k] * dp0[k + 1] * rei[k + 1] * rpen) < -0.1 * rhos0j) lflags |= UW_L_EMF;
@@ -1501,6 +1925,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     qtu_emf[k] = (qtu_emf[k + 1] * emf[k + 1] + qt0[k + 1] * (emf[k] - emf[k + 1])) / emf[k];
                     uu_emf[k] = (uu_emf[k + 1] * emf[k + 1] + GL(u0, k + 1) * (emf[k] - emf[k + 1])) / emf[k];
                     vu_emf[k] = (vu_emf[k + 1] * emf[k + 1] + GL(v0, k + 1) * (emf[k] - emf[k + 1])) / emf[k];
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++)
                         tru_emf[m][k] = (tru_emf[m][k + 1] * emf[k + 1] + GT(m + 1, k + 1) * (emf[k] - emf[k + 1])) / emf[k];
                 } else {
@@ -1508,6 +1933,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     qtu_emf[k] = qt0[k + 1];
                     uu_emf[k] = GL(u0, k + 1);
                     vu_emf[k] = GL(v0, k + 1);
+#pragma unroll 1
                     for (int m = 0; m < ncnst; m++) tru_emf[m][k] = GT(m + 1, k + 1);
                 }
             }
@@ -1518,37 +1944,44 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             Tl xtop = qt0[kinv + 1] + ssqt0[kinv + 1] * (ps0[kinv] - p0[kinv + 1]);
             Tl xbot = qt0[kinv - 1] + ssqt0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
             fluxbelowinv(cbmf, ps0, kinv, dt, xsrc, xmean, xtop, xbot, xflx);
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) if (k <= kinv - 1) qtflx[k] = xflx[k];
             xsrc = thlsrc;
             xmean = thl0[kinv];
             xtop = thl0[kinv + 1] + ssthl0[kinv + 1] * (ps0[kinv] - p0[kinv + 1]);
             xbot = thl0[kinv - 1] + ssthl0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
             fluxbelowinv(cbmf, ps0, kinv, dt, xsrc, xmean, xtop, xbot, xflx);
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) if (k <= kinv - 1) slflx[k] = cp * exns0[k] * xflx[k];
             xsrc = usrc;
             xmean = GL(u0, kinv);
             xtop = GL(u0, kinv + 1) + ssu0[kinv + 1] * (ps0[kinv] - p0[kinv + 1]);
             xbot = GL(u0, kinv - 1) + ssu0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
             fluxbelowinv(cbmf, ps0, kinv, dt, xsrc, xmean, xtop, xbot, xflx);
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) if (k <= kinv - 1) uflx[k] = xflx[k];
             xsrc = vsrc;
             xmean = GL(v0, kinv);
             xtop = GL(v0, kinv + 1) + ssv0[kinv + 1] * (ps0[kinv] - p0[kinv + 1]);
             xbot = GL(v0, kinv - 1) + ssv0[kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
             fluxbelowinv(cbmf, ps0, kinv, dt, xsrc, xmean, xtop, xbot, xflx);
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) if (k <= kinv - 1) vflx[k] = xflx[k];
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++) {
                 xsrc = trsrc[m];
                 xmean = GT(m + 1, kinv);
                 xtop = GT(m + 1, kinv + 1) + sstr0[m][kinv + 1] * (ps0[kinv] - p0[kinv + 1]);
                 xbot = GT(m + 1, kinv - 1) + sstr0[m][kinv - 1] * (ps0[kinv - 1] - p0[kinv - 1]);
                 fluxbelowinv(cbmf, ps0, kinv, dt, xsrc, xmean, xtop, xbot, xflx);
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) if (k <= kinv - 1) trflx[m][k] = xflx[k];
             }
         }
         // 2. non-buoyancy-sorting fluxes (:3300-3313)
         {
             Tl uplus = 0.0, vplus = 0.0;
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 if (k < kinv || k > krel - 1) continue;
                 const int kp1 = k + 1;
@@ -1558,11 +1991,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 vplus = vplus + PGFc * ssv0[k] * (ps0[k] - ps0[k - 1]);
                 uflx[k] = cbmf * (usrc + uplus - (GL(u0, kp1) + ssu0[kp1] * (ps0[k] - p0[kp1])));
                 vflx[k] = cbmf * (vsrc + vplus - (GL(v0, kp1) + ssv0[kp1] * (ps0[k] - p0[kp1])));
+#pragma unroll 1
                 for (int m = 0; m < ncnst; m++)
                     trflx[m][k] = cbmf * (trsrc[m] - (GT(m + 1, kp1) + sstr0[m][kp1] * (ps0[k] - p0[kp1])));
             }
         }
         // 3. buoyancy-sorting fluxes (:3322-3331)
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             if (k < krel || k > kbup - 1) continue;
             const int kp1 = k + 1;
@@ -1570,16 +2005,19 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             qtflx[k] = umf[k] * (qtu[k] - (qt0[kp1] + ssqt0[kp1] * (ps0[k] - p0[kp1])));
             uflx[k] = umf[k] * (uu[k] - (GL(u0, kp1) + ssu0[kp1] * (ps0[k] - p0[kp1])));
             vflx[k] = umf[k] * (vu[k] - (GL(v0, kp1) + ssv0[kp1] * (ps0[k] - p0[kp1])));
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++)
                 trflx[m][k] = umf[k] * (tru[m][k] - (GT(m + 1, kp1) + sstr0[m][kp1] * (ps0[k] - p0[kp1])));
         }
         // 4. penetrative-entrainment fluxes (:3392-3401)
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             if (k < kbup || k > kpen - 1) continue;
             slflx[k] = cp * exns0[k] * emf[k] * (thlu_emf[k] - (thl0[k] + ssthl0[k] * (ps0[k] - p0[k])));
             qtflx[k] = emf[k] * (qtu_emf[k] - (qt0[k] + ssqt0[k] * (ps0[k] - p0[k])));
             uflx[k] = emf[k] * (uu_emf[k] - (GL(u0, k) + ssu0[k] * (ps0[k] - p0[k])));
             vflx[k] = emf[k] * (vu_emf[k] - (GL(v0, k) + ssv0[k] * (ps0[k] - p0[k])));
+#pragma unroll 1
             for (int m = 0; m < ncnst; m++)
                 trflx[m][k] = emf[k] * (tru_emf[m][k] - (GT(m + 1, k) + sstr0[m][k] * (ps0[k] - p0[k])));
         }
@@ -1592,6 +2030,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     ((kk) <= kinv - 2 ? cbmf * (ps0[0] - ps0[(kk)]) / (ps0[0] - ps0[kinv - 1])                             \
                       : ((kk) <= krel - 1 ? cbmf : ((kk) <= kbup - 1 ? umf[(kk)] : ((kk) <= kpen - 1 ? emf[(kk)] : 0.0))))
             bool ldone = stop;
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {   // uniform
                 if (k > kpen) ldone = true;
                 if (!ldone) do {
@@ -1624,7 +2063,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 }
                 Tl thl_prog = thl0[k] + thlten_sub * dt;
                 Tl qt_prog = MX(qt0[k] + qtten_sub * dt, 1.e-12);
-                if (CONDEN(p0[k], exn0[k], thl_prog, qt_prog, thj, qvj, qlj, qij, tbl)) {
+                if (CONDEN(p0[k], exn0[k], thl_prog, qt_prog, thj, qvj, qlj, qij, rvj, tbl)) {
                     id_exit = true;
                     stop = true;
             break;
@@ -1640,6 +2079,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         UW_SYNC();
         if (!stop) do {
         // momentum tendency (:3488-3501)
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             if (k > kpen) continue;
             uten[k] = (uflx[k - 1] - uflx[k]) * g / dp0[k];
@@ -1656,6 +2096,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         {
             Tl qlubelow = 0.0, qiubelow = 0.0;
             bool ldone = stop;
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {   // uniform
                 if (k > kpen) ldone = true;
                 if (!ldone) do {
@@ -1695,10 +2136,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     qlj = 0.0;
                     qij = 0.0;
                 } else {
-                    // one conden call site for the release level, the cloud top and the levels between
+                    // the release level, the cloud top and the levels between
                     const bool atrel = (k == krel), attop = (k != krel && k == kpen);
+#if UW_TAPE_ORDER
                     if (atrel) {
-                        if (CONDEN(prel, exprel, thlu[krel - 1], qtu[krel - 1], thj, qvj, qlj, qij, tbl)) {
+                        if (CONDEN(prel, exprel, thlu[krel - 1], qtu[krel - 1], thj, qvj, qlj, qij, rvj, tbl)) {
                             xflags |= UW_X_CONDEN;
                             id_exit = true;
                             stop = true;
@@ -1708,12 +2150,26 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                         qiubelow = qij;
                     }
                     if (CONDEN(attop ? ps0[k - 1] + ppen : ps0[k], attop ? exntop : exns0[k], attop ? thlu_top : thlu[k],
-                               attop ? qtu_top : qtu[k], thj, qvj, qlj, qij, tbl)) {
+                               attop ? qtu_top : qtu[k], thj, qvj, qlj, qij, rvj, tbl)) {
                         xflags |= UW_X_CONDEN;
                         id_exit = true;
                         stop = true;
                         break;
                     }
+#else
+                    if (attop && id_top) {
+                        xflags |= UW_X_CONDEN;
+                        id_exit = true;
+                        stop = true;
+                        break;
+                    }
+                    if (atrel) {
+                        qlubelow = ql_rel;
+                        qiubelow = qi_rel;
+                    }
+                    qlj = attop ? ql_top : qltop[k];
+                    qij = attop ? qi_top : qitop[k];
+#endif
                     if (atrel) {
                         qlu_mid = 0.5 * (qlubelow + qlj) * (prel - ps0[k]) / (ps0[k - 1] - ps0[k]);
                         qiu_mid = 0.5 * (qiubelow + qij) * (prel - ps0[k]) / (ps0[k - 1] - ps0[k]);
@@ -1753,7 +2209,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     nc_lm = nc_lm - g * umf[k] * trl / (ps0[k - 1] - ps0[k]);
                     nc_im = nc_im - g * umf[k] * tri / (ps0[k - 1] - ps0[k]);
                     Tl ql_emf_kbup, qi_emf_kbup, thjj, qvjj;
-                    if (CONDEN(p0[k], exn0[k], thlu_emf[k], qtu_emf[k], thjj, qvjj, ql_emf_kbup, qi_emf_kbup, tbl)) {
+                    if (CONDEN(p0[k], exn0[k], thlu_emf[k], qtu_emf[k], thjj, qvjj, ql_emf_kbup, qi_emf_kbup, rvj, tbl)) {
                         id_exit = true;
                         stop = true;
             break;
@@ -1782,10 +2238,12 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         if (!stop) do {
         {
             Tl evpint_rain = 0.0, evpint_snow = 0.0;
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 flxrain[k] = 0.0;
                 flxsnow[k] = 0.0;
             }
+#pragma unroll 1
             for (int k = mkx; k >= 1; k--) {
                 Tl snowmlt;
                 if (t0[k] > 273.16) snowmlt = MX(0.0, flxsnow[k] * g / dp0[k]);
@@ -1830,6 +2288,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             snow = flxsnow[0] / 1000.0;
         }
         // remove detrained condensate (:3966-3981)
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             if (k > kpen) continue;
             qtten[k] = qtten[k] - qc[k];
@@ -1842,8 +2301,10 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         {
             const Tl qvmin = c.qmin[0], qlmin = c.qmin[1], qimin = c.qmin[2];
             Tl qvs[KP];
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) qvs[k] = qv0[k] + qvten[k] * dt;
             Tl dqv = 0.0;
+#pragma unroll 1
             for (int k = mkx; k >= 1; k--) {
                 Tl qlk = ql0[k] + qlten[k] * dt;
                 Tl qik = qi0[k] + qiten[k] * dt;
@@ -1865,10 +2326,12 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             }
             if (dqv > 1.e-20) {
                 Tl sum = 0.0;
+#pragma unroll 1
                 for (int k = 1; k <= mkx; k++)
                     if (qvs[k] > 2.0 * qvmin) sum = sum + qvs[k] * dp0[k];
                 Tl aa = dqv * dp0[1] / MX(1.e-20, sum);
                 if (aa < 0.5) {
+#pragma unroll 1
                     for (int k = 1; k <= mkx; k++) {
                         if (qvs[k] > 2.0 * qvmin) {
                             Tl dum = aa * qvs[k];
@@ -1879,30 +2342,36 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 }
             }
         }
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             qtten[k] = qvten[k] + qlten[k] + qiten[k];
             slten[k] = sten[k] - xlv * qlten[k] - xls * qiten[k];
         }
         // tracer tendencies (:4007-4076)
+#pragma unroll 1
         for (int m = 4; m <= ncnst; m++) {
             if (m != ixnumliq && m != ixnumice) {
                 const Tl trmin = c.qmin[m - 1];
                 const bool wet = c.wet[m - 1] != 0;
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) {
                     trflx_d[k] = 0.0;
                     trflx_u[k] = 0.0;
                 }
+#pragma unroll 1
                 for (int k = 1; k <= mkx - 1; k++) {
                     Tl pdelx = wet ? dp0[k] : GL(dpdry0, k);
                     Tl dum = (GT(m, k) - trmin) * pdelx / g / dt + trflx[m - 1][k - 1] - trflx[m - 1][k] + trflx_d[k - 1];
                     trflx_d[k] = MN(0.0, dum);
                 }
+#pragma unroll 1
                 for (int k = mkx; k >= 2; k--) {
                     Tl pdelx = wet ? dp0[k] : GL(dpdry0, k);
                     Tl dum = (GT(m, k) - trmin) * pdelx / g / dt + trflx[m - 1][k - 1] - trflx[m - 1][k] +
                                  trflx_d[k - 1] - trflx_d[k] - trflx_u[k];
                     trflx_u[k - 1] = MX(0.0, -dum);
                 }
+#pragma unroll 1
                 for (int k = 1; k <= mkx; k++) {
                     Tl pdelx = wet ? dp0[k] : GL(dpdry0, k);
                     trten[m - 1][k] = (trflx[m - 1][k - 1] - trflx[m - 1][k] + trflx_d[k - 1] - trflx_d[k] +
@@ -1911,24 +2380,36 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             }
         }
         // in-cloud diagnostics (:4092-4158)
-        if (CONDEN(prel, exprel, thlu[krel - 1], qtu[krel - 1], thj, qvj, qlj, qij, tbl)) {
+#if UW_TAPE_ORDER
+        if (CONDEN(prel, exprel, thlu[krel - 1], qtu[krel - 1], thj, qvj, qlj, qij, rvj, tbl)) {
             xflags |= UW_X_CONDEN;
             id_exit = true;
             stop = true;
             break;
         }
+#else
+        qlj = ql_rel;
+        qij = qi_rel;
+#endif
         } while (0);
         UW_SYNC();
         {
             Tl qcubelow = qlj + qij, qlubelow = qlj, qiubelow = qij;
             bool ldone = stop;
+#pragma unroll 1
             for (int j = 0; j <= mkx; j++) {   // uniform
                 const int k = krel + j;
                 if (k > kpen) ldone = true;
                 if (!ldone) do {
                 const bool attop = (k == kpen);
+#if UW_TAPE_ORDER
                 const int idc = CONDEN(attop ? ps0[k - 1] + ppen : ps0[k], attop ? exntop : exns0[k],
-                                       attop ? thlu_top : thlu[k], attop ? qtu_top : qtu[k], thj, qvj, qlj, qij, tbl);
+                                       attop ? thlu_top : thlu[k], attop ? qtu_top : qtu[k], thj, qvj, qlj, qij, rvj, tbl);
+#else
+                const bool idc = attop && id_top;
+                qlj = attop ? ql_top : qltop[k];
+                qij = attop ? qi_top : qitop[k];
+#endif
                 if (idc) {
                     xflags |= UW_X_CONDEN;
                     id_exit = true;
@@ -1974,17 +2455,20 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 
         if (iter == 1) {
             // Save the iteration-1 outputs into the output slots (the Fortran *_s copies, :4177-4277)
+#pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
                 { const Tl v_ = (umf[k]); OI(umf, k) = tl_val(v_); TOI(umf, k) = tl_der(v_); }
                 { const Tl v_ = (slflx[k]); OI(slflx, k) = tl_val(v_); TOI(slflx, k) = tl_der(v_); }
                 { const Tl v_ = (qtflx[k]); OI(qtflx, k) = tl_val(v_); TOI(qtflx, k) = tl_der(v_); }
             }
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {
                 { const Tl v_ = (qvten[k]); OL(qvten, k) = tl_val(v_); TOL(qvten, k) = tl_der(v_); } { const Tl v_ = (qlten[k]); OL(qlten, k) = tl_val(v_); TOL(qlten, k) = tl_der(v_); } { const Tl v_ = (qiten[k]); OL(qiten, k) = tl_val(v_); TOL(qiten, k) = tl_der(v_); }
                 { const Tl v_ = (sten[k]); OL(sten, k) = tl_val(v_); TOL(sten, k) = tl_der(v_); } { const Tl v_ = (uten[k]); OL(uten, k) = tl_val(v_); TOL(uten, k) = tl_der(v_); } { const Tl v_ = (vten[k]); OL(vten, k) = tl_val(v_); TOL(vten, k) = tl_der(v_); }
                 { const Tl v_ = (qrten[k]); OL(qrten, k) = tl_val(v_); TOL(qrten, k) = tl_der(v_); } { const Tl v_ = (qsten[k]); OL(qsten, k) = tl_val(v_); TOL(qsten, k) = tl_der(v_); } { const Tl v_ = (evapc[k]); OL(evapc, k) = tl_val(v_); TOL(evapc, k) = tl_der(v_); }
                 { const Tl v_ = (cufrc[k]); OL(cufrc, k) = tl_val(v_); TOL(cufrc, k) = tl_der(v_); } { const Tl v_ = (qcu[k]); OL(qcu, k) = tl_val(v_); TOL(qcu, k) = tl_der(v_); } { const Tl v_ = (qlu[k]); OL(qlu, k) = tl_val(v_); TOL(qlu, k) = tl_der(v_); }
                 { const Tl v_ = (qiu[k]); OL(qiu, k) = tl_val(v_); TOL(qiu, k) = tl_der(v_); } { const Tl v_ = (qc[k]); OL(qc, k) = tl_val(v_); TOL(qc, k) = tl_der(v_); }
+#pragma unroll 1
                 for (int m = 1; m <= ncnst; m++) { const Tl v_ = (trten[m - 1][k]); OT(m, k) = tl_val(v_); TOT(m, k) = tl_der(v_); }
             }
             { const Tl v_ = (precip); A.precip[i] = tl_val(v_); T.precip[i] = tl_der(v_); }
@@ -1999,6 +2483,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             pbup_s = ps0[kbup]; ppen_s = ps0[kpen - 1] + ppen; tkeavg_s = tkeavg;
             kinv_s = kinv; klcl_s = klcl; klfc_s = klfc; krel_s = krel; kbup_s = kbup; kpen_s = kpen;
             // advance the state for the second CIN estimate (:4177-4184, :4285-4327)
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {
                 Tl qv0s = qv0[k] + qvten[k] * dt;
                 Tl ql0s = ql0[k] + qlten[k] * dt;
@@ -2020,11 +2505,12 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         UW_SYNC();
         if (iter == 1) {   // uniform
             bool ldone = stop;
+#pragma unroll 1
             for (int k = 1; k <= mkx; k++) {   // uniform
                 if (!ldone) do {
                 Tl thl0bot = thl0[k] + ssthl0[k] * (ps0[k - 1] - p0[k]);
                 Tl qt0bot = qt0[k] + ssqt0[k] * (ps0[k - 1] - p0[k]);
-                if (CONDEN(ps0[k - 1], exns0[k - 1], thl0bot, qt0bot, thj, qvj, qlj, qij, tbl)) {
+                if (CONDEN(ps0[k - 1], exns0[k - 1], thl0bot, qt0bot, thj, qvj, qlj, qij, rvj, tbl)) {
                     xflags |= UW_X_CONDEN;
                     id_exit = true;
                     stop = true;
@@ -2034,7 +2520,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 thvl0bot[k] = thl0bot * (1.0 + zvir * qt0bot);
                 Tl thl0top = thl0[k] + ssthl0[k] * (ps0[k] - p0[k]);
                 Tl qt0top = qt0[k] + ssqt0[k] * (ps0[k] - p0[k]);
-                if (CONDEN(ps0[k], exns0[k], thl0top, qt0top, thj, qvj, qlj, qij, tbl)) {
+                if (CONDEN(ps0[k], exns0[k], thl0top, qt0top, thj, qvj, qlj, qij, rvj, tbl)) {
                     xflags |= UW_X_CONDEN;
                     id_exit = true;
                     stop = true;
@@ -2052,6 +2538,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 
     // ---- final outputs (uwshcu.F90:4337-4370) --------------------------------------------------
     if (!stop) {
+#pragma unroll 1
     for (int k = 0; k <= mkx; k++) {
         { const Tl v_ = (umf[k]); OI(umf, k) = tl_val(v_); TOI(umf, k) = tl_der(v_); }
         { const Tl v_ = (wu[k]); OI(wu, k) = tl_val(v_); TOI(wu, k) = tl_der(v_); }
@@ -2060,12 +2547,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         { const Tl v_ = (flxrain[k] + flxsnow[k]); OI(flxprc1, k) = tl_val(v_); TOI(flxprc1, k) = tl_der(v_); }
         { const Tl v_ = (flxsnow[k]); OI(flxsnow1, k) = tl_val(v_); TOI(flxsnow1, k) = tl_der(v_); }
     }
+#pragma unroll 1
     for (int k = 1; k <= mkx; k++) {
         { const Tl v_ = (qvten[k]); OL(qvten, k) = tl_val(v_); TOL(qvten, k) = tl_der(v_); } { const Tl v_ = (qlten[k]); OL(qlten, k) = tl_val(v_); TOL(qlten, k) = tl_der(v_); } { const Tl v_ = (qiten[k]); OL(qiten, k) = tl_val(v_); TOL(qiten, k) = tl_der(v_); }
         { const Tl v_ = (sten[k]); OL(sten, k) = tl_val(v_); TOL(sten, k) = tl_der(v_); } { const Tl v_ = (uten[k]); OL(uten, k) = tl_val(v_); TOL(uten, k) = tl_der(v_); } { const Tl v_ = (vten[k]); OL(vten, k) = tl_val(v_); TOL(vten, k) = tl_der(v_); }
         { const Tl v_ = (qrten[k]); OL(qrten, k) = tl_val(v_); TOL(qrten, k) = tl_der(v_); } { const Tl v_ = (qsten[k]); OL(qsten, k) = tl_val(v_); TOL(qsten, k) = tl_der(v_); } { const Tl v_ = (evapc[k]); OL(evapc, k) = tl_val(v_); TOL(evapc, k) = tl_der(v_); }
         { const Tl v_ = (cufrc[k]); OL(cufrc, k) = tl_val(v_); TOL(cufrc, k) = tl_der(v_); } { const Tl v_ = (qcu[k]); OL(qcu, k) = tl_val(v_); TOL(qcu, k) = tl_der(v_); } { const Tl v_ = (qlu[k]); OL(qlu, k) = tl_val(v_); TOL(qlu, k) = tl_der(v_); }
         { const Tl v_ = (qiu[k]); OL(qiu, k) = tl_val(v_); TOL(qiu, k) = tl_der(v_); } { const Tl v_ = (qc[k]); OL(qc, k) = tl_val(v_); TOL(qc, k) = tl_der(v_); }
+#pragma unroll 1
         for (int m = 1; m <= ncnst; m++) { const Tl v_ = (trten[m - 1][k]); OT(m, k) = tl_val(v_); TOT(m, k) = tl_der(v_); }
     }
     { const Tl v_ = (precip); A.precip[i] = tl_val(v_); T.precip[i] = tl_der(v_); }
@@ -2092,6 +2581,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     if (!cand && !handed) {
     if (id_exit) {
         xflags |= UW_X_UWCU;
+#pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             { const Tl v_ = (0.0); OI(umf, k) = tl_val(v_); TOI(umf, k) = tl_der(v_); }
             { const Tl v_ = (0.0); OI(wu, k) = tl_val(v_); TOI(wu, k) = tl_der(v_); }
@@ -2100,11 +2590,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             { const Tl v_ = (0.0); OI(flxprc1, k) = tl_val(v_); TOI(flxprc1, k) = tl_der(v_); }
             { const Tl v_ = (0.0); OI(flxsnow1, k) = tl_val(v_); TOI(flxsnow1, k) = tl_der(v_); }
         }
+#pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             { const Tl v_ = (0.0); OL(qvten, k) = tl_val(v_); TOL(qvten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qlten, k) = tl_val(v_); TOL(qlten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qiten, k) = tl_val(v_); TOL(qiten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(sten, k) = tl_val(v_); TOL(sten, k) = tl_der(v_); }
             { const Tl v_ = (0.0); OL(uten, k) = tl_val(v_); TOL(uten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(vten, k) = tl_val(v_); TOL(vten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qrten, k) = tl_val(v_); TOL(qrten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qsten, k) = tl_val(v_); TOL(qsten, k) = tl_der(v_); }
             { const Tl v_ = (0.0); OL(evapc, k) = tl_val(v_); TOL(evapc, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(cufrc, k) = tl_val(v_); TOL(cufrc, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qcu, k) = tl_val(v_); TOL(qcu, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qlu, k) = tl_val(v_); TOL(qlu, k) = tl_der(v_); }
             { const Tl v_ = (0.0); OL(qiu, k) = tl_val(v_); TOL(qiu, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qc, k) = tl_val(v_); TOL(qc, k) = tl_der(v_); }
+#pragma unroll 1
             for (int m = 1; m <= ncnst; m++) { const Tl v_ = (0.0); OT(m, k) = tl_val(v_); TOT(m, k) = tl_der(v_); }
         }
         { const Tl v_ = (0.0); A.precip[i] = tl_val(v_); T.precip[i] = tl_der(v_); }
@@ -2117,10 +2609,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         if (A.diag_real) {
             A.diag_real[UW_DR_CIN * (size_t)mix + i] = tl_val(-1.0);
             A.diag_real[UW_DR_CINLCL * (size_t)mix + i] = tl_val(-1.0);
+#pragma unroll 1
             for (int j = UW_DR_PLCL; j < UW_NDR; j++) A.diag_real[j * (size_t)mix + i] = tl_val(0.0);
         }
         if (A.diag_level)
+#pragma unroll 1
             for (int j = 0; j < UW_NDL; j++)
+#pragma unroll 1
                 for (int k = 0; k <= mkx; k++) DLV(j, k) = tl_val(0.0);
         kinv = klcl = klfc = krel = kbup = kpen = 0;
     }
@@ -2157,6 +2652,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     }
 #undef UW_SYNC
 #undef CONDEN
+#undef UW_QSAT_OF_CONDEN
 #undef RI
 #undef RL
 #undef CNT

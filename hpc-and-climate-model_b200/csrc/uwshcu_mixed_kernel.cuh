@@ -45,21 +45,6 @@ struct Kahan {
         s = t;
     }
 };
-// Kahan sums in the hand-off state of the sorted schedule (uw_state.cuh): two words (the scalar
-// overloads there stay visible next to these).
-using ::uw_st_get;
-using ::uw_st_put;
-__device__ __forceinline__ void uw_st_put(double* st, size_t& w, size_t cs, const Kahan& x)
-{
-    st[w++ * cs] = (double)x.s;
-    st[w++ * cs] = (double)x.e;
-}
-__device__ __forceinline__ void uw_st_get(const double* st, size_t& w, size_t cs, Kahan& x)
-{
-    x.s = (float)st[w++ * cs];
-    x.e = (float)st[w++ * cs];
-}
-
 __device__ __forceinline__ float estblf_f(float td, const float* __restrict__ tf)
 {
     const float tmin = (float)c.tmin, tmax = (float)c.tmax;
@@ -513,6 +498,16 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 #define OT(m, k) A.trten[((size_t)((m) - 1) * mkx + RL(k)) * mix + i]
 #define CNT(x) (inv ? (double)(mkx + 1) - (double)(x) : (double)(x))
 #define DLV(j, k) A.diag_level[((size_t)(j) * (mkx + 1) + (k)) * mix + i]
+// uemf(k), evaluated on demand with the same expressions as :3416-3422
+#define UEMF(kk)                                                                                          \
+    ((kk) <= kinv - 2 ? cbmf * (ps0[0] - ps0[(kk)]) / (ps0[0] - ps0[kinv - 1])                             \
+                      : ((kk) <= krel - 1 ? cbmf : ((kk) <= kbup - 1 ? umf[(kk)] : ((kk) <= kpen - 1 ? emf[(kk)] : 0.0f))))
+// the profiles that the per-level diagnostics show outside the updraft's levels as well
+#define ZERO_DIAG_PROFILES()                                                                              \
+    _Pragma("unroll 1") for (int k = 0; k <= mkx; k++) {                                                  \
+        ufrc[k] = 0.0f; thlu[k] = 0.0f; qtu[k] = 0.0f; thvu[k] = 0.0f; uu[k] = 0.0f; vu[k] = 0.0f;              \
+        dwten[k] = 0.0f; diten[k] = 0.0f; fer[k] = 0.0f; fdr[k] = 0.0f;                                       \
+    }
 // per-level diagnostics of the current state, levels bottom-up in both level orders
 // (uwshcu.F90:1945-1990 and :4383-4433)
 #define PUT_DIAG_LEVEL()                                                                                  \
@@ -589,33 +584,9 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 
     if constexpr (MODE != UW_MODE_RESUME) {   // uniform
 
-    // ---- output initialisation (uwshcu.F90:1087-1124) ------------------------------------------
-    if (MODE != UW_MODE_TRIGGER) {
-#pragma unroll 1
-    for (int k = 0; k <= mkx; k++) {
-        OI(umf, k) = 0.0f;
-        OI(slflx, k) = 0.0f;
-        OI(qtflx, k) = 0.0f;
-        OI(flxprc1, k) = 0.0f;
-        OI(flxsnow1, k) = 0.0f;
-        OI(wu, k) = 0.0f;
-    }
-#pragma unroll 1
-    for (int k = 1; k <= mkx; k++) {
-        OL(qvten, k) = 0.0f; OL(qlten, k) = 0.0f; OL(qiten, k) = 0.0f; OL(sten, k) = 0.0f;
-        OL(uten, k) = 0.0f; OL(vten, k) = 0.0f; OL(qrten, k) = 0.0f; OL(qsten, k) = 0.0f;
-        OL(evapc, k) = 0.0f; OL(cufrc, k) = 0.0f; OL(qcu, k) = 0.0f; OL(qlu, k) = 0.0f;
-        OL(qiu, k) = 0.0f; OL(qc, k) = 0.0f;
-#pragma unroll 1
-        for (int m = 1; m <= ncnst; m++) OT(m, k) = 0.0f;
-    }
-    A.precip[i] = 0.0f;
-    A.snow[i] = 0.0f;
-    A.cbmf[i] = 0.0f;
-    A.rliq[i] = 0.0f;
-    A.cnt[i] = CNT((R)mkx);
-    A.cnb[i] = CNT(0.0f);
-    }
+    // The Fortran zeroes every output here (uwshcu.F90:1087-1124).  Every way out of the column below
+    // writes all of them (the final outputs, label 333, or the explicit-CIN branch of iteration 2),
+    // so nothing is stored twice.
 
     // ---- inputs and findsp (uwshcu.F90:1216-1259), and non-finite inputs ----------------------
     // Non-finite inputs have no counterpart in the Fortran, where a NaN or Inf propagates into the
@@ -709,37 +680,16 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         thvl0top_o[k] = thvl0top[k];
     }
     if (!stop) {
-    // per-column initialisation (:1333-1408)
-#pragma unroll 1
-    for (int k = 0; k <= mkx; k++) {
-        umf[k] = 0.0f; emf[k] = 0.0f; slflx[k] = 0.0f; qtflx[k] = 0.0f; uflx[k] = 0.0f; vflx[k] = 0.0f;
-        ufrc[k] = 0.0f; thlu[k] = 0.0f; qtu[k] = 0.0f; uu[k] = 0.0f; vu[k] = 0.0f; wu[k] = 0.0f;
-        thvu[k] = 0.0f; thlu_emf[k] = 0.0f; qtu_emf[k] = 0.0f; uu_emf[k] = 0.0f; vu_emf[k] = 0.0f;
-#pragma unroll 1
-        for (int m = 0; m < ncnst; m++) {
-            trflx[m][k] = 0.0f;
-            tru[m][k] = 0.0f;
-            tru_emf[m][k] = 0.0f;
-        }
-    }
-#pragma unroll 1
-    for (int k = 1; k <= mkx; k++) {
-        qvten[k] = 0.0f; qlten[k] = 0.0f; qiten[k] = 0.0f; sten[k] = 0.0f; uten[k] = 0.0f; vten[k] = 0.0f;
-        qrten[k] = 0.0f; qsten[k] = 0.0f; dwten[k] = 0.0f; diten[k] = 0.0f; evapc[k] = 0.0f;
-        cufrc[k] = 0.0f; qcu[k] = 0.0f; qlu[k] = 0.0f; qiu[k] = 0.0f; fer[k] = 0.0f; fdr[k] = 0.0f;
-        qc[k] = 0.0f; qc_l[k] = 0.0f; qc_i[k] = 0.0f; qtten[k] = 0.0f; slten[k] = 0.0f;
-        qlten_sink[k] = 0.0f; qiten_sink[k] = 0.0f; nlten_sink[k] = 0.0f; niten_sink[k] = 0.0f;
-        rei[k] = 0.0f; uf[k] = 0.0f; vf[k] = 0.0f;
-#pragma unroll 1
-        for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0f;
-    }
+    // The Fortran zeroes some 80 profiles here and again at the implicit-CIN restore (:1333-1408,
+    // :1759-1889).  The sections below write every level that they, or the outputs, read (the zeroes
+    // outside the cloud included), each level once; only the per-level diagnostics show the others.
+    if (A.diag_level) ZERO_DIAG_PROFILES();
     cnt = (R)mkx;
     cnb = 0.0f;
     }
     } else {   // uniform
-        // the state UW_MODE_LIST1 stored at the implicit-CIN branch of iteration 2 (uw_state.cuh),
-        // and the arrays that the set-up and that branch's restore build from the inputs, rebuilt
-        // with the same operations
+        // the state UW_MODE_LIST1 stored at the implicit-CIN branch of iteration 2 (uw_state.cuh), and
+        // the environment profiles that the set-up builds from the inputs, with the same operations
         UW_LOAD_STATE(A.hand->state + i_in, (size_t)A.hand->cap, tscaleh_r);
 #pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
@@ -775,36 +725,10 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             s0[k] = GL(s0, k);
             qt0[k] = (qv0[k] + ql0[k] + qi0[k]);
             thl0[k] = (t0[k] - xlv * ql0[k] / cp - xls * qi0[k] / cp) / exn0[k];
-            thv0bot[k] = thv0bot_o[k];
-            thv0top[k] = thv0top_o[k];
-            thvl0bot[k] = thvl0bot_o[k];
-            thvl0top[k] = thvl0top_o[k];
         }
         slope<KP>(mkx, thl0, p0, ssthl0);
         slope<KP>(mkx, qt0, p0, ssqt0);
-#pragma unroll 1
-        for (int k = 0; k <= mkx; k++) {
-            umf[k] = 0.0f; emf[k] = 0.0f; slflx[k] = 0.0f; qtflx[k] = 0.0f; uflx[k] = 0.0f;
-            vflx[k] = 0.0f; ufrc[k] = 0.0f; thlu[k] = 0.0f; qtu[k] = 0.0f; uu[k] = 0.0f;
-            vu[k] = 0.0f; wu[k] = 0.0f; thvu[k] = 0.0f; thlu_emf[k] = 0.0f; qtu_emf[k] = 0.0f;
-            uu_emf[k] = 0.0f; vu_emf[k] = 0.0f;
-#pragma unroll 1
-            for (int m = 0; m < ncnst; m++) {
-                trflx[m][k] = 0.0f;
-                tru[m][k] = 0.0f;
-                tru_emf[m][k] = 0.0f;
-            }
-        }
-#pragma unroll 1
-        for (int k = 1; k <= mkx; k++) {
-            qvten[k] = 0.0f; qlten[k] = 0.0f; qiten[k] = 0.0f; sten[k] = 0.0f; uten[k] = 0.0f;
-            vten[k] = 0.0f; qrten[k] = 0.0f; qsten[k] = 0.0f; dwten[k] = 0.0f; diten[k] = 0.0f;
-            evapc[k] = 0.0f; cufrc[k] = 0.0f; qcu[k] = 0.0f; qlu[k] = 0.0f; qiu[k] = 0.0f;
-            fer[k] = 0.0f; fdr[k] = 0.0f; qc[k] = 0.0f; qc_l[k] = 0.0f; qc_i[k] = 0.0f;
-            qtten[k] = 0.0f; slten[k] = 0.0f;
-#pragma unroll 1
-            for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0f;
-        }
+        if (A.diag_level) ZERO_DIAG_PROFILES();
     }
 
     UW_SYNC();
@@ -1017,37 +941,40 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 }
                 slope<KP>(mkx, thl0, p0, ssthl0);
                 slope<KP>(mkx, qt0, p0, ssqt0);
-#pragma unroll 1
-                for (int k = 0; k <= mkx; k++) {
-                    umf[k] = 0.0f; emf[k] = 0.0f; slflx[k] = 0.0f; qtflx[k] = 0.0f; uflx[k] = 0.0f;
-                    vflx[k] = 0.0f; ufrc[k] = 0.0f; thlu[k] = 0.0f; qtu[k] = 0.0f; uu[k] = 0.0f;
-                    vu[k] = 0.0f; wu[k] = 0.0f; thvu[k] = 0.0f; thlu_emf[k] = 0.0f; qtu_emf[k] = 0.0f;
-                    uu_emf[k] = 0.0f; vu_emf[k] = 0.0f;
-#pragma unroll 1
-                    for (int m = 0; m < ncnst; m++) {
-                        trflx[m][k] = 0.0f;
-                        tru[m][k] = 0.0f;
-                        tru_emf[m][k] = 0.0f;
-                    }
-                }
-#pragma unroll 1
-                for (int k = 1; k <= mkx; k++) {
-                    qvten[k] = 0.0f; qlten[k] = 0.0f; qiten[k] = 0.0f; sten[k] = 0.0f; uten[k] = 0.0f;
-                    vten[k] = 0.0f; qrten[k] = 0.0f; qsten[k] = 0.0f; dwten[k] = 0.0f; diten[k] = 0.0f;
-                    evapc[k] = 0.0f; cufrc[k] = 0.0f; qcu[k] = 0.0f; qlu[k] = 0.0f; qiu[k] = 0.0f;
-                    fer[k] = 0.0f; fdr[k] = 0.0f; qc[k] = 0.0f; qc_l[k] = 0.0f; qc_i[k] = 0.0f;
-                    qtten[k] = 0.0f; slten[k] = 0.0f;
-#pragma unroll 1
-                    for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0f;
-                }
+                if (A.diag_level) ZERO_DIAG_PROFILES();
                 precip = 0.0f; snow = 0.0f; rliq.reset(); cbmf = 0.0f;
                 cnt = (R)mkx; cnb = 0.0f; ufrclcl = 0.0f; wlcl = 0.0f;
             } else {
-                // explicit CIN: the iteration-1 outputs already sit in the output slots (:1891-2011);
-                // flxprc1/flxsnow1 keep their initial zeros on this path, wu_out gets wu.
+                // explicit CIN: iteration 1's results are the column's (the Fortran's *_s copies,
+                // :1891-2011, :4177-4277).  The profiles still hold them (this iteration has rebuilt
+                // the environment only) and cush is in tscaleh; flxprc1/flxsnow1 are zero on this path.
                 lflags |= UW_L_DELCIN;
 #pragma unroll 1
-                for (int k = 0; k <= mkx; k++) OI(wu, k) = wu[k];
+                for (int k = 0; k <= mkx; k++) {
+                    OI(umf, k) = umf[k];
+                    OI(wu, k) = wu[k];
+                    OI(slflx, k) = slflx[k];
+                    OI(qtflx, k) = qtflx[k];
+                    OI(flxprc1, k) = 0.0f;
+                    OI(flxsnow1, k) = 0.0f;
+                }
+#pragma unroll 1
+                for (int k = 1; k <= mkx; k++) {
+                    OL(qvten, k) = qvten[k]; OL(qlten, k) = qlten[k]; OL(qiten, k) = qiten[k];
+                    OL(sten, k) = sten[k]; OL(uten, k) = uten[k]; OL(vten, k) = vten[k];
+                    OL(qrten, k) = qrten[k]; OL(qsten, k) = qsten[k]; OL(evapc, k) = evapc[k];
+                    OL(cufrc, k) = cufrc[k]; OL(qcu, k) = qcu[k]; OL(qlu, k) = qlu[k];
+                    OL(qiu, k) = qiu[k]; OL(qc, k) = qc[k];
+#pragma unroll 1
+                    for (int m = 1; m <= ncnst; m++) OT(m, k) = trten[m - 1][k];
+                }
+                A.precip[i] = precip;
+                A.snow[i] = snow;
+                A.cush[i] = tscaleh;
+                A.cbmf[i] = cbmf;
+                A.rliq[i] = rliq.s;
+                A.cnt[i] = CNT(cnt);
+                A.cnb[i] = CNT(cnb);
                 if (A.diag_real) {
                     A.diag_real[UW_DR_CIN * (size_t)mix + i] = cin_s;
                     A.diag_real[UW_DR_CINLCL * (size_t)mix + i] = cinlcl_s;
@@ -1059,6 +986,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     A.diag_real[UW_DR_TKEAVG * (size_t)mix + i] = tkeavg_s;
                 }
                 kinv = kinv_s; klcl = klcl_s; klfc = klfc_s; krel = krel_s; kbup = kbup_s; kpen = kpen_s;
+                PUT_DIAG_LEVEL();
                 id_exit = false;
                 stop = true;
             break;
@@ -1160,10 +1088,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             ufrc[krel - 1] = ufrclcl;
 #pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
-                if (k < kinv - 1 || k > krel - 1) continue;
-                umf[k] = cbmf;
-                wu[k] = winv;
+                const bool sub = k >= kinv - 1 && k <= krel - 1;
+                umf[k] = sub ? cbmf : 0.0f;
+                wu[k] = sub ? winv : 0.0f;
             }
+            fer[krel] = 0.0f;   // read at kpen = krel when no level is left for the updraft
         }
         } while (0);
         if (MODE == UW_MODE_TRIGGER) {
@@ -1852,30 +1781,20 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         }
         lflags &= ~UW_L_SHCU;
 #pragma unroll 1
-        for (int k = 0; k <= mkx; k++) {
-            if (k < kpen) continue;
-            umf[k] = 0.0f;
-            emf[k] = 0.0f;
-            ufrc[k] = 0.0f;
-        }
+        for (int k = kpen; k <= mkx; k++) umf[k] = 0.0f;
+        ufrc[kpen] = 0.0f;
+        if (A.diag_level) {
 #pragma unroll 1
-        for (int k = 0; k <= mkx; k++) {
-            if (k < kpen + 1) continue;
-            dwten[k] = 0.0f;
-            diten[k] = 0.0f;
-            fer[k] = 0.0f;
-            fdr[k] = 0.0f;
+            for (int k = kpen + 1; k <= mkx; k++) {
+                ufrc[k] = 0.0f;
+                dwten[k] = 0.0f;
+                diten[k] = 0.0f;
+                fer[k] = 0.0f;
+                fdr[k] = 0.0f;
+            }
         }
         // penetrative entrainment (:3055-3183)
-#pragma unroll 1
-        for (int k = 0; k <= mkx; k++) {
-            thlu_emf[k] = thlu[k];
-            qtu_emf[k] = qtu[k];
-            uu_emf[k] = uu[k];
-            vu_emf[k] = vu[k];
-#pragma unroll 1
-            for (int m = 0; m < ncnst; m++) tru_emf[m][k] = tru[m][k];
-        }
+        // (the *_emf profiles are read at kbup .. kpen - 1 only)
 #pragma unroll 1
         for (int k = mkx; k >= 0; k--) {
             if (k > kpen - 1 || k < kbup) continue;
@@ -1995,14 +1914,20 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             for (int m = 0; m < ncnst; m++)
                 trflx[m][k] = emf[k] * (tru_emf[m][k] - (GT(m + 1, k) + sstr0[m][k] * (ps0[k] - p0[k])));
         }
+        // none above
+#pragma unroll 1
+        for (int k = MX(kpen, kbup); k <= mkx; k++) {
+            slflx[k] = 0.0f;
+            qtflx[k] = 0.0f;
+            uflx[k] = 0.0f;
+            vflx[k] = 0.0f;
+#pragma unroll 1
+            for (int m = 0; m < ncnst; m++) trflx[m][k] = 0.0f;
+        }
         } while (0);
         UW_SYNC();
         // condensate tendency by compensating subsidence (:3416-3476)
         {
-            // uemf(k), evaluated on demand with the same expressions as :3416-3422
-#define UEMF(kk)                                                                                          \
-    ((kk) <= kinv - 2 ? cbmf * (ps0[0] - ps0[(kk)]) / (ps0[0] - ps0[kinv - 1])                             \
-                      : ((kk) <= krel - 1 ? cbmf : ((kk) <= kbup - 1 ? umf[(kk)] : ((kk) <= kpen - 1 ? emf[(kk)] : 0.0f))))
             bool ldone = stop;
 #pragma unroll 1
             for (int k = 1; k <= mkx; k++) {   // uniform
@@ -2055,7 +1980,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         // momentum tendency (:3488-3501)
 #pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
-            if (k > kpen) continue;
+            if (k > kpen) {
+                uten[k] = 0.0f;
+                vten[k] = 0.0f;
+                continue;
+            }
             uten[k] = (uflx[k - 1] - uflx[k]) * g / dp0[k];
             vten[k] = (vflx[k - 1] - vflx[k]) * g / dp0[k];
             uf[k] = GL(u0, k) + uten[k] * dt;
@@ -2072,9 +2001,20 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             bool ldone = stop;
 #pragma unroll 1
             for (int k = 1; k <= mkx; k++) {   // uniform
-                if (k > kpen) ldone = true;
+                if (k > kpen) {
+                    ldone = true;
+                    qrten[k] = 0.0f; qsten[k] = 0.0f; qlten[k] = 0.0f; qiten[k] = 0.0f; qvten[k] = 0.0f;
+                    sten[k] = 0.0f; qc[k] = 0.0f;
+                    trten[ixnumliq - 1][k] = 0.0f;
+                    trten[ixnumice - 1][k] = 0.0f;
+                }
                 if (!ldone) do {
                 const int km1 = k - 1;
+                if (k < krel) {   // below the updraft
+                    dwten[k] = 0.0f;
+                    diten[k] = 0.0f;
+                    fdr[k] = 0.0f;
+                }
                 dwten[k] = dwten[k] * 0.5f * (umf[k - 1] + umf[k]) * g / dp0[k];
                 diten[k] = diten[k] * 0.5f * (umf[k - 1] + umf[k]) * g / dp0[k];
                 qrten[k] = frc_rasn * dwten[k];
@@ -2240,6 +2180,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     evpsnow = tmp2;
                 }
                 evapc[k] = evprain + evpsnow;
+                cufrc[k] = 0.0f; qcu[k] = 0.0f; qlu[k] = 0.0f; qiu[k] = 0.0f;   // in cloud: below
                 evpint_rain.add(evprain * dp0[k] / g);
                 evpint_snow.add(evpsnow * dp0[k] / g);
                 R ntraprd = qrten[k] - evprain + snowmlt;
@@ -2322,8 +2263,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         }
         // tracer tendencies (:4007-4076)
 #pragma unroll 1
-        for (int m = 4; m <= ncnst; m++) {
-            if (m != ixnumliq && m != ixnumice) {
+        for (int m = 1; m <= ncnst; m++) {
+            if (m < 4) {
+                if (m != ixnumliq && m != ixnumice) {   // qv, ql and qi: their tendencies are outputs of their own
+#pragma unroll 1
+                    for (int k = 1; k <= mkx; k++) trten[m - 1][k] = 0.0f;
+                }
+            } else if (m != ixnumliq && m != ixnumice) {
                 const R trmin = c.qmin[m - 1];
                 const bool wet = c.wet[m - 1] != 0;
 #pragma unroll 1
@@ -2427,31 +2373,6 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         cnb = (R)(krel - 1);
 
         if (iter == 1) {
-            // Save the iteration-1 outputs into the output slots (the Fortran *_s copies, :4177-4277)
-#pragma unroll 1
-            for (int k = 0; k <= mkx; k++) {
-                OI(umf, k) = umf[k];
-                OI(slflx, k) = slflx[k];
-                OI(qtflx, k) = qtflx[k];
-            }
-#pragma unroll 1
-            for (int k = 1; k <= mkx; k++) {
-                OL(qvten, k) = qvten[k]; OL(qlten, k) = qlten[k]; OL(qiten, k) = qiten[k];
-                OL(sten, k) = sten[k]; OL(uten, k) = uten[k]; OL(vten, k) = vten[k];
-                OL(qrten, k) = qrten[k]; OL(qsten, k) = qsten[k]; OL(evapc, k) = evapc[k];
-                OL(cufrc, k) = cufrc[k]; OL(qcu, k) = qcu[k]; OL(qlu, k) = qlu[k];
-                OL(qiu, k) = qiu[k]; OL(qc, k) = qc[k];
-#pragma unroll 1
-                for (int m = 1; m <= ncnst; m++) OT(m, k) = trten[m - 1][k];
-            }
-            A.precip[i] = precip;
-            A.snow[i] = snow;
-            A.cush[i] = cush;
-            A.cbmf[i] = cbmf;
-            A.rliq[i] = rliq.s;
-            A.cnt[i] = CNT(cnt);
-            A.cnb[i] = CNT(cnb);
-            PUT_DIAG_LEVEL();
             cin_s = cin; cinlcl_s = cinlcl; plcl_s = plcl; pinv_s = ps0[kinv - 1]; plfc_s = plfc;
             pbup_s = ps0[kbup]; ppen_s = ps0[kpen - 1] + ppen; tkeavg_s = tkeavg;
             kinv_s = kinv; klcl_s = klcl; klfc_s = klfc; krel_s = krel; kbup_s = kbup; kpen_s = kpen;
@@ -2637,6 +2558,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 #undef OT
 #undef DLV
 #undef PUT_DIAG_LEVEL
+#undef ZERO_DIAG_PROFILES
 #undef UEMF
 }
 

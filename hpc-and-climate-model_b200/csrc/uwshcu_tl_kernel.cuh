@@ -544,6 +544,16 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 #define SEEDI(a, da, k) Tl(GI(a, k), T.da ? __ldg(&T.da[(size_t)RI(k) * mix + i]) : 0.0)
 #define CNT(x) (inv ? (Tl)(mkx + 1) - (x) : (x))
 #define DLV(j, k) A.diag_level[((size_t)(j) * (mkx + 1) + (k)) * mix + i]
+// uemf(k), evaluated on demand with the same expressions as :3416-3422
+#define UEMF(kk)                                                                                          \
+    ((kk) <= kinv - 2 ? cbmf * (ps0[0] - ps0[(kk)]) / (ps0[0] - ps0[kinv - 1])                             \
+                      : ((kk) <= krel - 1 ? cbmf : ((kk) <= kbup - 1 ? umf[(kk)] : ((kk) <= kpen - 1 ? emf[(kk)] : 0.0))))
+// the profiles that the per-level diagnostics show outside the updraft's levels as well
+#define ZERO_DIAG_PROFILES()                                                                              \
+    _Pragma("unroll 1") for (int k = 0; k <= mkx; k++) {                                                  \
+        ufrc[k] = 0.0; thlu[k] = 0.0; qtu[k] = 0.0; thvu[k] = 0.0; uu[k] = 0.0; vu[k] = 0.0;              \
+        dwten[k] = 0.0; diten[k] = 0.0; fer[k] = 0.0; fdr[k] = 0.0;                                       \
+    }
 // per-level diagnostics of the current state, levels bottom-up in both level orders
 // (uwshcu.F90:1945-1990 and :4383-4433)
 #define PUT_DIAG_LEVEL()                                                                                  \
@@ -616,33 +626,9 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 
     if constexpr (MODE != UW_MODE_RESUME) {   // uniform
 
-    // ---- output initialisation (uwshcu.F90:1087-1124) ------------------------------------------
-    if (MODE != UW_MODE_TRIGGER) {
-#pragma unroll 1
-    for (int k = 0; k <= mkx; k++) {
-        { const Tl v_ = (0.0); OI(umf, k) = tl_val(v_); TOI(umf, k) = tl_der(v_); }
-        { const Tl v_ = (0.0); OI(slflx, k) = tl_val(v_); TOI(slflx, k) = tl_der(v_); }
-        { const Tl v_ = (0.0); OI(qtflx, k) = tl_val(v_); TOI(qtflx, k) = tl_der(v_); }
-        { const Tl v_ = (0.0); OI(flxprc1, k) = tl_val(v_); TOI(flxprc1, k) = tl_der(v_); }
-        { const Tl v_ = (0.0); OI(flxsnow1, k) = tl_val(v_); TOI(flxsnow1, k) = tl_der(v_); }
-        { const Tl v_ = (0.0); OI(wu, k) = tl_val(v_); TOI(wu, k) = tl_der(v_); }
-    }
-#pragma unroll 1
-    for (int k = 1; k <= mkx; k++) {
-        { const Tl v_ = (0.0); OL(qvten, k) = tl_val(v_); TOL(qvten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qlten, k) = tl_val(v_); TOL(qlten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qiten, k) = tl_val(v_); TOL(qiten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(sten, k) = tl_val(v_); TOL(sten, k) = tl_der(v_); }
-        { const Tl v_ = (0.0); OL(uten, k) = tl_val(v_); TOL(uten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(vten, k) = tl_val(v_); TOL(vten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qrten, k) = tl_val(v_); TOL(qrten, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qsten, k) = tl_val(v_); TOL(qsten, k) = tl_der(v_); }
-        { const Tl v_ = (0.0); OL(evapc, k) = tl_val(v_); TOL(evapc, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(cufrc, k) = tl_val(v_); TOL(cufrc, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qcu, k) = tl_val(v_); TOL(qcu, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qlu, k) = tl_val(v_); TOL(qlu, k) = tl_der(v_); }
-        { const Tl v_ = (0.0); OL(qiu, k) = tl_val(v_); TOL(qiu, k) = tl_der(v_); } { const Tl v_ = (0.0); OL(qc, k) = tl_val(v_); TOL(qc, k) = tl_der(v_); }
-#pragma unroll 1
-        for (int m = 1; m <= ncnst; m++) { const Tl v_ = (0.0); OT(m, k) = tl_val(v_); TOT(m, k) = tl_der(v_); }
-    }
-    { const Tl v_ = (0.0); A.precip[i] = tl_val(v_); T.precip[i] = tl_der(v_); }
-    { const Tl v_ = (0.0); A.snow[i] = tl_val(v_); T.snow[i] = tl_der(v_); }
-    { const Tl v_ = (0.0); A.cbmf[i] = tl_val(v_); T.cbmf[i] = tl_der(v_); }
-    { const Tl v_ = (0.0); A.rliq[i] = tl_val(v_); T.rliq[i] = tl_der(v_); }
-    A.cnt[i] = tl_val(CNT((Tl)mkx));
-    A.cnb[i] = tl_val(CNT(0.0));
-    }
+    // The Fortran zeroes every output here (uwshcu.F90:1087-1124).  Every way out of the column below
+    // writes all of them (the final outputs, label 333, or the explicit-CIN branch of iteration 2),
+    // so nothing is stored twice.
 
     // ---- inputs and findsp (uwshcu.F90:1216-1259), and non-finite inputs ----------------------
     // Non-finite inputs have no counterpart in the Fortran, where a NaN or Inf propagates into the
@@ -736,37 +722,16 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         thvl0top_o[k] = thvl0top[k];
     }
     if (!stop) {
-    // per-column initialisation (:1333-1408)
-#pragma unroll 1
-    for (int k = 0; k <= mkx; k++) {
-        umf[k] = 0.0; emf[k] = 0.0; slflx[k] = 0.0; qtflx[k] = 0.0; uflx[k] = 0.0; vflx[k] = 0.0;
-        ufrc[k] = 0.0; thlu[k] = 0.0; qtu[k] = 0.0; uu[k] = 0.0; vu[k] = 0.0; wu[k] = 0.0;
-        thvu[k] = 0.0; thlu_emf[k] = 0.0; qtu_emf[k] = 0.0; uu_emf[k] = 0.0; vu_emf[k] = 0.0;
-#pragma unroll 1
-        for (int m = 0; m < ncnst; m++) {
-            trflx[m][k] = 0.0;
-            tru[m][k] = 0.0;
-            tru_emf[m][k] = 0.0;
-        }
-    }
-#pragma unroll 1
-    for (int k = 1; k <= mkx; k++) {
-        qvten[k] = 0.0; qlten[k] = 0.0; qiten[k] = 0.0; sten[k] = 0.0; uten[k] = 0.0; vten[k] = 0.0;
-        qrten[k] = 0.0; qsten[k] = 0.0; dwten[k] = 0.0; diten[k] = 0.0; evapc[k] = 0.0;
-        cufrc[k] = 0.0; qcu[k] = 0.0; qlu[k] = 0.0; qiu[k] = 0.0; fer[k] = 0.0; fdr[k] = 0.0;
-        qc[k] = 0.0; qc_l[k] = 0.0; qc_i[k] = 0.0; qtten[k] = 0.0; slten[k] = 0.0;
-        qlten_sink[k] = 0.0; qiten_sink[k] = 0.0; nlten_sink[k] = 0.0; niten_sink[k] = 0.0;
-        rei[k] = 0.0; uf[k] = 0.0; vf[k] = 0.0;
-#pragma unroll 1
-        for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0;
-    }
+    // The Fortran zeroes some 80 profiles here and again at the implicit-CIN restore (:1333-1408,
+    // :1759-1889).  The sections below write every level that they, or the outputs, read (the zeroes
+    // outside the cloud included), each level once; only the per-level diagnostics show the others.
+    if (A.diag_level) ZERO_DIAG_PROFILES();
     cnt = (Tl)mkx;
     cnb = 0.0;
     }
     } else {   // uniform
-        // the state UW_MODE_LIST1 stored at the implicit-CIN branch of iteration 2 (uw_state.cuh),
-        // and the arrays that the set-up and that branch's restore build from the inputs, rebuilt
-        // with the same operations
+        // the state UW_MODE_LIST1 stored at the implicit-CIN branch of iteration 2 (uw_state.cuh), and
+        // the environment profiles that the set-up builds from the inputs, with the same operations
 #pragma unroll 1
         for (int k = 0; k <= mkx; k++) {
             ps0[k] = GI(ps0, k);
@@ -801,36 +766,10 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             s0[k] = GL(s0, k);
             qt0[k] = (qv0[k] + ql0[k] + qi0[k]);
             thl0[k] = (t0[k] - xlv * ql0[k] / cp - xls * qi0[k] / cp) / exn0[k];
-            thv0bot[k] = thv0bot_o[k];
-            thv0top[k] = thv0top_o[k];
-            thvl0bot[k] = thvl0bot_o[k];
-            thvl0top[k] = thvl0top_o[k];
         }
         slope<KP>(mkx, thl0, p0, ssthl0);
         slope<KP>(mkx, qt0, p0, ssqt0);
-#pragma unroll 1
-        for (int k = 0; k <= mkx; k++) {
-            umf[k] = 0.0; emf[k] = 0.0; slflx[k] = 0.0; qtflx[k] = 0.0; uflx[k] = 0.0;
-            vflx[k] = 0.0; ufrc[k] = 0.0; thlu[k] = 0.0; qtu[k] = 0.0; uu[k] = 0.0;
-            vu[k] = 0.0; wu[k] = 0.0; thvu[k] = 0.0; thlu_emf[k] = 0.0; qtu_emf[k] = 0.0;
-            uu_emf[k] = 0.0; vu_emf[k] = 0.0;
-#pragma unroll 1
-            for (int m = 0; m < ncnst; m++) {
-                trflx[m][k] = 0.0;
-                tru[m][k] = 0.0;
-                tru_emf[m][k] = 0.0;
-            }
-        }
-#pragma unroll 1
-        for (int k = 1; k <= mkx; k++) {
-            qvten[k] = 0.0; qlten[k] = 0.0; qiten[k] = 0.0; sten[k] = 0.0; uten[k] = 0.0;
-            vten[k] = 0.0; qrten[k] = 0.0; qsten[k] = 0.0; dwten[k] = 0.0; diten[k] = 0.0;
-            evapc[k] = 0.0; cufrc[k] = 0.0; qcu[k] = 0.0; qlu[k] = 0.0; qiu[k] = 0.0;
-            fer[k] = 0.0; fdr[k] = 0.0; qc[k] = 0.0; qc_l[k] = 0.0; qc_i[k] = 0.0;
-            qtten[k] = 0.0; slten[k] = 0.0;
-#pragma unroll 1
-            for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0;
-        }
+        if (A.diag_level) ZERO_DIAG_PROFILES();
     }
 
     UW_SYNC();
@@ -1044,37 +983,40 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 }
                 slope<KP>(mkx, thl0, p0, ssthl0);
                 slope<KP>(mkx, qt0, p0, ssqt0);
-#pragma unroll 1
-                for (int k = 0; k <= mkx; k++) {
-                    umf[k] = 0.0; emf[k] = 0.0; slflx[k] = 0.0; qtflx[k] = 0.0; uflx[k] = 0.0;
-                    vflx[k] = 0.0; ufrc[k] = 0.0; thlu[k] = 0.0; qtu[k] = 0.0; uu[k] = 0.0;
-                    vu[k] = 0.0; wu[k] = 0.0; thvu[k] = 0.0; thlu_emf[k] = 0.0; qtu_emf[k] = 0.0;
-                    uu_emf[k] = 0.0; vu_emf[k] = 0.0;
-#pragma unroll 1
-                    for (int m = 0; m < ncnst; m++) {
-                        trflx[m][k] = 0.0;
-                        tru[m][k] = 0.0;
-                        tru_emf[m][k] = 0.0;
-                    }
-                }
-#pragma unroll 1
-                for (int k = 1; k <= mkx; k++) {
-                    qvten[k] = 0.0; qlten[k] = 0.0; qiten[k] = 0.0; sten[k] = 0.0; uten[k] = 0.0;
-                    vten[k] = 0.0; qrten[k] = 0.0; qsten[k] = 0.0; dwten[k] = 0.0; diten[k] = 0.0;
-                    evapc[k] = 0.0; cufrc[k] = 0.0; qcu[k] = 0.0; qlu[k] = 0.0; qiu[k] = 0.0;
-                    fer[k] = 0.0; fdr[k] = 0.0; qc[k] = 0.0; qc_l[k] = 0.0; qc_i[k] = 0.0;
-                    qtten[k] = 0.0; slten[k] = 0.0;
-#pragma unroll 1
-                    for (int m = 0; m < ncnst; m++) trten[m][k] = 0.0;
-                }
+                if (A.diag_level) ZERO_DIAG_PROFILES();
                 precip = 0.0; snow = 0.0; rliq = 0.0; cbmf = 0.0;
                 cnt = (Tl)mkx; cnb = 0.0; ufrclcl = 0.0; wlcl = 0.0;
             } else {
-                // explicit CIN: the iteration-1 outputs already sit in the output slots (:1891-2011);
-                // flxprc1/flxsnow1 keep their initial zeros on this path, wu_out gets wu.
+                // explicit CIN: iteration 1's results are the column's (the Fortran's *_s copies,
+                // :1891-2011, :4177-4277).  The profiles still hold them (this iteration has rebuilt
+                // the environment only) and cush is in tscaleh; flxprc1/flxsnow1 are zero on this path.
                 lflags |= UW_L_DELCIN;
 #pragma unroll 1
-                for (int k = 0; k <= mkx; k++) { const Tl v_ = (wu[k]); OI(wu, k) = tl_val(v_); TOI(wu, k) = tl_der(v_); }
+                for (int k = 0; k <= mkx; k++) {
+                    { const Tl v_ = (umf[k]); OI(umf, k) = tl_val(v_); TOI(umf, k) = tl_der(v_); }
+                    { const Tl v_ = (wu[k]); OI(wu, k) = tl_val(v_); TOI(wu, k) = tl_der(v_); }
+                    { const Tl v_ = (slflx[k]); OI(slflx, k) = tl_val(v_); TOI(slflx, k) = tl_der(v_); }
+                    { const Tl v_ = (qtflx[k]); OI(qtflx, k) = tl_val(v_); TOI(qtflx, k) = tl_der(v_); }
+                    { const Tl v_ = (0.0); OI(flxprc1, k) = tl_val(v_); TOI(flxprc1, k) = tl_der(v_); }
+                    { const Tl v_ = (0.0); OI(flxsnow1, k) = tl_val(v_); TOI(flxsnow1, k) = tl_der(v_); }
+                }
+#pragma unroll 1
+                for (int k = 1; k <= mkx; k++) {
+                    { const Tl v_ = (qvten[k]); OL(qvten, k) = tl_val(v_); TOL(qvten, k) = tl_der(v_); } { const Tl v_ = (qlten[k]); OL(qlten, k) = tl_val(v_); TOL(qlten, k) = tl_der(v_); } { const Tl v_ = (qiten[k]); OL(qiten, k) = tl_val(v_); TOL(qiten, k) = tl_der(v_); }
+                    { const Tl v_ = (sten[k]); OL(sten, k) = tl_val(v_); TOL(sten, k) = tl_der(v_); } { const Tl v_ = (uten[k]); OL(uten, k) = tl_val(v_); TOL(uten, k) = tl_der(v_); } { const Tl v_ = (vten[k]); OL(vten, k) = tl_val(v_); TOL(vten, k) = tl_der(v_); }
+                    { const Tl v_ = (qrten[k]); OL(qrten, k) = tl_val(v_); TOL(qrten, k) = tl_der(v_); } { const Tl v_ = (qsten[k]); OL(qsten, k) = tl_val(v_); TOL(qsten, k) = tl_der(v_); } { const Tl v_ = (evapc[k]); OL(evapc, k) = tl_val(v_); TOL(evapc, k) = tl_der(v_); }
+                    { const Tl v_ = (cufrc[k]); OL(cufrc, k) = tl_val(v_); TOL(cufrc, k) = tl_der(v_); } { const Tl v_ = (qcu[k]); OL(qcu, k) = tl_val(v_); TOL(qcu, k) = tl_der(v_); } { const Tl v_ = (qlu[k]); OL(qlu, k) = tl_val(v_); TOL(qlu, k) = tl_der(v_); }
+                    { const Tl v_ = (qiu[k]); OL(qiu, k) = tl_val(v_); TOL(qiu, k) = tl_der(v_); } { const Tl v_ = (qc[k]); OL(qc, k) = tl_val(v_); TOL(qc, k) = tl_der(v_); }
+#pragma unroll 1
+                    for (int m = 1; m <= ncnst; m++) { const Tl v_ = (trten[m - 1][k]); OT(m, k) = tl_val(v_); TOT(m, k) = tl_der(v_); }
+                }
+                { const Tl v_ = (precip); A.precip[i] = tl_val(v_); T.precip[i] = tl_der(v_); }
+                { const Tl v_ = (snow); A.snow[i] = tl_val(v_); T.snow[i] = tl_der(v_); }
+                { const Tl v_ = (tscaleh); A.cush[i] = tl_val(v_); T.cush[i] = tl_der(v_); }
+                { const Tl v_ = (cbmf); A.cbmf[i] = tl_val(v_); T.cbmf[i] = tl_der(v_); }
+                { const Tl v_ = (rliq); A.rliq[i] = tl_val(v_); T.rliq[i] = tl_der(v_); }
+                A.cnt[i] = tl_val(CNT(cnt));
+                A.cnb[i] = tl_val(CNT(cnb));
                 if (A.diag_real) {
                     A.diag_real[UW_DR_CIN * (size_t)mix + i] = tl_val(cin_s);
                     A.diag_real[UW_DR_CINLCL * (size_t)mix + i] = tl_val(cinlcl_s);
@@ -1086,6 +1028,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     A.diag_real[UW_DR_TKEAVG * (size_t)mix + i] = tl_val(tkeavg_s);
                 }
                 kinv = kinv_s; klcl = klcl_s; klfc = klfc_s; krel = krel_s; kbup = kbup_s; kpen = kpen_s;
+                PUT_DIAG_LEVEL();
                 id_exit = false;
                 stop = true;
             break;
@@ -1186,10 +1129,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             ufrc[krel - 1] = ufrclcl;
 #pragma unroll 1
             for (int k = 0; k <= mkx; k++) {
-                if (k < kinv - 1 || k > krel - 1) continue;
-                umf[k] = cbmf;
-                wu[k] = winv;
+                const bool sub = k >= kinv - 1 && k <= krel - 1;
+                umf[k] = sub ? cbmf : 0.0;
+                wu[k] = sub ? winv : 0.0;
             }
+            fer[krel] = 0.0;   // read at kpen = krel when no level is left for the updraft
         }
         } while (0);
         if (MODE == UW_MODE_TRIGGER) {
@@ -1878,30 +1822,20 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         }
         lflags &= ~UW_L_SHCU;
 #pragma unroll 1
-        for (int k = 0; k <= mkx; k++) {
-            if (k < kpen) continue;
-            umf[k] = 0.0;
-            emf[k] = 0.0;
-            ufrc[k] = 0.0;
-        }
+        for (int k = kpen; k <= mkx; k++) umf[k] = 0.0;
+        ufrc[kpen] = 0.0;
+        if (A.diag_level) {
 #pragma unroll 1
-        for (int k = 0; k <= mkx; k++) {
-            if (k < kpen + 1) continue;
-            dwten[k] = 0.0;
-            diten[k] = 0.0;
-            fer[k] = 0.0;
-            fdr[k] = 0.0;
+            for (int k = kpen + 1; k <= mkx; k++) {
+                ufrc[k] = 0.0;
+                dwten[k] = 0.0;
+                diten[k] = 0.0;
+                fer[k] = 0.0;
+                fdr[k] = 0.0;
+            }
         }
         // penetrative entrainment (:3055-3183)
-#pragma unroll 1
-        for (int k = 0; k <= mkx; k++) {
-            thlu_emf[k] = thlu[k];
-            qtu_emf[k] = qtu[k];
-            uu_emf[k] = uu[k];
-            vu_emf[k] = vu[k];
-#pragma unroll 1
-            for (int m = 0; m < ncnst; m++) tru_emf[m][k] = tru[m][k];
-        }
+        // (the *_emf profiles are read at kbup .. kpen - 1 only)
 #pragma unroll 1
         for (int k = mkx; k >= 0; k--) {
             if (k > kpen - 1 || k < kbup) continue;
@@ -2021,14 +1955,20 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             for (int m = 0; m < ncnst; m++)
                 trflx[m][k] = emf[k] * (tru_emf[m][k] - (GT(m + 1, k) + sstr0[m][k] * (ps0[k] - p0[k])));
         }
+        // none above
+#pragma unroll 1
+        for (int k = MX(kpen, kbup); k <= mkx; k++) {
+            slflx[k] = 0.0;
+            qtflx[k] = 0.0;
+            uflx[k] = 0.0;
+            vflx[k] = 0.0;
+#pragma unroll 1
+            for (int m = 0; m < ncnst; m++) trflx[m][k] = 0.0;
+        }
         } while (0);
         UW_SYNC();
         // condensate tendency by compensating subsidence (:3416-3476)
         {
-            // uemf(k), evaluated on demand with the same expressions as :3416-3422
-#define UEMF(kk)                                                                                          \
-    ((kk) <= kinv - 2 ? cbmf * (ps0[0] - ps0[(kk)]) / (ps0[0] - ps0[kinv - 1])                             \
-                      : ((kk) <= krel - 1 ? cbmf : ((kk) <= kbup - 1 ? umf[(kk)] : ((kk) <= kpen - 1 ? emf[(kk)] : 0.0))))
             bool ldone = stop;
 #pragma unroll 1
             for (int k = 1; k <= mkx; k++) {   // uniform
@@ -2081,7 +2021,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         // momentum tendency (:3488-3501)
 #pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
-            if (k > kpen) continue;
+            if (k > kpen) {
+                uten[k] = 0.0;
+                vten[k] = 0.0;
+                continue;
+            }
             uten[k] = (uflx[k - 1] - uflx[k]) * g / dp0[k];
             vten[k] = (vflx[k - 1] - vflx[k]) * g / dp0[k];
             uf[k] = GL(u0, k) + uten[k] * dt;
@@ -2098,9 +2042,20 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             bool ldone = stop;
 #pragma unroll 1
             for (int k = 1; k <= mkx; k++) {   // uniform
-                if (k > kpen) ldone = true;
+                if (k > kpen) {
+                    ldone = true;
+                    qrten[k] = 0.0; qsten[k] = 0.0; qlten[k] = 0.0; qiten[k] = 0.0; qvten[k] = 0.0;
+                    sten[k] = 0.0; qc[k] = 0.0;
+                    trten[ixnumliq - 1][k] = 0.0;
+                    trten[ixnumice - 1][k] = 0.0;
+                }
                 if (!ldone) do {
                 const int km1 = k - 1;
+                if (k < krel) {   // below the updraft
+                    dwten[k] = 0.0;
+                    diten[k] = 0.0;
+                    fdr[k] = 0.0;
+                }
                 dwten[k] = dwten[k] * 0.5 * (umf[k - 1] + umf[k]) * g / dp0[k];
                 diten[k] = diten[k] * 0.5 * (umf[k - 1] + umf[k]) * g / dp0[k];
                 qrten[k] = frc_rasn * dwten[k];
@@ -2266,6 +2221,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     evpsnow = tmp2;
                 }
                 evapc[k] = evprain + evpsnow;
+                cufrc[k] = 0.0; qcu[k] = 0.0; qlu[k] = 0.0; qiu[k] = 0.0;   // in cloud: below
                 evpint_rain = evpint_rain + evprain * dp0[k] / g;
                 evpint_snow = evpint_snow + evpsnow * dp0[k] / g;
                 Tl ntraprd = qrten[k] - evprain + snowmlt;
@@ -2349,8 +2305,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         }
         // tracer tendencies (:4007-4076)
 #pragma unroll 1
-        for (int m = 4; m <= ncnst; m++) {
-            if (m != ixnumliq && m != ixnumice) {
+        for (int m = 1; m <= ncnst; m++) {
+            if (m < 4) {
+                if (m != ixnumliq && m != ixnumice) {   // qv, ql and qi: their tendencies are outputs of their own
+#pragma unroll 1
+                    for (int k = 1; k <= mkx; k++) trten[m - 1][k] = 0.0;
+                }
+            } else if (m != ixnumliq && m != ixnumice) {
                 const Tl trmin = c.qmin[m - 1];
                 const bool wet = c.wet[m - 1] != 0;
 #pragma unroll 1
@@ -2454,31 +2415,6 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         cnb = (Tl)(krel - 1);
 
         if (iter == 1) {
-            // Save the iteration-1 outputs into the output slots (the Fortran *_s copies, :4177-4277)
-#pragma unroll 1
-            for (int k = 0; k <= mkx; k++) {
-                { const Tl v_ = (umf[k]); OI(umf, k) = tl_val(v_); TOI(umf, k) = tl_der(v_); }
-                { const Tl v_ = (slflx[k]); OI(slflx, k) = tl_val(v_); TOI(slflx, k) = tl_der(v_); }
-                { const Tl v_ = (qtflx[k]); OI(qtflx, k) = tl_val(v_); TOI(qtflx, k) = tl_der(v_); }
-            }
-#pragma unroll 1
-            for (int k = 1; k <= mkx; k++) {
-                { const Tl v_ = (qvten[k]); OL(qvten, k) = tl_val(v_); TOL(qvten, k) = tl_der(v_); } { const Tl v_ = (qlten[k]); OL(qlten, k) = tl_val(v_); TOL(qlten, k) = tl_der(v_); } { const Tl v_ = (qiten[k]); OL(qiten, k) = tl_val(v_); TOL(qiten, k) = tl_der(v_); }
-                { const Tl v_ = (sten[k]); OL(sten, k) = tl_val(v_); TOL(sten, k) = tl_der(v_); } { const Tl v_ = (uten[k]); OL(uten, k) = tl_val(v_); TOL(uten, k) = tl_der(v_); } { const Tl v_ = (vten[k]); OL(vten, k) = tl_val(v_); TOL(vten, k) = tl_der(v_); }
-                { const Tl v_ = (qrten[k]); OL(qrten, k) = tl_val(v_); TOL(qrten, k) = tl_der(v_); } { const Tl v_ = (qsten[k]); OL(qsten, k) = tl_val(v_); TOL(qsten, k) = tl_der(v_); } { const Tl v_ = (evapc[k]); OL(evapc, k) = tl_val(v_); TOL(evapc, k) = tl_der(v_); }
-                { const Tl v_ = (cufrc[k]); OL(cufrc, k) = tl_val(v_); TOL(cufrc, k) = tl_der(v_); } { const Tl v_ = (qcu[k]); OL(qcu, k) = tl_val(v_); TOL(qcu, k) = tl_der(v_); } { const Tl v_ = (qlu[k]); OL(qlu, k) = tl_val(v_); TOL(qlu, k) = tl_der(v_); }
-                { const Tl v_ = (qiu[k]); OL(qiu, k) = tl_val(v_); TOL(qiu, k) = tl_der(v_); } { const Tl v_ = (qc[k]); OL(qc, k) = tl_val(v_); TOL(qc, k) = tl_der(v_); }
-#pragma unroll 1
-                for (int m = 1; m <= ncnst; m++) { const Tl v_ = (trten[m - 1][k]); OT(m, k) = tl_val(v_); TOT(m, k) = tl_der(v_); }
-            }
-            { const Tl v_ = (precip); A.precip[i] = tl_val(v_); T.precip[i] = tl_der(v_); }
-            { const Tl v_ = (snow); A.snow[i] = tl_val(v_); T.snow[i] = tl_der(v_); }
-            { const Tl v_ = (cush); A.cush[i] = tl_val(v_); T.cush[i] = tl_der(v_); }
-            { const Tl v_ = (cbmf); A.cbmf[i] = tl_val(v_); T.cbmf[i] = tl_der(v_); }
-            { const Tl v_ = (rliq); A.rliq[i] = tl_val(v_); T.rliq[i] = tl_der(v_); }
-            A.cnt[i] = tl_val(CNT(cnt));
-            A.cnb[i] = tl_val(CNT(cnb));
-            PUT_DIAG_LEVEL();
             cin_s = cin; cinlcl_s = cinlcl; plcl_s = plcl; pinv_s = ps0[kinv - 1]; plfc_s = plfc;
             pbup_s = ps0[kbup]; ppen_s = ps0[kpen - 1] + ppen; tkeavg_s = tkeavg;
             kinv_s = kinv; klcl_s = klcl; klfc_s = klfc; krel_s = krel; kbup_s = kbup; kpen_s = kpen;
@@ -2669,6 +2605,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 #undef TOI
 #undef DLV
 #undef PUT_DIAG_LEVEL
+#undef ZERO_DIAG_PROFILES
 #undef UEMF
 }
 

@@ -639,14 +639,15 @@ def run_batched(args):
                    "trigger_fraction": trig, "l2": "inputs larger than L2",
                    "launch": ("CUDA graph: per level class one trigger launch, a persistent first "
                               "worklist launch (4 blocks/SM) and a persistent resume launch (5 blocks/SM), "
-                              "3 sort kernels per member; autotuned block %d, %d column(s) per lane per "
+                              "2 ordering kernels per member; autotuned block %d, %d column(s) per lane per "
                               "task" % (tuned[0], tuned[2])
                               if sorted_plan else
                               "CUDA graph: per level class one trigger launch + one persistent worklist "
                               "launch; autotuned block %d, register cap %d blocks/SM, %d column(s) "
                               "per lane per task" % tuned),
                    "schedule": args.schedule},
-        "gpu_launches": args.steps * ((3 * nclass + 3 * len(BATCH_MEMBERS)) if sorted_plan else 2 * nclass),
+        "gpu_launches": args.steps * ((3 * nclass + 2 * len(BATCH_MEMBERS)) if sorted_plan else
+                                         2 * nclass + len(BATCH_MEMBERS)),
         "status": st,
         "roofline": {"fp64_algorithmic": fp64_alg},
         "precisions": others,
@@ -982,8 +983,8 @@ def main():
         "schedule": args.schedule,
         "precision": args.precision,
         "phases": phases,
-        # trigger + worklist; sorted: trigger, first worklist launch, 3 sort kernels, second launch
-        "gpu_launches": args.steps * ((6 if sorted_pass else 2) if two_phase else 1),
+        # trigger, worklist order, worklist; sorted: first worklist launch, hand-off order, second launch
+        "gpu_launches": args.steps * ((5 if sorted_pass else 3) if two_phase else 1),
         "status": st,
     }
     if e2e is not None:

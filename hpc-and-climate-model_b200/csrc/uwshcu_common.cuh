@@ -114,15 +114,14 @@ struct UwConst {
 // Hand-off between the two launches of the split worklist pass (UW_MODE_LIST1 -> UW_MODE_RESUME),
 // one region of device memory per stream that runs the pass.  Slots beyond cap are not handed off:
 // those columns finish in the first launch.
-#define UW_HAND_KEYS 64   // sort keys: 63 - iteration-1 updraft depth (deepest first)
+#define UW_HAND_KEYS 4096   // sort keys: 64 x release level + 63 - iteration-1 updraft depth (deepest first)
 struct UwHand {
     double* state;   // (uw_state_words, cap): word w of slot s at state[w * cap + s]
     int cap;         // slots
     int* count;      // slots requested by the first launch (may exceed cap)
     int* col;        // column of each slot
     int* key;        // sort key of each slot
-    int* order;      // slots in key order (counting sort)
-    int* hist;       // UW_HAND_KEYS counters of the sort
+    int* order;      // slots in key order, tile by tile
 };
 
 // One batch of the adjoint model (device addresses): slot t is worklist entry wl[b0 + t], t < nb, and
@@ -167,7 +166,24 @@ struct UwArgs {
     unsigned int *err;   // device error word
     const UwHand *hand;  // UW_MODE_LIST1 / UW_MODE_RESUME only: device copy of the hand-off region
     int *depth_key;      // optional (mix): each computed column's ordering key for the next call
+    unsigned char *trig_key;   // optional (mix), UW_MODE_TRIGGER: the release level of a column that goes on to the
+                         // worklist pass, 0 for the others; the caller builds the worklist from it
+    int spread;          // worklist launches: spread a short worklist over this many warps (0: full warps)
 };
+
+#if defined(__CUDACC__)
+// The worklist entry of thread tid, -1 for none: 32 per warp, or as few (a power of two) as spread the n
+// entries over at most `spread` warps.  The fewer columns a warp holds, the fewer branches it runs for
+// the others': 16 columns 8.5 -> 7.3 ms, 512 columns 9.5 -> 8.3 ms, 4,096 columns 9.9 -> 9.8 ms at one warp
+// per scheduler (592); at four per scheduler 4,096 columns take 11.4 ms (instruction fetch).
+__device__ __forceinline__ int uw_spread(int n, int spread, int tid)
+{
+    int lanes = 32;
+    while (lanes > 1 && (n + lanes / 2 - 1) / (lanes / 2) <= spread) lanes /= 2;
+    const int t = (tid >> 5) * lanes + (tid & 31);
+    return (tid & 31) < lanes && t < n ? t : -1;
+}
+#endif
 
 // ---- batched launches --------------------------------------------------------------------------
 // Members of one batch that share a level/tracer class run in one trigger launch and one persistent

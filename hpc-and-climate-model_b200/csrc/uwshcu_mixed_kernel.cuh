@@ -432,18 +432,22 @@ __device__ R findsp_point(R q, R t, R p, unsigned int& errbits, const double* __
 //   UW_MODE_ALL      every column 0..iend-1 runs the whole scheme (single pass);
 //   UW_MODE_TRIGGER  every column runs up to the end of the iteration-1 closure (uwshcu.F90:2184).
 //                    Columns that leave the scheme on the way write their final outputs (the
-//                    label-333 zeroes); the others are appended to the worklist `wl` (warp ballot,
-//                    one atomicAdd per warp) and write nothing;
-//   UW_MODE_LIST     thread t runs the whole scheme for column wl[t], t < *wl_count;
+//                    label-333 zeroes); the others write nothing and get their release level in
+//                    A.trig_key, from which the caller builds the worklist, or without A.trig_key
+//                    are appended to the worklist `wl` (warp ballot, one atomicAdd per warp);
+//   UW_MODE_LIST     runs the whole scheme for the columns wl[0 .. *wl_count), 32 to a warp or fewer
+//                    (uw_spread);
 //   UW_MODE_LIST1    as UW_MODE_LIST, except that a column taking the implicit-CIN branch of
 //                    iteration 2 (uwshcu.F90:1759-1889) stores its state in the hand-off region
 //                    A.hand (a free slot permitting) and stops there;
-//   UW_MODE_RESUME   thread t continues hand-off slot order[t] from that point to the end.
+//   UW_MODE_RESUME   continues the hand-off slots order[] from that point to the end.
 // The worklist path recomputes the phase-1 part of a convecting column instead of storing it: the
 // heavy buoyancy-sorting work then runs in warps made only of convecting columns.  The split at the
 // CIN decision drops the columns that end in iteration 1 or take the explicit-CIN branch from the
-// warps of iteration 2, and sorts the rest by their iteration-1 updraft depth, which predicts the
-// iteration-2 depth (lanes whose updraft has stopped wait for the deepest one in their warp).
+// warps of iteration 2, and sorts the rest by release level and iteration-1 updraft depth, which predicts
+// the iteration-2 depth (lanes whose updraft has stopped wait for the deepest one in their warp).  The
+// worklist itself is in order of the release level: lanes that start their updraft at the same level
+// access the same rows of their profiles, one line instead of one per level.
 #define UW_MODE_LIST1 3
 #define UW_MODE_RESUME 4
 #define UW_MODE_IS_LIST(m) ((m) == UW_MODE_LIST || (m) == UW_MODE_LIST1 || (m) == UW_MODE_RESUME)
@@ -1011,7 +1015,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                 const int slot = base + __popc(want & ((1u << ln) - 1u));
                 if (!stop && slot < H.cap) {
                     H.col[slot] = i;
-                    H.key[slot] = UW_HAND_KEYS - 1 - MN(MX(kpen_s - krel_s, 0), UW_HAND_KEYS - 1);
+                    H.key[slot] = krel_s * 64 + 63 - MN(MX(kpen_s - krel_s, 0), 63);
                     UW_SAVE_STATE(H.state + slot, (size_t)H.cap, tscaleh);
                     handed = true;
                     stop = true;
@@ -2530,9 +2534,10 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         A.depth_key[i] = ((lflags & UW_L_DELCIN) ? 0 : 64) + (depth < 0 ? 0 : (depth > 63 ? 63 : depth));
     }
     }
+    if (MODE == UW_MODE_TRIGGER && A.trig_key) A.trig_key[i] = (unsigned char)(cand ? krel : 0);
     if (errbits) atomicOr(A.err, errbits);
     }  // active
-    if (MODE == UW_MODE_TRIGGER) {
+    if (MODE == UW_MODE_TRIGGER && !A.trig_key) {
         // warp-aggregated append of this warp's candidates
         const unsigned lane = threadIdx.x & 31u;
         const unsigned mask = __ballot_sync(0xffffffffu, cand);
@@ -2585,12 +2590,13 @@ uwshcu_mixed_kernel(const __grid_constant__ UwArgs A, int* __restrict__ wl, int*
     int i;
     bool active;
     if (MODE == UW_MODE_LIST || MODE == UW_MODE_LIST1) {
-        active = tid < *wl_count;
-        i = active ? wl[tid] : 0;
+        const int t = uw_spread(*wl_count, A.spread, tid);
+        active = t >= 0;
+        i = active ? wl[t] : 0;
     } else if (MODE == UW_MODE_RESUME) {
-        const int n = MN(*A.hand->count, A.hand->cap);
-        active = tid < n;
-        i = active ? A.hand->order[tid] : 0;   // a hand-off slot
+        const int t = uw_spread(MN(*A.hand->count, A.hand->cap), A.spread, tid);
+        active = t >= 0;
+        i = active ? A.hand->order[t] : 0;   // a hand-off slot
     } else {
         active = tid < A.iend;
         i = tid;

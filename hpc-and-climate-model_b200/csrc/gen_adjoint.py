@@ -258,6 +258,9 @@ def main():
     s = s[: s.index("// ---- kernels ------")].rstrip() + "\n"
     s = rep(s, '#include "uw_math.h"', '#define UW_MATH_INLINE 1\n#include "uw_math.h"\n#include "uw_adj.h"\n\n#define UW_TAPE_ORDER 1')
     s = rep(s, '#include "uwshcu_common.cuh"', '#include "uwshcu_common.cuh"\n#include "uwshcu.h"')
+    # without the FP64-only conden
+    i0 = s.index("// ---- conden in FP64 (not in the generated kernels) ----")
+    s = s[:i0] + s[s.index("// The column code's saturation adjustment: one call", i0):]
     s = re.sub(r"\bdouble\b", "Ad", s)
     # tables and constants stay double
     s = s.replace("__constant__ Ad c_estbl[UW_TBL];", "__constant__ double c_estbl[UW_TBL];")

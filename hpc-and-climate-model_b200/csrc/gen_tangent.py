@@ -33,6 +33,14 @@ def main():
     # drop the batched and fast-mode kernels: the tangent kernel has its own launches
     s = s[: s.index("// Batched trigger pass: every column of every member of B")].rstrip() + "\n\n}  // namespace\n"
     s = rep(s, '#include "uw_math.h"', '#include "uw_math.h"\n#include "uw_dual.h"')
+    # the FP64-only conden is conden here
+    i0 = s.index("// ---- conden in FP64 (not in the generated kernels) ----")
+    i1 = s.index("// ---- end of conden in FP64 ----\n\n")
+    body = s[i0:i1]
+    out = body[body.index("struct CondenOut {"): body.index("__device__ __noinline__ CondenOut conden_any")]
+    s = s[:i0] + out + s[i1 + len("// ---- end of conden in FP64 ----\n\n"):]
+    s = rep(s, "    if (!FAST) return conden_f64(p, ex, thl, qt, tbl);\n    CondenOut r;\n    r.id = conden_fast(",
+            "    CondenOut r;\n    r.id = conden(")
     s = re.sub(r"\bdouble\b", "Tl", s)
     # tables stay double
     s = s.replace("__constant__ Tl c_estbl[UW_TBL];", "__constant__ double c_estbl[UW_TBL];")

@@ -93,7 +93,7 @@ struct UwConst {
     // uwshcu module (uwshcu.F90:25-37)
     double xlv, xlf, xls, cp, zvir, r, g, ep2, p00, rovcp, rpen;
     double rle, rkm, criqc;   // compute_uwshcu parameters (uwshcu.F90:1036, 1038, 1065)
-    double rinv;              // 1 / r, correctly rounded (divisions by r in conden)
+    double rinv, cpinv;       // 1 / r and 1 / cp, correctly rounded (divisions by r and cp in conden)
     // compute_zwshcu options (zwshcu.F90:30-59, cloud_fraction.F90:52), in force for calls that pass
     // omega: zmh_shallow_lf, zmh_shallow_ent, zmh_cloud_sh, zmh_shallow_fwcrit, zmh_ent0, zmh_ufrcd,
     // zmh_ufrc0, zmh_ufrcz
@@ -103,6 +103,7 @@ struct UwConst {
     double tmin, tmax, ttrice, epsqs, rgasv, hlatf, hlatv, cpws, tmelt;
     double pcf[6];
     double omeps, trinv;   // 1 - epsqs and 1/ttrice, as vqsatd computes them on every call
+    int tlo, tnum;         // high words of the doubles strictly between tmin and tmax: tlo .. tlo + tnum - 1
     double findsp_c3;      // rair (7.5 log 10) / cpws of findsp (uwshcu.F90:5164-5454)
     int icephs;
     // constituents

@@ -1043,6 +1043,7 @@ int uwshcu_init(double xlv, double cp, double xlf, double zvir, double r, double
     k.p00 = 1.e5;
     k.rovcp = k.r / k.cp;
     k.rinv = 1.0 / k.r;
+    k.cpinv = 1.0 / k.cp;
     k.rpen = rpen;
     k.rle = s.init ? s.k.rle : 0.1;       // uwshcu.F90:1036
     k.rkm = s.init ? s.k.rkm : 14.0;      // uwshcu.F90:1038
@@ -1075,6 +1076,16 @@ int uwshcu_init(double xlv, double cp, double xlf, double zvir, double r, double
     k.pcf[5] = 0.0;
     k.omeps = 1.0 - k.epsqs;
     k.trinv = (ttrice != 0.0) ? 1.0 / ttrice : 0.0;
+    {
+        auto high_word = [](double x) {
+            long long b;
+            std::memcpy(&b, &x, sizeof(b));
+            return (int)(b >> 32);
+        };
+        const bool ordered = tmin > 0.0 && tmax > tmin;   // the high words of positive doubles are in their order
+        k.tlo = ordered ? high_word(tmin) + 1 : 0;
+        k.tnum = ordered ? std::max(high_word(tmax) - k.tlo, 0) : 0;
+    }
     k.findsp_c3 = 287.04 * (7.5 * uw_log(10.0)) / k.cpws;
     k.ncnst = ncnst;
     k.ixnumliq = ixnumliq;

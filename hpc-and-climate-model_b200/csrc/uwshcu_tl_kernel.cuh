@@ -169,19 +169,18 @@ __device__ __forceinline__ int conden_fast(Tl p, Tl ex, Tl thl, Tl qt, Tl& th, T
     return id_check;
 }
 
-// The column code's saturation adjustment: one call for its ~20 sites (inlined at each of them, the stall
-// on instruction fetch doubled the run time), with the results by value, in registers (through
-// references they went through the stack, a store and a load each around every call).
 struct CondenOut {
     Tl th, qv, ql, qi, rv0;
     int id;
 };
+// The column code's saturation adjustment: one call for its ~20 sites (inlined at each of them, the stall
+// on instruction fetch doubled the run time), with the results by value, in registers (through
+// references they went through the stack, a store and a load each around every call).
 template <int FAST>
 __device__ __noinline__ CondenOut conden_out(Tl p, Tl ex, Tl thl, Tl qt, const double* __restrict__ tbl)
 {
     CondenOut r;
-    if (FAST) r.id = conden_fast(p, ex, thl, qt, r.th, r.qv, r.ql, r.qi, r.rv0, tbl);
-    else r.id = conden(p, ex, thl, qt, r.th, r.qv, r.ql, r.qi, r.rv0, tbl);
+    r.id = conden(p, ex, thl, qt, r.th, r.qv, r.ql, r.qi, r.rv0, tbl);
     return r;
 }
 template <int FAST>

@@ -453,8 +453,12 @@ __device__ Ad findsp_point(Ad q, Ad t, Ad p, unsigned int& errbits, const double
     }
 #pragma unroll 1
     for (int l = 1; l <= 8 && doit == 0; l++) {
+#if UW_TAPE_ORDER
         es = estblf(tsp, tbl);
         qs = MN(c.epsqs * es / (p - omeps * es), 1.0);
+#else
+        qs = qsp;   // es and qsp are those of tsp already
+#endif
         Ad tc = tsp - tt0;
         bool lflg = (tc >= -c.ttrice && tc < 0.0);
         Ad weight = MN(-tc * trinv, 1.0);
@@ -542,6 +546,8 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     // lanes of this warp that run a column; UW_SYNC() joins them where every one of them arrives
     const unsigned live = __ballot_sync(0xffffffffu, active);
 #define UW_SYNC() ad_align(live)
+// one level of slope: the limited slope from the difference quotients above and below
+#define UW_SLOPE(above, below) ((above) > 0.0 ? MX(0.0, MN(above, below)) : MN(0.0, MX(above, below)))
     if (active) {
 
     const int mix = A.mix, mkx = A.mkx, ncnst = A.ncnst;
@@ -617,7 +623,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     Ad flxrain[KP], flxsnow[KP], cufrc[KP], qcu[KP], qlu[KP], qiu[KP], trten[NC][KP];
     Ad qw0[KP], trflx_d[KP], trflx_u[KP];
 #if !UW_TAPE_ORDER
-    Ad qltop[KP], qitop[KP];
+    Ad qltop[KP], qitop[KP], env_thv[KP], env_exc[KP], env_rho[KP], env_rei[KP];
 #endif
     Ad trsrc[NC], tre[NC];
 
@@ -765,21 +771,6 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             p0[k] = GL(p0, k);
             dp0[k] = GL(dp0, k);
         }
-        {
-            Ad tmpf[KP];
-#pragma unroll 1
-            for (int k = 1; k <= mkx; k++) tmpf[k] = GL(u0, k);
-            slope<KP>(mkx, tmpf, p0, ssu0);
-#pragma unroll 1
-            for (int k = 1; k <= mkx; k++) tmpf[k] = GL(v0, k);
-            slope<KP>(mkx, tmpf, p0, ssv0);
-#pragma unroll 1
-            for (int m = 1; m <= ncnst; m++) {
-#pragma unroll 1
-                for (int k = 1; k <= mkx; k++) tmpf[k] = GT(m, k);
-                slope<KP>(mkx, tmpf, p0, sstr0[m - 1]);
-            }
-        }
 #pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             qv0[k] = Ad(GL(qv0, k), mkx + (k) - 1);
@@ -790,8 +781,52 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             qt0[k] = (qv0[k] + ql0[k] + qi0[k]);
             thl0[k] = (t0[k] - xlv * ql0[k] / cp - xls * qi0[k] / cp) / exn0[k];
         }
-        slope<KP>(mkx, thl0, p0, ssthl0);
-        slope<KP>(mkx, qt0, p0, ssqt0);
+        {
+            // as in the set-up
+            Ad pp = p0[1], pt = thl0[1], pq = qt0[1], pu = GL(u0, 1), pv = GL(v0, 1), bt = 0.0, bq = 0.0, bu = 0.0,
+                   bv = 0.0, ptr[NC], btr[NC];
+#pragma unroll (NC <= 5 ? NC : 1)
+            for (int m = 0; m < NC; m++) {
+                btr[m] = 0.0;
+                ptr[m] = 0.0;
+                if (m < ncnst) {
+                    ptr[m] = GT(m + 1, 1);
+                }
+            }
+#pragma unroll 1
+            for (int k = 2; k <= mkx; k++) {
+                const Ad xu = GL(u0, k), xv = GL(v0, k), xt = thl0[k], xq = qt0[k], xp = p0[k], dpk = xp - pp;
+                const Ad at = (xt - pt) / dpk, aq = (xq - pq) / dpk, au = (xu - pu) / dpk, av = (xv - pv) / dpk;
+                if (k == 2) {
+                    bt = at;
+                    bq = aq;
+                    bu = au;
+                    bv = av;
+                }
+                ssthl0[k - 1] = UW_SLOPE(at, bt);
+                ssqt0[k - 1] = UW_SLOPE(aq, bq);
+                ssu0[k - 1] = UW_SLOPE(au, bu);
+                ssv0[k - 1] = UW_SLOPE(av, bv);
+#pragma unroll (NC <= 5 ? NC : 1)
+                for (int m = 0; m < NC; m++) {
+                    if (m < ncnst) {
+                        const Ad xr = GT(m + 1, k), ar = (xr - ptr[m]) / dpk;
+                        if (k == 2) btr[m] = ar;
+                        sstr0[m][k - 1] = UW_SLOPE(ar, btr[m]);
+                        btr[m] = ar;
+                        ptr[m] = xr;
+                    }
+                }
+                pp = xp; pt = xt; pq = xq; pu = xu; pv = xv;
+                bt = at; bq = aq; bu = au; bv = av;
+            }
+            ssthl0[mkx] = ssthl0[mkx - 1];
+            ssqt0[mkx] = ssqt0[mkx - 1];
+            ssu0[mkx] = ssu0[mkx - 1];
+            ssv0[mkx] = ssv0[mkx - 1];
+#pragma unroll 1
+            for (int m = 0; m < ncnst; m++) sstr0[m][mkx] = sstr0[m][mkx - 1];
+        }
         if (A.diag_level) ZERO_DIAG_PROFILES();
     }
 
@@ -1218,6 +1253,9 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         UW_SYNC();
 
         {
+#if !UW_TAPE_ORDER
+            int kenv = krel - 1;   // the environment at the midpoints of layers krel .. kenv is known
+#endif
             Ad scaleh = tscaleh;
             if (tscaleh < 0.0) scaleh = 1000.0;
             // ---- buoyancy-sorting updraft, iter_scaleh loop (:2306-2952) ----------------------
@@ -1499,9 +1537,33 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     Ad wue = wu_b;
                     wtwb = wtw;
                     bool xdone = false;
-                    // environment at the layer midpoint: the same in both iter_xc passes, so the
-                    // second pass reuses the first one's results (same bits)
+                    // environment at the layer midpoint: the same in both iter_xc passes and in every
+                    // updraft of this iteration, so the first one to reach the level computes it
                     Ad thv0j = 0.0, excess0 = 0.0, reib = 0.0;
+                    if (k > kenv) {
+                        if (CONDEN(pe, exne, thle, qte, thj, qvj, qlj, qij, rvj, tbl)) {
+                            xflags |= UW_X_CONDEN;
+                            id_exit = true;
+                            stop = true;
+                            break;
+                        }
+                        thv0j = thj * (1.0 + zvir * qvj - qlj - qij);
+                        excess0 = qte - UW_QSAT_OF_CONDEN(thle * exne, pe);
+                        rho0j = pe / (r * thv0j * exne);
+                        reib = (0.5 * rkm / GL(z0, k) / g / rho0j);
+                        env_thv[k] = thv0j;
+                        env_exc[k] = excess0;
+                        env_rho[k] = rho0j;
+                        env_rei[k] = reib;
+                        kenv = k;
+                    } else {
+                        thv0j = env_thv[k];
+                        excess0 = env_exc[k];
+                        rho0j = env_rho[k];
+                        reib = env_rei[k];
+                    }
+                    Ad lgf = 0.0;        // the factor of the entrainment limit below, once it is needed
+                    bool lgf_set = false;
                     Ad thlu_k = 0.0, qtu_k = 0.0, thvu_k = 0.0, fer_k = 0.0, fdr_k = 0.0, rei_k = 0.0, ef_k = 0.0,
                            dmf_k = 0.0, dw_k = 0.0, di_k = 0.0;
                     const Ad cridis = rle * scaleh;
@@ -1509,18 +1571,6 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     for (int iter_xc = 1; iter_xc <= 2; iter_xc++) {
                         if (!xdone && !stop) do {
                         wtw = wu_b * wu_b;
-                        if (iter_xc == 1) {
-                            if (CONDEN(pe, exne, thle, qte, thj, qvj, qlj, qij, rvj, tbl)) {
-                                xflags |= UW_X_CONDEN;
-                                id_exit = true;
-                                stop = true;
-                                break;
-                            }
-                            thv0j = thj * (1.0 + zvir * qvj - qlj - qij);
-                            excess0 = qte - UW_QSAT_OF_CONDEN(thle * exne, pe);
-                            rho0j = pe / (r * thv0j * exne);
-                            reib = (0.5 * rkm / GL(z0, k) / g / rho0j);
-                        }
                         if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, rvj, tbl)) {
                             xflags |= UW_X_CONDEN;
                             id_exit = true;
@@ -1593,7 +1643,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                         Ad ee2 = xc * xc;
                         Ad ud2 = 1.0 - 2.0 * xc + xc * xc;
                         rei_k = reib;
-                        if (xc > 0.5) rei_k = MN(rei_k, 0.9 * uw_log(dp0[k] / g / dt / umf_b + 1.0) / dpe / (2.0 * xc - 1.0));
+                        if (xc > 0.5) {
+                            if (!lgf_set) {
+                                lgf = 0.9 * uw_log(dp0[k] / g / dt / umf_b + 1.0) / dpe;
+                                lgf_set = true;
+                            }
+                            rei_k = MN(rei_k, lgf / (2.0 * xc - 1.0));
+                        }
                         fer_k = rei_k * ee2;
                         fdr_k = rei_k * ud2;
                         // compute_zwshcu's entrainment option (zwshcu.F90:2818-2844)
@@ -2611,6 +2667,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         }
     }
 #undef UW_SYNC
+#undef UW_SLOPE
 #undef CONDEN
 #undef UW_QSAT_OF_CONDEN
 #undef RI

@@ -479,6 +479,8 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     // lanes of this warp that run a column; UW_SYNC() joins them where every one of them arrives
     const unsigned live = __ballot_sync(0xffffffffu, active);
 #define UW_SYNC() __syncwarp(live)
+// one level of slope: the limited slope from the difference quotients above and below
+#define UW_SLOPE(above, below) ((above) > 0.0f ? MX(0.0f, MN(above, below)) : MN(0.0f, MX(above, below)))
     if (active) {
 
     const int mix = A.mix, mkx = A.mkx, ncnst = A.ncnst;
@@ -552,7 +554,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     R flxrain[KP], flxsnow[KP], cufrc[KP], qcu[KP], qlu[KP], qiu[KP], trten[NC][KP];
     R qw0[KP], trflx_d[KP], trflx_u[KP];
 #if !UW_TAPE_ORDER
-    R qltop[KP], qitop[KP];
+    R qltop[KP], qitop[KP], env_thv[KP], env_exc[KP], env_rho[KP], env_rei[KP];
 #endif
     R trsrc[NC], tre[NC];
 
@@ -705,21 +707,6 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             p0[k] = GL(p0, k);
             dp0[k] = GL(dp0, k);
         }
-        {
-            R tmpf[KP];
-#pragma unroll 1
-            for (int k = 1; k <= mkx; k++) tmpf[k] = GL(u0, k);
-            slope<KP>(mkx, tmpf, p0, ssu0);
-#pragma unroll 1
-            for (int k = 1; k <= mkx; k++) tmpf[k] = GL(v0, k);
-            slope<KP>(mkx, tmpf, p0, ssv0);
-#pragma unroll 1
-            for (int m = 1; m <= ncnst; m++) {
-#pragma unroll 1
-                for (int k = 1; k <= mkx; k++) tmpf[k] = GT(m, k);
-                slope<KP>(mkx, tmpf, p0, sstr0[m - 1]);
-            }
-        }
 #pragma unroll 1
         for (int k = 1; k <= mkx; k++) {
             qv0[k] = GL(qv0, k);
@@ -730,8 +717,52 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
             qt0[k] = (qv0[k] + ql0[k] + qi0[k]);
             thl0[k] = (t0[k] - xlv * ql0[k] / cp - xls * qi0[k] / cp) / exn0[k];
         }
-        slope<KP>(mkx, thl0, p0, ssthl0);
-        slope<KP>(mkx, qt0, p0, ssqt0);
+        {
+            // as in the set-up
+            R pp = p0[1], pt = thl0[1], pq = qt0[1], pu = GL(u0, 1), pv = GL(v0, 1), bt = 0.0f, bq = 0.0f, bu = 0.0f,
+                   bv = 0.0f, ptr[NC], btr[NC];
+#pragma unroll (NC <= 5 ? NC : 1)
+            for (int m = 0; m < NC; m++) {
+                btr[m] = 0.0f;
+                ptr[m] = 0.0f;
+                if (m < ncnst) {
+                    ptr[m] = GT(m + 1, 1);
+                }
+            }
+#pragma unroll 1
+            for (int k = 2; k <= mkx; k++) {
+                const R xu = GL(u0, k), xv = GL(v0, k), xt = thl0[k], xq = qt0[k], xp = p0[k], dpk = xp - pp;
+                const R at = (xt - pt) / dpk, aq = (xq - pq) / dpk, au = (xu - pu) / dpk, av = (xv - pv) / dpk;
+                if (k == 2) {
+                    bt = at;
+                    bq = aq;
+                    bu = au;
+                    bv = av;
+                }
+                ssthl0[k - 1] = UW_SLOPE(at, bt);
+                ssqt0[k - 1] = UW_SLOPE(aq, bq);
+                ssu0[k - 1] = UW_SLOPE(au, bu);
+                ssv0[k - 1] = UW_SLOPE(av, bv);
+#pragma unroll (NC <= 5 ? NC : 1)
+                for (int m = 0; m < NC; m++) {
+                    if (m < ncnst) {
+                        const R xr = GT(m + 1, k), ar = (xr - ptr[m]) / dpk;
+                        if (k == 2) btr[m] = ar;
+                        sstr0[m][k - 1] = UW_SLOPE(ar, btr[m]);
+                        btr[m] = ar;
+                        ptr[m] = xr;
+                    }
+                }
+                pp = xp; pt = xt; pq = xq; pu = xu; pv = xv;
+                bt = at; bq = aq; bu = au; bv = av;
+            }
+            ssthl0[mkx] = ssthl0[mkx - 1];
+            ssqt0[mkx] = ssqt0[mkx - 1];
+            ssu0[mkx] = ssu0[mkx - 1];
+            ssv0[mkx] = ssv0[mkx - 1];
+#pragma unroll 1
+            for (int m = 0; m < ncnst; m++) sstr0[m][mkx] = sstr0[m][mkx - 1];
+        }
         if (A.diag_level) ZERO_DIAG_PROFILES();
     }
 
@@ -1158,6 +1189,9 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         UW_SYNC();
 
         {
+#if !UW_TAPE_ORDER
+            int kenv = krel - 1;   // the environment at the midpoints of layers krel .. kenv is known
+#endif
             R scaleh = tscaleh;
             if (tscaleh < 0.0f) scaleh = 1000.0f;
             // ---- buoyancy-sorting updraft, iter_scaleh loop (:2306-2952) ----------------------
@@ -1439,9 +1473,33 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     R wue = wu_b;
                     wtwb = wtw;
                     bool xdone = false;
-                    // environment at the layer midpoint: the same in both iter_xc passes, so the
-                    // second pass reuses the first one's results (same bits)
+                    // environment at the layer midpoint: the same in both iter_xc passes and in every
+                    // updraft of this iteration, so the first one to reach the level computes it
                     R thv0j = 0.0f, excess0 = 0.0f, reib = 0.0f;
+                    if (k > kenv) {
+                        if (CONDEN(pe, exne, thle, qte, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
+                            xflags |= UW_X_CONDEN;
+                            id_exit = true;
+                            stop = true;
+                            break;
+                        }
+                        thv0j = thj * (1.0f + zvir * qvj - qlj - qij);
+                        excess0 = qte - UW_QSAT_OF_CONDEN(thle * exne, pe);
+                        rho0j = pe / (r * thv0j * exne);
+                        reib = (0.5f * rkm / GL(z0, k) / g / rho0j);
+                        env_thv[k] = thv0j;
+                        env_exc[k] = excess0;
+                        env_rho[k] = rho0j;
+                        env_rei[k] = reib;
+                        kenv = k;
+                    } else {
+                        thv0j = env_thv[k];
+                        excess0 = env_exc[k];
+                        rho0j = env_rho[k];
+                        reib = env_rei[k];
+                    }
+                    R lgf = 0.0f;        // the factor of the entrainment limit below, once it is needed
+                    bool lgf_set = false;
                     R thlu_k = 0.0f, qtu_k = 0.0f, thvu_k = 0.0f, fer_k = 0.0f, fdr_k = 0.0f, rei_k = 0.0f, ef_k = 0.0f,
                            dmf_k = 0.0f, dw_k = 0.0f, di_k = 0.0f;
                     const R cridis = rle * scaleh;
@@ -1449,18 +1507,6 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                     for (int iter_xc = 1; iter_xc <= 2; iter_xc++) {
                         if (!xdone && !stop) do {
                         wtw = wu_b * wu_b;
-                        if (iter_xc == 1) {
-                            if (CONDEN(pe, exne, thle, qte, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
-                                xflags |= UW_X_CONDEN;
-                                id_exit = true;
-                                stop = true;
-                                break;
-                            }
-                            thv0j = thj * (1.0f + zvir * qvj - qlj - qij);
-                            excess0 = qte - UW_QSAT_OF_CONDEN(thle * exne, pe);
-                            rho0j = pe / (r * thv0j * exne);
-                            reib = (0.5f * rkm / GL(z0, k) / g / rho0j);
-                        }
                         if (CONDEN(pe, exne, thlue, qtue, thj, qvj, qlj, qij, rvj, tbld, tblf)) {
                             xflags |= UW_X_CONDEN;
                             id_exit = true;
@@ -1533,7 +1579,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                         R ee2 = xc * xc;
                         R ud2 = 1.0f - 2.0f * xc + xc * xc;
                         rei_k = reib;
-                        if (xc > 0.5f) rei_k = MN(rei_k, 0.9f * logf(dp0[k] / g / dt / umf_b + 1.0f) / dpe / (2.0f * xc - 1.0f));
+                        if (xc > 0.5f) {
+                            if (!lgf_set) {
+                                lgf = 0.9f * logf(dp0[k] / g / dt / umf_b + 1.0f) / dpe;
+                                lgf_set = true;
+                            }
+                            rei_k = MN(rei_k, lgf / (2.0f * xc - 1.0f));
+                        }
                         fer_k = rei_k * ee2;
                         fdr_k = rei_k * ud2;
                         // compute_zwshcu's entrainment option (zwshcu.F90:2818-2844)
@@ -2550,6 +2602,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
         }
     }
 #undef UW_SYNC
+#undef UW_SLOPE
 #undef CONDEN
 #undef UW_QSAT_OF_CONDEN
 #undef RI

@@ -125,8 +125,8 @@ __device__ __forceinline__ Ad operator-(Ad a, Ad b)
 __device__ __forceinline__ Ad operator*(Ad a, Ad b) { return ad_rec(a.v * b.v, a.i, b.v, b.i, a.v); }
 __device__ __forceinline__ Ad operator/(Ad a, Ad b)
 {
-    const double q = a.v / b.v;
-    return ad_rec(q, a.i, 1.0 / b.v, b.i, -q / b.v);
+    const UwQuotient r = uw_quotient(a.v, b.v);
+    return ad_rec(r.q, a.i, r.y, b.i, r.z);
 }
 __device__ __forceinline__ Ad operator-(Ad a) { return Ad(-a.v, ad_neg(a.i)); }
 __device__ __forceinline__ Ad operator+(Ad a) { return a; }
@@ -144,8 +144,8 @@ __device__ __forceinline__ double tl_val(double x) { return x; }
 
 __device__ __forceinline__ Ad uw_div_by(Ad a, Ad b, Ad y)
 {
-    const double q = uw_div_by(a.v, b.v, y.v);
-    return ad_rec(q, a.i, 1.0 / b.v, b.i, -q / b.v);
+    const double q = uw_div_by(a.v, b.v, y.v);   // y.v = RN(1 / b.v)
+    return ad_rec(q, a.i, y.v, b.i, uw_quot(-q, b.v, y.v));
 }
 __device__ __forceinline__ bool uw_isfinite(const Ad& x) { return isfinite(x.v); }
 __device__ __forceinline__ Ad uw_exp(Ad x)
@@ -209,8 +209,8 @@ __device__ __forceinline__ Fd4 operator-(const Fd4& a, const Fd4& b) { return fd
 __device__ __forceinline__ Fd4 operator*(const Fd4& a, const Fd4& b) { return fd4_lin(a.v * b.v, a, b.v, b, a.v); }
 __device__ __forceinline__ Fd4 operator/(const Fd4& a, const Fd4& b)
 {
-    const double q = a.v / b.v;
-    return fd4_lin(q, a, 1.0 / b.v, b, -q / b.v);
+    const UwQuotient r = uw_quotient(a.v, b.v);
+    return fd4_lin(r.q, a, r.y, b, r.z);
 }
 __device__ __forceinline__ Fd4 operator-(const Fd4& a) { return fd4_lin(-a.v, a, -1.0); }
 __device__ __forceinline__ bool operator<(const Fd4& a, const Fd4& b) { return a.v < b.v; }
@@ -219,8 +219,8 @@ __device__ __forceinline__ bool operator<=(const Fd4& a, const Fd4& b) { return 
 __device__ __forceinline__ bool operator>=(const Fd4& a, const Fd4& b) { return a.v >= b.v; }
 __device__ __forceinline__ Fd4 uw_div_by(const Fd4& a, const Fd4& b, const Fd4& y)
 {
-    const double q = uw_div_by(a.v, b.v, y.v);
-    return fd4_lin(q, a, 1.0 / b.v, b, -q / b.v);
+    const double q = uw_div_by(a.v, b.v, y.v);   // y.v = RN(1 / b.v)
+    return fd4_lin(q, a, y.v, b, uw_quot(-q, b.v, y.v));
 }
 __device__ __forceinline__ Fd4 fabs(const Fd4& x) { return fd4_lin(fabs(x.v), x, x.v < 0.0 ? -1.0 : 1.0); }
 __device__ __forceinline__ Fd4 trunc(const Fd4& x) { return Fd4(trunc(x.v)); }

@@ -62,6 +62,52 @@ UW_HD double uw_div_by(double a, double b, double y)
     return fma(e, y, q);
 }
 
+#if defined(__CUDACC__)
+// 1 / b correctly rounded, b within 2^+-100: the hardware's approximation (relative error below 2^-20), one
+// cubic step to about 2^-53, one Newton step with an exact residual (P. Markstein, IBM J. Res. Dev. 34
+// (1990) 111-119).  The one significand for which the last step fails, all ones, is left to the IEEE
+// division (uw_rcp_ok).
+static __device__ __forceinline__ double uw_rcp(double b)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    y = fma(y, fma(e, e, e), y);
+    return fma(y, fma(-b, y, 1.0), y);
+}
+// whether b lies within 2^+-100 (positive) and the low half of its significand is not all ones
+static __device__ __forceinline__ bool uw_rcp_ok(double b)
+{
+    return (unsigned)(__double2hiint(b) - 0x39b00000) < 0x0c800000u && __double2loint(b) != -1;
+}
+
+// x / b, every bit of it, from y = RN(1/b): uw_div_by where x and the quotient (and with them b) are within
+// 2^+-400, the IEEE division otherwise.
+static __device__ __noinline__ double uw_div_ieee(double x, double b) { return x / b; }
+static __device__ __forceinline__ double uw_quot(double x, double b, double y)
+{
+    const double q = UW_MUL(x, y);
+    const unsigned hx = (unsigned)__double2hiint(x) & 0x7fffffffu, hq = (unsigned)__double2hiint(q) & 0x7fffffffu;
+    if (hx - 0x27000000u < 0x31e00000u && hq - 0x27000000u < 0x31e00000u) {
+        const double e = fma(-b, q, x);
+        return fma(e, y, q);
+    }
+    return x == 0.0 && fabs(y) < HUGE_VAL ? q : uw_div_ieee(x, b);   // a zero numerator is common: no division
+}
+// A quotient and what its derivatives take: q = a / b, y = 1 / b, z = -q / b.
+struct UwQuotient {
+    double q, y, z;
+};
+static __device__ __forceinline__ UwQuotient uw_quotient(double a, double b)
+{
+    UwQuotient r;
+    r.y = 1.0 / b;
+    r.q = uw_quot(a, b, r.y);
+    r.z = uw_quot(-r.q, b, r.y);
+    return r;
+}
+#endif
+
 // ---------------------------------------------------------------------------------------------
 // Correctly rounded exp, log and pow (round to nearest), after Ziv's strategy (A. Ziv, "Fast
 // evaluation of elementary mathematical functions with correctly rounded last bit", ACM TOMS 17

@@ -199,24 +199,6 @@ __device__ __forceinline__ int conden_fast(double p, double ex, double thl, doub
 // conversion: a 16-column call takes 6.3 instead of 7.2 ms, 4,096 columns 8.6 instead of 9.7 ms, 1,048,576
 // columns (which wait for memory and instructions) 113.6 instead of 116.1 ms.
 
-// 1 / b correctly rounded, b within 2^+-100: the hardware's approximation (relative error below 2^-20), one
-// cubic step to about 2^-53, one Newton step with an exact residual (P. Markstein, IBM J. Res. Dev. 34
-// (1990) 111-119).  The one significand for which the last step fails, all ones, is left to the IEEE
-// division (uw_rcp_ok).
-__device__ __forceinline__ double uw_rcp(double b)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = fma(-b, y, 1.0);
-    y = fma(y, fma(e, e, e), y);
-    return fma(y, fma(-b, y, 1.0), y);
-}
-// whether b lies within 2^+-100 (positive) and the low half of its significand is not all ones
-__device__ __forceinline__ bool uw_rcp_ok(double b)
-{
-    return (unsigned)(__double2hiint(b) - 0x39b00000) < 0x0c800000u && __double2loint(b) != -1;
-}
-
 // qsat_qs; ok is cleared where the divisor is out of range.
 __device__ __forceinline__ double qsat_qs_f64(double t, double p, bool& ok, const double* __restrict__ tbl)
 {

@@ -94,10 +94,11 @@ def main():
     # the compute_zwshcu instantiation (ZW) is FP64 only: the tangent kernel is compute_uwshcu's
     s = s.replace("uw_column<KP, NC, MODE, 0, ZW>(A, tbl, i, active, wl, wl_count);",
                   "uw_column<KP, NC, MODE, 0>(A, tbl, i, active, wl, wl_count);")
-    s = s.replace("template <int KP, int NC, int MODE, int ZW = 0>\n__global__", "template <int KP, int NC, int MODE>\n__global__")
+    s = s.replace("template <int KP, int NC, int MODE, int ZW = 0, int DENSE = 0>\n__global__",
+                  "template <int KP, int NC, int MODE>\n__global__")
     s = rep(s, "uw_column<KP, NC, MODE, 0>(A, tbl, i, active, wl, wl_count);",
             "uw_column<KP, NC, MODE, 0>(A, tbl, i, active, wl, wl_count, T);")
-    s = rep(s, "__launch_bounds__(128, UW_LIST_MINB(MODE))", "__launch_bounds__(128)")
+    s = rep(s, "__launch_bounds__(128, UW_LIST_MINB(MODE, DENSE))", "__launch_bounds__(128)")
     # the split worklist pass (UW_MODE_LIST1 / UW_MODE_RESUME) is FP64 and FAST only: no state copies here
     s = re.sub(r"\n[ ]*UW_(SAVE|LOAD)_STATE\([^;]*\);", "", s)
     for u in ("TOI", "TOL", "TOT", "SEEDL", "SEEDI"):

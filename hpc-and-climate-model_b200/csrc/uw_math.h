@@ -81,9 +81,12 @@ static __device__ __forceinline__ bool uw_rcp_ok(double b)
     return (unsigned)(__double2hiint(b) - 0x39b00000) < 0x0c800000u && __double2loint(b) != -1;
 }
 
+static __device__ __noinline__ double uw_div_ieee(double x, double b)
+{
+    return x / b;
+}
 // x / b, every bit of it, from y = RN(1/b): uw_div_by where x and the quotient (and with them b) are within
 // 2^+-400, the IEEE division otherwise.
-static __device__ __noinline__ double uw_div_ieee(double x, double b) { return x / b; }
 static __device__ __forceinline__ double uw_quot(double x, double b, double y)
 {
     const double q = UW_MUL(x, y);

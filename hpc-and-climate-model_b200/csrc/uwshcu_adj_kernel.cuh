@@ -1262,12 +1262,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 #pragma unroll 1
             for (int iter_scaleh = 1; iter_scaleh <= 3; iter_scaleh++) {   // uniform
                 Ad pe = 0.0, dpe = 0.0, exne = 1.0, thvebot = 0.0, thle = 0.0, qte = 0.0, ue = 0.0, ve = 0.0;
+                const bool last = UW_TAPE_ORDER || iter_scaleh == 3;
 #if !UW_TAPE_ORDER
                 // The first two passes only find the scale height: the winds and tracers of the updraft feed
                 // nothing back into it, and of the level profiles only wu (an output at every level) and
                 // fer outlive the pass, so the last pass alone computes and stores the rest.  (The
-                // per-level diagnostics also show what an earlier, deeper pass left above the cloud top.)
-                const bool full = iter_scaleh == 3 || A.diag_level != nullptr;
+                // per-level diagnostics also show what an earlier, deeper pass left above the cloud top;
+                // they hold no tracers.)
+                const bool full = last || A.diag_level != nullptr;
                 // the updraft at the level below
                 Ad thlu_b = 0.0, qtu_b = 0.0, thvu_b = 0.0, umf_b = 0.0;
 #endif
@@ -1290,11 +1292,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 #endif
                     ue = GL(u0, krel) + ssu0[krel] * (pe - p0[krel]);
                     ve = GL(v0, krel) + ssv0[krel] * (pe - p0[krel]);
-#pragma unroll 1
-                    for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, krel) + sstr0[m][krel] * (pe - p0[krel]);
 #if !UW_TAPE_ORDER
                     }
 #endif
+#pragma unroll 1
+                    for (int m = 0; last && m < ncnst; m++) tre[m] = GT(m + 1, krel) + sstr0[m][krel] * (pe - p0[krel]);
                 }
 
 #if UW_TAPE_ORDER
@@ -1734,7 +1736,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             uu[k] = uu[km1] + (ue + ssu0[k] * dpe / 2.0 - uu[km1]) * fer_k * dpe - PGFc * ssu0[k] * dpe;
                             vu[k] = vu[km1] + (ve + ssv0[k] * dpe / 2.0 - vu[km1]) * fer_k * dpe - PGFc * ssv0[k] * dpe;
 #pragma unroll 1
-                            for (int m = 0; m < ncnst; m++)
+                            for (int m = 0; last && m < ncnst; m++)
                                 tru[m][k] = tru[m][km1] + (tre[m] + sstr0[m][k] * dpe / 2.0 - tru[m][km1]) * fer_k * dpe;
                         } else {
                             uu[k] = (ue + (1.0 - PGFc) * ssu0[k] / fer_k - ssu0[k] * dpe / 2.0) -
@@ -1742,7 +1744,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             vu[k] = (ve + (1.0 - PGFc) * ssv0[k] / fer_k - ssv0[k] * dpe / 2.0) -
                                     (ve + ssv0[k] * dpe / 2.0 - vu[km1] + (1.0 - PGFc) * ssv0[k] / fer_k) * ef_k;
 #pragma unroll 1
-                            for (int m = 0; m < ncnst; m++)
+                            for (int m = 0; last && m < ncnst; m++)
                                 tru[m][k] = (tre[m] + sstr0[m][k] / fer_k - sstr0[m][k] * dpe / 2.0) -
                                             (tre[m] + sstr0[m][k] * dpe / 2.0 - tru[m][km1] + sstr0[m][k] / fer_k) * ef_k;
                         }
@@ -1795,7 +1797,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                         ue = GL(u0, k + 1);
                         ve = GL(v0, k + 1);
 #pragma unroll 1
-                        for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, k + 1);
+                        for (int m = 0; last && m < ncnst; m++) tre[m] = GT(m + 1, k + 1);
                     }
                     } while (0);
                     if (stop) ldone = true;

@@ -22,6 +22,10 @@ extern "C" cudaError_t uw_fp64_launch_k64n5(const UwArgs* a, int mode, int* wl, 
         else if (mode == UW_MODE_LIST1) uwshcu_fp64_kernel<64, 5, UW_MODE_LIST1, 1><<<grid, block, 0, stream>>>(*a, wl, wl_count);
         else if (mode == UW_MODE_RESUME) uwshcu_fp64_kernel<64, 5, UW_MODE_RESUME, 1><<<grid, block, 0, stream>>>(*a, wl, wl_count);
         else uwshcu_fp64_kernel<64, 5, UW_MODE_LIST, 1><<<grid, block, 0, stream>>>(*a, wl, wl_count);
+    } else if (a->dense && mode == UW_MODE_LIST1) {
+        uwshcu_fp64_kernel<64, 5, UW_MODE_LIST1, 0, 1><<<grid, block, 0, stream>>>(*a, wl, wl_count);
+    } else if (a->dense && mode == UW_MODE_RESUME) {
+        uwshcu_fp64_kernel<64, 5, UW_MODE_RESUME, 0, 1><<<grid, block, 0, stream>>>(*a, wl, wl_count);
     } else {
         if (mode == UW_MODE_ALL) uwshcu_fp64_kernel<64, 5, UW_MODE_ALL><<<grid, block, 0, stream>>>(*a, wl, wl_count);
         else if (mode == UW_MODE_TRIGGER) uwshcu_fp64_kernel<64, 5, UW_MODE_TRIGGER><<<grid, block, 0, stream>>>(*a, wl, wl_count);
@@ -44,12 +48,14 @@ extern "C" cudaError_t uw_fp64_batch_k64n5(const UwBatch* b, int phase, int grid
         uwshcu_batch_trigger<64, 5, 0><<<grid, block, 0, stream>>>(*b);
         return cudaGetLastError();
     }
-    if (phase == 2) {   // sorted schedule: first worklist launch (register cap of minb 4)
-        uwshcu_batch_list<64, 5, 4, 0, UW_MODE_LIST1><<<grid, block, 0, stream>>>(*b);
+    if (phase == 2) {   // sorted schedule: first worklist launch (register cap of minb 4 or 7)
+        if (minb == 7) uwshcu_batch_list<64, 5, 7, 0, UW_MODE_LIST1><<<grid, block, 0, stream>>>(*b);
+        else uwshcu_batch_list<64, 5, 4, 0, UW_MODE_LIST1><<<grid, block, 0, stream>>>(*b);
         return cudaGetLastError();
     }
-    if (phase == 3) {   // sorted schedule: resume launch
-        uwshcu_batch_resume<64, 5, 0><<<grid, block, 0, stream>>>(*b);
+    if (phase == 3) {   // sorted schedule: resume launch (register cap of 5 or 7 blocks)
+        if (minb == 7) uwshcu_batch_resume<64, 5, 0, 7><<<grid, block, 0, stream>>>(*b);
+        else uwshcu_batch_resume<64, 5, 0><<<grid, block, 0, stream>>>(*b);
         return cudaGetLastError();
     }
     if (minb == 3) {

@@ -636,6 +636,12 @@ size_t key_ints(size_t n) { return (n + sizeof(int) - 1) / sizeof(int); }
 // shared between the streams that the caller has used or the chunks that run at the same time.
 int spread_warps(const DeviceState& d, int sharers) { return 4 * d.nsm / std::max(sharers, 1); }
 
+// Whether calls of so many columns at a time fill more than 4 blocks of worklist threads per SM (11/5 columns
+// per thread: 46 % of the benchmark soundings go on the worklist).  The launches then take more blocks of
+// fewer registers (UW_LIST_MINB): 163,840 columns 16.5 ms without and 18.0 ms with them, 196,608 columns 22.9 and
+// 19.9 ms, 262,144 columns 26.0 and 24.1 ms.
+int dense_call(const DeviceState& d, size_t columns) { return columns * 5 > (size_t)d.nsm * 4 * 128 * 11; }
+
 // dkey (optional): each column's ordering key, read to order list[] before the first worklist
 // launch and rewritten by it for the next call (uwshcu_set_depth_order).
 cudaError_t worklist_pass(HandRegion& h, UwArgs A, int* list, int* count, cudaStream_t st, int* dkey)
@@ -681,6 +687,7 @@ int enqueue(DeviceState& d, StreamCtx& c, UwArgs A, cudaStream_t st)
     int sharers = 0;
     for (const StreamCtx& x : d.sctx) sharers += x.used;
     A.spread = spread_warps(d, sharers);
+    A.dense = dense_call(d, A.iend);
     d.last_count = count;
     cudaEvent_t* ev = nullptr;
     if (s.profiling && d.nrec < DeviceState::kSlots) {
@@ -941,6 +948,7 @@ int host_call(int inv, int mix, int mkx, int iend, int ncnst, double dt, const d
                 return cuda_fail(e);
         } else {
             A.spread = spread_warps(*d, (int)std::min(nch, nstreams));
+            A.dense = dense_call(*d, std::min(n, csz * nstreams));
             if ((e = trigger_pass(A, keys + c0, wreg + 2, wreg, st)) != cudaSuccess) return cuda_fail(e);
             if ((e = worklist_pass(d->hand[1 + c % nstreams], A, wreg + 2, wreg, st,
                                    s.depth_order ? d->hkey + c0 : nullptr)) != cudaSuccess)
@@ -2145,6 +2153,9 @@ bool batch_has_minb(int prec, int cls, int minb)
     return minb == 4;
 }
 
+// the 7-block launches of the sorted schedule: FP64 with up to 5 tracers
+bool batch_has_dense(int prec, int cls) { return prec == UWSHCU_PREC_FP64 && cls < 2; }
+
 struct BatchPlan {
     int dev = 0;
     int prec = UWSHCU_PREC_FP64;  // precision mode at creation
@@ -2162,6 +2173,7 @@ struct BatchPlan {
     double* d_cush_save = nullptr; // autotune only
     int block = 128, minb = 4, chunk = 1;
     int nsm = 1;
+    bool dense[kClasses] = {};     // sorted schedule, per used class: enough columns for 7 blocks per SM (dense_call)
     cudaGraphExec_t exec = nullptr;
 };
 
@@ -2185,10 +2197,9 @@ int plan_enqueue(BatchPlan& P, cudaStream_t st)
     if (P.sorted) {
         // first worklist launch per class, the sort of each member's hand-off slots, resume launch
         for (int c = 0; c < P.ncls; c++) {
-            int per_sm = 0;
-            if ((e = batch_occupancy(P.prec, P.cls_id[c], 4, P.block, &per_sm)) != cudaSuccess) return cuda_fail(e);
-            if (per_sm <= 0) return UWSHCU_ERR_BAD_ARGS;
-            if ((e = batch_launch(P.prec, P.cls_id[c], &P.b[c], 2, P.nsm * per_sm, P.block, 4, st)) != cudaSuccess)
+            // the grid: the blocks of 128 threads (or twice as many of 64) that the register cap makes resident
+            const int minb = P.dense[c] ? 7 : 4;
+            if ((e = batch_launch(P.prec, P.cls_id[c], &P.b[c], 2, P.nsm * minb * (128 / P.block), P.block, minb, st)) != cudaSuccess)
                 return cuda_fail(e);
         }
         for (int j = 0; j < P.nm; j++) {
@@ -2197,9 +2208,11 @@ int plan_enqueue(BatchPlan& P, cudaStream_t st)
             if (n > 0) hand_tile_kernel<<<tiles(n), tile_threads(n), 0, st>>>(H);
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e);
-        for (int c = 0; c < P.ncls; c++)   // 5 resident blocks of 128 threads per SM (launch bounds)
-            if ((e = batch_launch(P.prec, P.cls_id[c], &P.b[c], 3, P.nsm * 5 * (128 / P.block), P.block, 0, st)) != cudaSuccess)
+        for (int c = 0; c < P.ncls; c++) {   // 5 or 7 resident blocks of 128 threads per SM (launch bounds)
+            const int minb = P.dense[c] ? 7 : 5;
+            if ((e = batch_launch(P.prec, P.cls_id[c], &P.b[c], 3, P.nsm * minb * (128 / P.block), P.block, minb, st)) != cudaSuccess)
                 return cuda_fail(e);
+        }
         return UWSHCU_OK;
     }
     for (int c = 0; c < P.ncls; c++) {
@@ -2309,6 +2322,9 @@ extern "C" int uwshcu_batch_create(int nmembers, const uwshcu_member* members, v
         for (int j = 0; j < b.nm; j++)
             b.block_start[j + 1] = b.block_start[j] + (b.m[j].iend + P->block - 1) / P->block;
         P->trig_grid[c] = b.block_start[b.nm];
+        size_t columns = 0;
+        for (int j = 0; j < b.nm; j++) columns += (size_t)b.m[j].iend;
+        P->dense[c] = dense_call(*d, columns) && batch_has_dense(P->prec, P->cls_id[c]);
     }
     *plan = P;
     return UWSHCU_OK;

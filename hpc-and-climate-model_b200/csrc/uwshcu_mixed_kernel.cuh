@@ -1198,12 +1198,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 #pragma unroll 1
             for (int iter_scaleh = 1; iter_scaleh <= 3; iter_scaleh++) {   // uniform
                 R pe = 0.0f, dpe = 0.0f, exne = 1.0f, thvebot = 0.0f, thle = 0.0f, qte = 0.0f, ue = 0.0f, ve = 0.0f;
+                const bool last = UW_TAPE_ORDER || iter_scaleh == 3;
 #if !UW_TAPE_ORDER
                 // The first two passes only find the scale height: the winds and tracers of the updraft feed
                 // nothing back into it, and of the level profiles only wu (an output at every level) and
                 // fer outlive the pass, so the last pass alone computes and stores the rest.  (The
-                // per-level diagnostics also show what an earlier, deeper pass left above the cloud top.)
-                const bool full = iter_scaleh == 3 || A.diag_level != nullptr;
+                // per-level diagnostics also show what an earlier, deeper pass left above the cloud top;
+                // they hold no tracers.)
+                const bool full = last || A.diag_level != nullptr;
                 // the updraft at the level below
                 R thlu_b = 0.0f, qtu_b = 0.0f, thvu_b = 0.0f, umf_b = 0.0f;
 #endif
@@ -1226,11 +1228,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 #endif
                     ue = GL(u0, krel) + ssu0[krel] * (pe - p0[krel]);
                     ve = GL(v0, krel) + ssv0[krel] * (pe - p0[krel]);
-#pragma unroll 1
-                    for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, krel) + sstr0[m][krel] * (pe - p0[krel]);
 #if !UW_TAPE_ORDER
                     }
 #endif
+#pragma unroll 1
+                    for (int m = 0; last && m < ncnst; m++) tre[m] = GT(m + 1, krel) + sstr0[m][krel] * (pe - p0[krel]);
                 }
 
 #if UW_TAPE_ORDER
@@ -1670,7 +1672,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             uu[k] = uu[km1] + (ue + ssu0[k] * dpe / 2.0f - uu[km1]) * fer_k * dpe - PGFc * ssu0[k] * dpe;
                             vu[k] = vu[km1] + (ve + ssv0[k] * dpe / 2.0f - vu[km1]) * fer_k * dpe - PGFc * ssv0[k] * dpe;
 #pragma unroll 1
-                            for (int m = 0; m < ncnst; m++)
+                            for (int m = 0; last && m < ncnst; m++)
                                 tru[m][k] = tru[m][km1] + (tre[m] + sstr0[m][k] * dpe / 2.0f - tru[m][km1]) * fer_k * dpe;
                         } else {
                             uu[k] = (ue + (1.0f - PGFc) * ssu0[k] / fer_k - ssu0[k] * dpe / 2.0f) -
@@ -1678,7 +1680,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             vu[k] = (ve + (1.0f - PGFc) * ssv0[k] / fer_k - ssv0[k] * dpe / 2.0f) -
                                     (ve + ssv0[k] * dpe / 2.0f - vu[km1] + (1.0f - PGFc) * ssv0[k] / fer_k) * ef_k;
 #pragma unroll 1
-                            for (int m = 0; m < ncnst; m++)
+                            for (int m = 0; last && m < ncnst; m++)
                                 tru[m][k] = (tre[m] + sstr0[m][k] / fer_k - sstr0[m][k] * dpe / 2.0f) -
                                             (tre[m] + sstr0[m][k] * dpe / 2.0f - tru[m][km1] + sstr0[m][k] / fer_k) * ef_k;
                         }
@@ -1731,7 +1733,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                         ue = GL(u0, k + 1);
                         ve = GL(v0, k + 1);
 #pragma unroll 1
-                        for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, k + 1);
+                        for (int m = 0; last && m < ncnst; m++) tre[m] = GT(m + 1, k + 1);
                     }
                     } while (0);
                     if (stop) ldone = true;
@@ -2626,9 +2628,9 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 // 1,048,576 x 30 columns: 103.9 ms against 115.6 ms at the FP64 kernel's 4 and 5 blocks, 109.8 ms
 // at 6, 104.5 ms at 8), the trigger pass at 72 too (7 blocks: 103.1-103.4 ms against 104.8 ms at 5),
 // the single pass at 168.
-#define UW_LIST_MINB(m) ((m) == UW_MODE_RESUME ? 7 : (UW_MODE_IS_LIST(m) ? 7 : ((m) == UW_MODE_TRIGGER ? 7 : 3)))
+#define UW_LIST_MINB(m, dense) ((m) == UW_MODE_RESUME ? 7 : (UW_MODE_IS_LIST(m) ? 7 : ((m) == UW_MODE_TRIGGER ? 7 : 3)))
 template <int KP, int NC, int MODE>
-__global__ void __launch_bounds__(128, UW_LIST_MINB(MODE))
+__global__ void __launch_bounds__(128, UW_LIST_MINB(MODE, 0))
 uwshcu_mixed_kernel(const __grid_constant__ UwArgs A, int* __restrict__ wl, int* __restrict__ wl_count)
 {
     __shared__ double tbld[UW_TBL];
@@ -2726,8 +2728,8 @@ __global__ void __launch_bounds__(128, MINB) uwshcu_batch_list(const __grid_cons
 // Batched resume launch of the sorted schedule, persistent: each warp takes the next task (32
 // consecutive entries of one member's hand-off slots in sorted order) from *B.task_head2 until every
 // member's slots are done.  Member m has min(*count, cap) slots in its region B.m[m].hand.
-template <int KP, int NC, int FAST>
-__global__ void __launch_bounds__(128, 5) uwshcu_batch_resume(const __grid_constant__ UwBatch B)
+template <int KP, int NC, int FAST, int MINB = 5>
+__global__ void __launch_bounds__(128, MINB) uwshcu_batch_resume(const __grid_constant__ UwBatch B)
 {
     __shared__ double tbld[UW_TBL];
     __shared__ float tblf[UW_TBL];

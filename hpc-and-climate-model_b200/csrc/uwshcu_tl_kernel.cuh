@@ -1242,12 +1242,14 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 #pragma unroll 1
             for (int iter_scaleh = 1; iter_scaleh <= 3; iter_scaleh++) {   // uniform
                 Tl pe = 0.0, dpe = 0.0, exne = 1.0, thvebot = 0.0, thle = 0.0, qte = 0.0, ue = 0.0, ve = 0.0;
+                const bool last = UW_TAPE_ORDER || iter_scaleh == 3;
 #if !UW_TAPE_ORDER
                 // The first two passes only find the scale height: the winds and tracers of the updraft feed
                 // nothing back into it, and of the level profiles only wu (an output at every level) and
                 // fer outlive the pass, so the last pass alone computes and stores the rest.  (The
-                // per-level diagnostics also show what an earlier, deeper pass left above the cloud top.)
-                const bool full = iter_scaleh == 3 || A.diag_level != nullptr;
+                // per-level diagnostics also show what an earlier, deeper pass left above the cloud top;
+                // they hold no tracers.)
+                const bool full = last || A.diag_level != nullptr;
                 // the updraft at the level below
                 Tl thlu_b = 0.0, qtu_b = 0.0, thvu_b = 0.0, umf_b = 0.0;
 #endif
@@ -1270,11 +1272,11 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 #endif
                     ue = GL(u0, krel) + ssu0[krel] * (pe - p0[krel]);
                     ve = GL(v0, krel) + ssv0[krel] * (pe - p0[krel]);
-#pragma unroll 1
-                    for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, krel) + sstr0[m][krel] * (pe - p0[krel]);
 #if !UW_TAPE_ORDER
                     }
 #endif
+#pragma unroll 1
+                    for (int m = 0; last && m < ncnst; m++) tre[m] = GT(m + 1, krel) + sstr0[m][krel] * (pe - p0[krel]);
                 }
 
 #if UW_TAPE_ORDER
@@ -1714,7 +1716,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             uu[k] = uu[km1] + (ue + ssu0[k] * dpe / 2.0 - uu[km1]) * fer_k * dpe - PGFc * ssu0[k] * dpe;
                             vu[k] = vu[km1] + (ve + ssv0[k] * dpe / 2.0 - vu[km1]) * fer_k * dpe - PGFc * ssv0[k] * dpe;
 #pragma unroll 1
-                            for (int m = 0; m < ncnst; m++)
+                            for (int m = 0; last && m < ncnst; m++)
                                 tru[m][k] = tru[m][km1] + (tre[m] + sstr0[m][k] * dpe / 2.0 - tru[m][km1]) * fer_k * dpe;
                         } else {
                             uu[k] = (ue + (1.0 - PGFc) * ssu0[k] / fer_k - ssu0[k] * dpe / 2.0) -
@@ -1722,7 +1724,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                             vu[k] = (ve + (1.0 - PGFc) * ssv0[k] / fer_k - ssv0[k] * dpe / 2.0) -
                                     (ve + ssv0[k] * dpe / 2.0 - vu[km1] + (1.0 - PGFc) * ssv0[k] / fer_k) * ef_k;
 #pragma unroll 1
-                            for (int m = 0; m < ncnst; m++)
+                            for (int m = 0; last && m < ncnst; m++)
                                 tru[m][k] = (tre[m] + sstr0[m][k] / fer_k - sstr0[m][k] * dpe / 2.0) -
                                             (tre[m] + sstr0[m][k] * dpe / 2.0 - tru[m][km1] + sstr0[m][k] / fer_k) * ef_k;
                         }
@@ -1775,7 +1777,7 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
                         ue = GL(u0, k + 1);
                         ve = GL(v0, k + 1);
 #pragma unroll 1
-                        for (int m = 0; m < ncnst; m++) tre[m] = GT(m + 1, k + 1);
+                        for (int m = 0; last && m < ncnst; m++) tre[m] = GT(m + 1, k + 1);
                     }
                     } while (0);
                     if (stop) ldone = true;
@@ -2672,13 +2674,16 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 
 // ---- kernels ---------------------------------------------------------------------------------------
 
-// Register caps (resident blocks of 128 per SM): the worklist launches at 128 registers (4 blocks
-// instead of 3 at their natural 168; the extra warps hide more FP64 and local-memory latency than
-// the added spills cost, -10 % time on the benchmark workload; 5 blocks cost +1.5 % for
-// UW_MODE_LIST1), the UW_MODE_RESUME launch, which spills less, at 85 (6 blocks: 177.1-177.4 ms
-// per 1,048,576-column step against 178.7-178.8 at 5 with the correctly rounded math routines),
-// the trigger pass at 102 (6 blocks: no change), the single pass at 168.
-#define UW_LIST_MINB(m) ((m) == UW_MODE_RESUME ? 6 : (UW_MODE_IS_LIST(m) ? 4 : ((m) == UW_MODE_TRIGGER ? 5 : 3)))
+// Register caps (resident blocks of 128 per SM).  The worklist launches take 128 and 85 registers (4 and 6
+// blocks) for short worklists, whose warps each run alone on their scheduler and lose to every spill, and
+// 72 (7 blocks) for those that fill more than 4 blocks per SM (`dense`), whose warps hide each other's
+// waits for memory and instructions.  LIST1 / RESUME blocks, ms per call of 16 / 65,536 / 163,840 / 262,144 /
+// 1,048,576 columns: 4 / 6: 6.3 / 11.4 / 17.1 / 26.5 / 113.6; 7 / 7: 6.6 / 11.9 / 18.6 / 24.6 / 107.9; 5 / 5, 6 / 6
+// and 8 / 8 are no better than these at either end.  The trigger pass takes 80 (6 blocks: 8.9 ms at
+// 1,048,576 columns, 9.6 ms at 5), the single pass 168.
+#define UW_LIST_MINB(m, dense)                                                                            \
+    ((m) == UW_MODE_RESUME ? ((dense) ? 7 : 6)                                                            \
+                           : (UW_MODE_IS_LIST(m) ? ((dense) ? 7 : 4) : ((m) == UW_MODE_TRIGGER ? 6 : 3)))
 template <int KP, int NC, int MODE>
 __global__ void __launch_bounds__(128)
 uwshcu_tl_kernel(const __grid_constant__ UwArgs A, int* __restrict__ wl, int* __restrict__ wl_count,

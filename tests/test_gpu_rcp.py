@@ -23,6 +23,7 @@ def kernels(cuda):
     torch = cuda
     math = open(os.path.join(CSRC, "uw_math.h")).read()
     src = ("#define UW_MUL(a, b) __dmul_rn((a), (b))\n#define HUGE_VAL __longlong_as_double(0x7ff0000000000000ll)\n"
+           + _function(math, "static __device__ __noinline__ double uw_div_ieee(")
            + "".join(_function(math, "static __device__ __forceinline__ " + f) for f in (
                "double uw_rcp(", "bool uw_rcp_ok(", "double uw_quot("))
            + "__device__ " + _function(math, "UW_HD double uw_div_by(")

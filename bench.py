@@ -54,15 +54,14 @@ G = 9.80616
 
 
 # From the ncu capture of the worklist pass on the 65,536-column case of this workload (29,956
-# worklist columns; summary in profiles/uwshcu_fp64_kernel_bench65k.txt, correctly rounded math,
-# non-finite check fused into the loads): DRAM bytes read + written per worklist column by its two
-# launches (UW_MODE_LIST1 7.420 GB + UW_MODE_RESUME 3.876 GB), and FP64 operations executed per
-# worklist column (2 x DFMA + DADD + DMUL thread instructions per cycle x cycles of each launch:
-# 707.70 x 17,051,704 + 561.79 x 14,282,396; the Newton steps of the IEEE divisions included).  Both
+# worklist columns; summary in profiles/uwshcu_fp64_kernel_bench65k.txt): DRAM bytes read + written per
+# worklist column by its two launches (UW_MODE_LIST1 3.953 GB + UW_MODE_RESUME 2.708 GB), and FP64
+# operations executed per worklist column (2 x DFMA + DADD + DMUL thread instructions per cycle x
+# cycles of each launch: 1021.90 x 10,627,641 + 721.55 x 10,037,494).  Both
 # scale with the columns a launch processes.  Constants of one capture: a change to the column code
 # needs a new capture (the command is in the summary).
-NCU_DRAM_BYTES_PER_LIST_COLUMN = 11.295961e9 / 29_956
-NCU_FP64_OPS_PER_LIST_COLUMN = (707.70 * 17_051_704 + 561.79 * 14_282_396) / 29_956
+NCU_DRAM_BYTES_PER_LIST_COLUMN = 6.661621e9 / 29_956
+NCU_FP64_OPS_PER_LIST_COLUMN = (1021.90 * 10_627_641 + 721.55 * 10_037_494) / 29_956
 FP64_DFMA_PER_CYCLE = 9472    # ncu sm__sass_thread_inst_executed_op_dfma_pred_on.sum.peak_sustained
 # Algorithmic FP64 operations per convecting / other column of each workload, counted by the
 # oracle's operation-counting build (written by oracle/opcount.py; a data file, read as text).

@@ -637,8 +637,8 @@ def run_batched(args):
                                "5 tracers, dt=1800 s", "pver": [m[1] for m in BATCH_MEMBERS],
                    "trigger_fraction": trig, "l2": "inputs larger than L2",
                    "launch": ("CUDA graph: per level class one trigger launch, a persistent first "
-                              "worklist launch (4 blocks/SM) and a persistent resume launch (5 blocks/SM), "
-                              "2 ordering kernels per member; autotuned block %d, %d column(s) per lane per "
+                              "worklist launch (4 blocks/SM, 7 for a class of more than 166,707 columns) and a "
+                              "persistent resume launch (5 or 7 blocks/SM), 2 ordering kernels per member; autotuned block %d, %d column(s) per lane per "
                               "task" % (tuned[0], tuned[2])
                               if sorted_plan else
                               "CUDA graph: per level class one trigger launch + one persistent worklist "

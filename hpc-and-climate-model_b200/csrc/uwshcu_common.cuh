@@ -8,6 +8,7 @@
 // and writes 32 consecutive doubles for every (k, m): level-major structure of arrays.
 #pragma once
 #include <cstdint>
+#include "uw_schedule.h"
 
 #define UW_NCMAX 32      // largest tracer count the kernels accept
 #define UW_TBL 250       // saturation-vapour-pressure table length (wv_saturation.F90:43)
@@ -172,20 +173,6 @@ struct UwArgs {
     int spread;          // worklist launches: spread a short worklist over this many warps (0: full warps)
     int dense;           // worklist launches: 1 for a call of enough columns to fill 7 blocks per SM (UW_LIST_MINB)
 };
-
-#if defined(__CUDACC__)
-// The worklist entry of thread tid, -1 for none: 32 per warp, or as few (a power of two) as spread the n
-// entries over at most `spread` warps.  The fewer columns a warp holds, the fewer branches it runs for
-// the others': 16 columns 8.5 -> 7.3 ms, 512 columns 9.5 -> 8.3 ms, 4,096 columns 9.9 -> 9.8 ms at one warp
-// per scheduler (592); at four per scheduler 4,096 columns take 11.4 ms (instruction fetch).
-__device__ __forceinline__ int uw_spread(int n, int spread, int tid)
-{
-    int lanes = 32;
-    while (lanes > 1 && (n + lanes / 2 - 1) / (lanes / 2) <= spread) lanes /= 2;
-    const int t = (tid >> 5) * lanes + (tid & 31);
-    return (tid & 31) < lanes && t < n ? t : -1;
-}
-#endif
 
 // ---- batched launches --------------------------------------------------------------------------
 // Members of one batch that share a level/tracer class run in one trigger launch and one persistent

@@ -497,9 +497,6 @@ __global__ void __launch_bounds__(kTileThreads) hand_tile_kernel(const UwHand* _
     for (int s = s0 + threadIdx.x; s < s1; s += blockDim.x) H->order[s0 + atomicAdd(&off[H->key[s]], 1)] = s;
 }
 
-// Threads of a worklist launch over at most n entries: one each, or a warp for each of `spread` warps.
-int list_threads(int n, int spread) { return n >= 32 * spread ? n : 32 * std::min(n, spread); }
-
 // Hand-off region r sized for calls of iend columns with mkx levels and ncnst tracers; nullptr when
 // the device has no room for it (the caller then runs the unsplit worklist pass).
 // Offset of the count in a hand-off region.
@@ -633,8 +630,15 @@ cudaError_t trigger_pass(UwArgs A, unsigned char* keys, int* list, int* count, c
 size_t key_ints(size_t n) { return (n + sizeof(int) - 1) / sizeof(int); }
 
 // Warps that a call's worklist launches spread a short worklist over (uw_spread): one per scheduler,
-// shared between the streams that the caller has used or the chunks that run at the same time.
+// shared between the streams in use (a captured call keeps what it was captured with) or the chunks that run
+// at the same time.
 int spread_warps(const DeviceState& d, int sharers) { return 4 * d.nsm / std::max(sharers, 1); }
+int spread_warps(const DeviceState& d)
+{
+    int sharers = 0;
+    for (const StreamCtx& x : d.sctx) sharers += x.used && uw_stream_shares(x.last, d.tick);
+    return spread_warps(d, sharers);
+}
 
 // Whether calls of so many columns at a time fill more than 4 blocks of worklist threads per SM (11/5 columns
 // per thread: 46 % of the benchmark soundings go on the worklist).  The launches then take more blocks of
@@ -654,18 +658,18 @@ cudaError_t worklist_pass(HandRegion& h, UwArgs A, int* list, int* count, cudaSt
     }
     const UwHand* H = nullptr;
     if (s.schedule == UWSHCU_SCHED_SORTED) H = hand_region(h, A.iend, A.mkx, A.ncnst);
-    if (!H) return launch_mode(&A, s.precision, kModeList, list, count, list_threads(A.iend, A.spread), s.block, st);
+    if (!H) return launch_mode(&A, s.precision, kModeList, list, count, uw_list_threads(A.iend, A.spread), s.block, st);
     cudaError_t e;
     A.hand = H;
     int* cnt = reinterpret_cast<int*>(h.base + kHandCountOffset);
     if ((e = cudaMemsetAsync(cnt, 0, sizeof(int), st)) != cudaSuccess) return e;
-    if ((e = launch_mode(&A, s.precision, kModeList1, list, count, list_threads(A.iend, A.spread), s.block, st)) != cudaSuccess)
+    if ((e = launch_mode(&A, s.precision, kModeList1, list, count, uw_list_threads(A.iend, A.spread), s.block, st)) != cudaSuccess)
         return e;
     const int slots = (int)std::min(h.cap, (size_t)A.iend);   // at most one per column of the call
     if (slots == 0) return cudaSuccess;
     hand_tile_kernel<<<tiles(slots), tile_threads(slots), 0, st>>>(H);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    return launch_mode(&A, s.precision, kModeResume, nullptr, nullptr, list_threads(slots, A.spread), s.block, st);
+    return launch_mode(&A, s.precision, kModeResume, nullptr, nullptr, uw_list_threads(slots, A.spread), s.block, st);
 }
 
 // Enqueue the column computation for A on st with the selected schedule.
@@ -684,9 +688,7 @@ int enqueue(DeviceState& d, StreamCtx& c, UwArgs A, cudaStream_t st)
     int* count = c.wl;
     int* list = c.wl + 1;
     unsigned char* keys = reinterpret_cast<unsigned char*>(list + A.iend);
-    int sharers = 0;
-    for (const StreamCtx& x : d.sctx) sharers += x.used;
-    A.spread = spread_warps(d, sharers);
+    A.spread = spread_warps(d);
     A.dense = dense_call(d, A.iend);
     d.last_count = count;
     cudaEvent_t* ev = nullptr;
@@ -1667,14 +1669,12 @@ int uwshcu_tangent_device(const uwshcu_member* m, const uwshcu_tangent* t, void*
     if ((rc = grow_ints(c->wl, c->wl_cap, (size_t)m->iend + 1 + key_ints(m->iend))) != UWSHCU_OK) return rc;
     int* wl = c->wl;
     A.trig_key = reinterpret_cast<unsigned char*>(wl + 1 + m->iend);
-    int sharers = 0;
-    for (const StreamCtx& x : d->sctx) sharers += x.used;
-    A.spread = spread_warps(*d, sharers);
+    A.spread = spread_warps(*d);
     if ((e = cudaMemsetAsync(wl, 0, sizeof(int), st)) != cudaSuccess) return cuda_fail(e);
     if ((e = launch(&A, t, kModeTrigger, wl + 1, wl, m->iend, 128, st)) != cudaSuccess) return cuda_fail(e);
     list_tile_kernel<<<tiles(m->iend), tile_threads(m->iend), 0, st>>>(A.trig_key, m->iend, wl + 1, wl);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e);
-    if ((e = launch(&A, t, kModeList, wl + 1, wl, list_threads(m->iend, A.spread), 128, st)) != cudaSuccess) return cuda_fail(e);
+    if ((e = launch(&A, t, kModeList, wl + 1, wl, uw_list_threads(m->iend, A.spread), 128, st)) != cudaSuccess) return cuda_fail(e);
     return UWSHCU_OK;
 }
 

@@ -32,3 +32,15 @@ UW_RULE int uw_list_threads(int n, int spread)
 // a single stream has them to itself from its 32nd call on.  (With every stream ever used counted, a process
 // that once ran on 32 of them spread its later calls over 18 warps: 256 columns 7.5 instead of 6.8 ms.)
 UW_RULE bool uw_stream_shares(unsigned long long last, unsigned long long tick) { return tick - last < 32; }
+
+// Worklist entries up to which the FP64 worklist launches take 4 (UW_MODE_RESUME 6, in a batch 5) resident blocks
+// of 128 threads per multiprocessor, and above which 7 (UW_LIST_MINB, `dense`): what 4 blocks hold.  A short
+// worklist's time is its slowest columns' chain, which the spills of the smaller register cap lengthen by 4 to 7 %; a
+// longer one at 4 blocks waits for a second wave.  Both caps, ms, at 148 multiprocessors (75,776 entries),
+// entries / columns: 12 levels 74,392 / 254,439 6.3 and 6.6, 77,808 / 266,393 6.9 and 6.7; 30 levels 74,444 / 162,480
+// 16.3 and 17.6, 77,922 / 170,113 19.7 and 18.0, of dry columns 74,726 / 395,925 18.9 and 19.7, 78,145 / 414,526 22.5
+// and 20.2, of moist ones 74,665 / 111,410 16.0 and 17.1, 78,116 / 116,644 19.8 and 18.0; 63 levels 74,352 35.4 and
+// 36.8, 77,871 40.7 and 37.6; 30 levels 458,106 101.9 and 98.8.  A plan with 64,197 and 65,410 entries in its two
+// classes 46.2 and 51.6, with 85,469 and 87,106 61.1 and 59.4.  (At 137,000 to 151,000 entries, two waves at either
+// cap, 4 blocks are 1 to 6 % faster from 30 levels on and up to 6 % slower below 20.)
+UW_RULE int uw_short_list(int multiprocessors) { return 4 * 128 * multiprocessors; }

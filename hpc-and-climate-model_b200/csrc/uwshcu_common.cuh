@@ -171,7 +171,7 @@ struct UwArgs {
     unsigned char *trig_key;   // optional (mix), UW_MODE_TRIGGER: the release level of a column that goes on to the
                          // worklist pass, 0 for the others; the caller builds the worklist from it
     int spread;          // worklist launches: spread a short worklist over this many warps (0: full warps)
-    int dense;           // worklist launches: 1 for a call of enough columns to fill 7 blocks per SM (UW_LIST_MINB)
+    int dense;           // worklist launches: 1 for the instantiations of 7 blocks per SM (UW_LIST_MINB)
 };
 
 // ---- batched launches --------------------------------------------------------------------------

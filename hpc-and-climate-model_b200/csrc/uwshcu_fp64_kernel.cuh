@@ -2768,13 +2768,13 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
 
 // ---- kernels ---------------------------------------------------------------------------------------
 
-// Register caps (resident blocks of 128 per SM).  The worklist launches take 128 and 85 registers (4 and 6
+// Register caps (resident blocks of 128 per SM).  The worklist launches take 128 and 80 registers (4 and 6
 // blocks) for short worklists, whose warps each run alone on their scheduler and lose to every spill, and
-// 72 (7 blocks) for those that fill more than 4 blocks per SM (`dense`), whose warps hide each other's
-// waits for memory and instructions.  LIST1 / RESUME blocks, ms per call of 16 / 65,536 / 163,840 / 262,144 /
-// 1,048,576 columns: 4 / 6: 6.3 / 11.4 / 17.1 / 26.5 / 113.6; 7 / 7: 6.6 / 11.9 / 18.6 / 24.6 / 107.9; 5 / 5, 6 / 6
-// and 8 / 8 are no better than these at either end.  The trigger pass takes 80 (6 blocks: 8.9 ms at
-// 1,048,576 columns, 9.6 ms at 5), the single pass 168.
+// 72 (7 blocks) for long ones (`dense`; where the line lies, with both sides measured: uw_short_list), whose
+// warps hide each other's waits for memory and instructions; 5, 6 and 8 blocks for both are no better at either
+// end.  Which it is the device decides by handing each of the two launches its count, the worklist's or 0: a
+// test of the length at the kernel's entry changed the compiler's code (1,048,576 columns 104.2 -> 106.0 ms).
+// The trigger pass takes 80 (6 blocks: 8.9 ms at 1,048,576 columns, 9.6 ms at 5), the single pass 168.
 #define UW_LIST_MINB(m, dense)                                                                            \
     ((m) == UW_MODE_RESUME ? ((dense) ? 7 : 6)                                                            \
                            : (UW_MODE_IS_LIST(m) ? ((dense) ? 7 : 4) : ((m) == UW_MODE_TRIGGER ? 6 : 3)))

@@ -499,15 +499,17 @@ __global__ void __launch_bounds__(kTileThreads) hand_tile_kernel(const UwHand* _
 
 // Hand-off region r sized for calls of iend columns with mkx levels and ncnst tracers; nullptr when
 // the device has no room for it (the caller then runs the unsplit worklist pass).
-// Offset of the count in a hand-off region.
-constexpr size_t kHandCountOffset = (sizeof(UwHand) + 255) & ~(size_t)255;
+// At the start of a hand-off region: its UwHand, and the same with the counts of the two resume launches
+// (cap_launches); at kHandCountOffset these counts.
+enum { kHandAll = 0, kHandShort = 1, kHandDense = 2 };
+constexpr size_t kHandCountOffset = (3 * sizeof(UwHand) + 255) & ~(size_t)255;
+int* hand_counts(const UwHand* H) { return reinterpret_cast<int*>((char*)H + kHandCountOffset); }
 
-// One hand-off region of cap slots of words doubles: its device UwHand at the start; nullptr when
-// the device has no room for it.
+// One hand-off region of cap slots of words doubles; nullptr when the device has no room for it.
 char* hand_alloc(size_t cap, size_t words)
 {
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    const size_t o_cnt = kHandCountOffset, o_col = o_cnt + up(sizeof(int)),
+    const size_t o_cnt = kHandCountOffset, o_col = o_cnt + up(3 * sizeof(int)),
                  o_key = o_col + up(cap * sizeof(int)), o_ord = o_key + up(cap * sizeof(int)),
                  o_st = o_ord + up(cap * sizeof(int)), bytes = o_st + words * cap * sizeof(double);
     char* base = nullptr;
@@ -515,14 +517,16 @@ char* hand_alloc(size_t cap, size_t words)
         cudaGetLastError();
         return nullptr;
     }
-    UwHand u{};
-    u.state = reinterpret_cast<double*>(base + o_st);
-    u.cap = (int)cap;
-    u.count = reinterpret_cast<int*>(base + o_cnt);
-    u.col = reinterpret_cast<int*>(base + o_col);
-    u.key = reinterpret_cast<int*>(base + o_key);
-    u.order = reinterpret_cast<int*>(base + o_ord);
-    if (cudaMemcpy(base, &u, sizeof(u), cudaMemcpyHostToDevice) != cudaSuccess) {
+    UwHand u[3]{};
+    for (int j = 0; j < 3; j++) {
+        u[j].state = reinterpret_cast<double*>(base + o_st);
+        u[j].cap = (int)cap;
+        u[j].count = reinterpret_cast<int*>(base + o_cnt) + j;
+        u[j].col = reinterpret_cast<int*>(base + o_col);
+        u[j].key = reinterpret_cast<int*>(base + o_key);
+        u[j].order = reinterpret_cast<int*>(base + o_ord);
+    }
+    if (cudaMemcpy(base, u, sizeof(u), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(base);
         return nullptr;
@@ -640,15 +644,68 @@ int spread_warps(const DeviceState& d)
     return spread_warps(d, sharers);
 }
 
-// Whether calls of so many columns at a time fill more than 4 blocks of worklist threads per SM (11/5 columns
-// per thread: 46 % of the benchmark soundings go on the worklist).  The launches then take more blocks of
-// fewer registers (UW_LIST_MINB): 163,840 columns 16.5 ms without and 18.0 ms with them, 196,608 columns 22.9 and
-// 19.9 ms, 262,144 columns 26.0 and 24.1 ms.
-int dense_call(const DeviceState& d, size_t columns) { return columns * 5 > (size_t)d.nsm * 4 * 128 * 11; }
+// A worklist pass whose worklist may be short or long (uw_short_list) is launched at both register caps, each launch
+// with counts of its own: those of the pass in one, 0 in the other, whose warps then leave at once (the 4-block
+// launches of 1,048,576 columns in 0.005 ms each).  m lists: one, or those of the members of one level class.
+struct CapCounts {
+    int m, limit;
+    const int* list[UW_MAXM];   // their worklist lengths, which decide together
+    const int* n[UW_MAXM];      // what the launches work on: the worklists or the hand-off slots
+    int* few[UW_MAXM];          // counts of the 4-block launch
+    int* many[UW_MAXM];         // and of the 7-block one
+};
+__global__ void cap_counts_kernel(const __grid_constant__ CapCounts C)
+{
+    long long total = 0;
+    for (int j = 0; j < C.m; j++) total += *C.list[j];
+    const bool dense = total > C.limit;
+    for (int j = 0; j < C.m; j++) {
+        *C.few[j] = dense ? 0 : *C.n[j];
+        *C.many[j] = dense ? *C.n[j] : 0;
+    }
+}
+cudaError_t cap_counts(const CapCounts& C, cudaStream_t st)
+{
+    cap_counts_kernel<<<1, 1, 0, st>>>(C);
+    return cudaGetLastError();
+}
+
+// The worklist length above which a pass over `columns` takes the 7-block launches, 0 where none is that long or they
+// do not exist (they do for compute_uwshcu in FP64 with up to 5 tracers).
+int short_list(const DeviceState& d, size_t columns, int prec, int ncnst, bool zw)
+{
+    const int limit = uw_short_list(d.nsm);
+    return prec == UWSHCU_PREC_FP64 && ncnst <= 5 && !zw && columns > (size_t)limit ? limit : 0;
+}
+
+// The two worklist launches of the split pass at both register caps; limit: short_list.
+cudaError_t cap_launches(UwArgs A, const UwHand* H, int* list, int* count, int slots, int limit, int block, cudaStream_t st)
+{
+    int* const cnt = hand_counts(H);
+    CapCounts C{1, limit, {count}, {count}, {cnt + kHandShort}, {cnt + kHandDense}};
+    cudaError_t e = cap_counts(C, st);
+    for (int dense = 0; dense < 2 && e == cudaSuccess; dense++) {
+        A.dense = dense;
+        e = launch_mode(&A, UWSHCU_PREC_FP64, kModeList1, list, dense ? C.many[0] : C.few[0],
+                        uw_list_threads(dense ? A.iend : std::min(A.iend, limit), A.spread), block, st);
+    }
+    if (e != cudaSuccess || slots == 0) return e;
+    hand_tile_kernel<<<tiles(slots), tile_threads(slots), 0, st>>>(H);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    C.n[0] = cnt;
+    e = cap_counts(C, st);
+    for (int dense = 0; dense < 2 && e == cudaSuccess; dense++) {
+        A.dense = dense;
+        A.hand = H + (dense ? kHandDense : kHandShort);
+        e = launch_mode(&A, UWSHCU_PREC_FP64, kModeResume, nullptr, nullptr,
+                        uw_list_threads(dense ? slots : std::min(slots, limit), A.spread), block, st);
+    }
+    return e;
+}
 
 // dkey (optional): each column's ordering key, read to order list[] before the first worklist
-// launch and rewritten by it for the next call (uwshcu_set_depth_order).
-cudaError_t worklist_pass(HandRegion& h, UwArgs A, int* list, int* count, cudaStream_t st, int* dkey)
+// launch and rewritten by it for the next call (uwshcu_set_depth_order).  limit: short_list.
+cudaError_t worklist_pass(HandRegion& h, UwArgs A, int* list, int* count, cudaStream_t st, int* dkey, int limit)
 {
     State& s = S();
     if (dkey) {
@@ -661,11 +718,11 @@ cudaError_t worklist_pass(HandRegion& h, UwArgs A, int* list, int* count, cudaSt
     if (!H) return launch_mode(&A, s.precision, kModeList, list, count, uw_list_threads(A.iend, A.spread), s.block, st);
     cudaError_t e;
     A.hand = H;
-    int* cnt = reinterpret_cast<int*>(h.base + kHandCountOffset);
-    if ((e = cudaMemsetAsync(cnt, 0, sizeof(int), st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(hand_counts(H), 0, sizeof(int), st)) != cudaSuccess) return e;
+    const int slots = (int)std::min(h.cap, (size_t)A.iend);   // at most one per column of the call
+    if (limit > 0) return cap_launches(A, H, list, count, slots, limit, s.block, st);
     if ((e = launch_mode(&A, s.precision, kModeList1, list, count, uw_list_threads(A.iend, A.spread), s.block, st)) != cudaSuccess)
         return e;
-    const int slots = (int)std::min(h.cap, (size_t)A.iend);   // at most one per column of the call
     if (slots == 0) return cudaSuccess;
     hand_tile_kernel<<<tiles(slots), tile_threads(slots), 0, st>>>(H);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -689,7 +746,6 @@ int enqueue(DeviceState& d, StreamCtx& c, UwArgs A, cudaStream_t st)
     int* list = c.wl + 1;
     unsigned char* keys = reinterpret_cast<unsigned char*>(list + A.iend);
     A.spread = spread_warps(d);
-    A.dense = dense_call(d, A.iend);
     d.last_count = count;
     cudaEvent_t* ev = nullptr;
     if (s.profiling && d.nrec < DeviceState::kSlots) {
@@ -707,7 +763,8 @@ int enqueue(DeviceState& d, StreamCtx& c, UwArgs A, cudaStream_t st)
         if ((rc = grow_keys(c.dkey, c.dkey_cap, (size_t)A.iend)) != UWSHCU_OK) return rc;
         dkey = c.dkey;
     }
-    if ((e = worklist_pass(c.hand, A, list, count, st, dkey)) != cudaSuccess) return cuda_fail(e);
+    const int limit = short_list(d, A.iend, s.precision, A.ncnst, A.omega != nullptr);
+    if ((e = worklist_pass(c.hand, A, list, count, st, dkey, limit)) != cudaSuccess) return cuda_fail(e);
     if (ev && (e = cudaEventRecord(ev[2], st)) != cudaSuccess) return cuda_fail(e);
     return UWSHCU_OK;
 }
@@ -950,10 +1007,12 @@ int host_call(int inv, int mix, int mkx, int iend, int ncnst, double dt, const d
                 return cuda_fail(e);
         } else {
             A.spread = spread_warps(*d, (int)std::min(nch, nstreams));
-            A.dense = dense_call(*d, std::min(n, csz * nstreams));
             if ((e = trigger_pass(A, keys + c0, wreg + 2, wreg, st)) != cudaSuccess) return cuda_fail(e);
             if ((e = worklist_pass(d->hand[1 + c % nstreams], A, wreg + 2, wreg, st,
-                                   s.depth_order ? d->hkey + c0 : nullptr)) != cudaSuccess)
+                                   s.depth_order ? d->hkey + c0 : nullptr,
+                                   // by the chunk's own worklist: by that of the chunks in flight, 500,000 and 700,000
+                                   // moist columns took 112 and 135 ms instead of 106 and 124
+                                   short_list(*d, nc, s.precision, ncnst, omega != nullptr))) != cudaSuccess)
                 return cuda_fail(e);
         }
         if ((e = cudaEventRecord(d->ev_comp[c], st)) != cudaSuccess) return cuda_fail(e);
@@ -2153,9 +2212,6 @@ bool batch_has_minb(int prec, int cls, int minb)
     return minb == 4;
 }
 
-// the 7-block launches of the sorted schedule: FP64 with up to 5 tracers
-bool batch_has_dense(int prec, int cls) { return prec == UWSHCU_PREC_FP64 && cls < 2; }
-
 struct BatchPlan {
     int dev = 0;
     int prec = UWSHCU_PREC_FP64;  // precision mode at creation
@@ -2165,22 +2221,58 @@ struct BatchPlan {
     int cls_id[kClasses];          // class of each used slot
     UwBatch b[kClasses];           // per used class
     int trig_grid[kClasses];
-    int* d_scratch = nullptr;      // [0, 64): counts of all members, [64, 64 + kClasses): task heads,
-                                   // [64 + kClasses, 64 + 2 kClasses): resume task heads, worklists, trigger keys
+    int* d_scratch = nullptr;      // [0, 64): counts of all members, and from kShortCounts and kDenseCounts on those
+                                   // of the launches at either register cap; [64, 64 + kClasses): task heads,
+                                   // [64 + kClasses, 64 + 2 kClasses): resume task heads, the same of the 7-block
+                                   // launches, from 64 + 4 kClasses on worklists, trigger keys
     bool sorted = false;           // created under the sorted schedule, with a region per member
     char* hand[UWSHCU_MAX_MEMBERS] = {};
     unsigned int* d_err = nullptr;
     double* d_cush_save = nullptr; // autotune only
     int block = 128, minb = 4, chunk = 1;
     int nsm = 1;
-    bool dense[kClasses] = {};     // sorted schedule, per used class: enough columns for 7 blocks per SM (dense_call)
+    int limit[kClasses] = {};      // sorted schedule, per used class: short_list
     cudaGraphExec_t exec = nullptr;
 };
+
+constexpr int kShortCounts = 16, kDenseCounts = 32;
+static_assert(UWSHCU_MAX_MEMBERS <= 16, "the counts of all members before kShortCounts");
+
+// One phase of class c in the sorted schedule: the worklists (phase 2) or their hand-off slots (3), with minb
+// resident blocks of 128 threads per SM (twice as many of 64), or at both register caps (P.limit).
+cudaError_t plan_list(BatchPlan& P, int c, int phase, int minb, cudaStream_t st)
+{
+    const int per_sm = P.nsm * (128 / P.block);
+    const UwBatch& b = P.b[c];
+    if (P.limit[c] == 0) return batch_launch(P.prec, P.cls_id[c], &b, phase, per_sm * minb, P.block, minb, st);
+    CapCounts C{};
+    C.m = b.nm;
+    C.limit = P.limit[c];
+    for (int j = 0; j < b.nm; j++) {
+        int* const cnt = hand_counts(b.m[j].hand);
+        C.list[j] = b.count + j;
+        C.n[j] = phase == 2 ? b.count + j : cnt;
+        C.few[j] = phase == 2 ? b.count + kShortCounts + j : cnt + kHandShort;
+        C.many[j] = phase == 2 ? b.count + kDenseCounts + j : cnt + kHandDense;
+    }
+    cudaError_t e = cap_counts(C, st);
+    for (int dense = 0; dense < 2 && e == cudaSuccess; dense++) {
+        UwBatch x = b;
+        if (phase == 2) x.count = b.count + (dense ? kDenseCounts : kShortCounts);
+        for (int j = 0; j < b.nm && phase == 3; j++) x.m[j].hand = b.m[j].hand + (dense ? kHandDense : kHandShort);
+        // the launch without work takes a task for every warp: its own counters
+        x.task_head = b.task_head + (dense ? kClasses * 2 : 0);
+        x.task_head2 = b.task_head2 + (dense ? kClasses * 2 : 0);
+        const int blocks = dense ? 7 : minb;
+        e = batch_launch(P.prec, P.cls_id[c], &x, phase, per_sm * blocks, P.block, blocks, st);
+    }
+    return e;
+}
 
 int plan_enqueue(BatchPlan& P, cudaStream_t st)
 {
     cudaError_t e;
-    if ((e = cudaMemsetAsync(P.d_scratch, 0, (64 + 2 * kClasses) * sizeof(int), st)) != cudaSuccess) return cuda_fail(e);
+    if ((e = cudaMemsetAsync(P.d_scratch, 0, (64 + 4 * kClasses) * sizeof(int), st)) != cudaSuccess) return cuda_fail(e);
     for (int j = 0; j < P.nm && P.sorted; j++)
         if ((e = cudaMemsetAsync(P.hand[j] + kHandCountOffset, 0, sizeof(int), st)) != cudaSuccess) return cuda_fail(e);
     for (int c = 0; c < P.ncls; c++) {
@@ -2197,10 +2289,7 @@ int plan_enqueue(BatchPlan& P, cudaStream_t st)
     if (P.sorted) {
         // first worklist launch per class, the sort of each member's hand-off slots, resume launch
         for (int c = 0; c < P.ncls; c++) {
-            // the grid: the blocks of 128 threads (or twice as many of 64) that the register cap makes resident
-            const int minb = P.dense[c] ? 7 : 4;
-            if ((e = batch_launch(P.prec, P.cls_id[c], &P.b[c], 2, P.nsm * minb * (128 / P.block), P.block, minb, st)) != cudaSuccess)
-                return cuda_fail(e);
+            if ((e = plan_list(P, c, 2, 4, st)) != cudaSuccess) return cuda_fail(e);
         }
         for (int j = 0; j < P.nm; j++) {
             const UwHand* H = reinterpret_cast<const UwHand*>(P.hand[j]);
@@ -2208,11 +2297,8 @@ int plan_enqueue(BatchPlan& P, cudaStream_t st)
             if (n > 0) hand_tile_kernel<<<tiles(n), tile_threads(n), 0, st>>>(H);
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e);
-        for (int c = 0; c < P.ncls; c++) {   // 5 or 7 resident blocks of 128 threads per SM (launch bounds)
-            const int minb = P.dense[c] ? 7 : 5;
-            if ((e = batch_launch(P.prec, P.cls_id[c], &P.b[c], 3, P.nsm * minb * (128 / P.block), P.block, minb, st)) != cudaSuccess)
-                return cuda_fail(e);
-        }
+        for (int c = 0; c < P.ncls; c++)
+            if ((e = plan_list(P, c, 3, 5, st)) != cudaSuccess) return cuda_fail(e);
         return UWSHCU_OK;
     }
     for (int c = 0; c < P.ncls; c++) {
@@ -2265,14 +2351,14 @@ extern "C" int uwshcu_batch_create(int nmembers, const uwshcu_member* members, v
         plan_free(P);
         return cuda_fail(e);
     }
-    if ((e = cudaMalloc(&P->d_scratch, (64 + 2 * kClasses + total + key_ints(total)) * sizeof(int))) != cudaSuccess ||
+    if ((e = cudaMalloc(&P->d_scratch, (64 + 4 * kClasses + total + key_ints(total)) * sizeof(int))) != cudaSuccess ||
         (e = cudaMalloc(&P->d_err, sizeof(unsigned int))) != cudaSuccess ||
         (e = cudaMemset(P->d_err, 0, sizeof(unsigned int))) != cudaSuccess) {
         plan_free(P);
         return cuda_fail(e);
     }
     int cls_slot[kClasses] = {-1, -1, -1, -1};
-    size_t wl_off = 64 + 2 * kClasses;
+    size_t wl_off = 64 + 4 * kClasses;
     unsigned char* keys = reinterpret_cast<unsigned char*>(P->d_scratch + wl_off + total);
     // sorted schedule: a hand-off region per member (a plan without room for them runs two-phase)
     P->sorted = s.schedule == UWSHCU_SCHED_SORTED;
@@ -2324,7 +2410,7 @@ extern "C" int uwshcu_batch_create(int nmembers, const uwshcu_member* members, v
         P->trig_grid[c] = b.block_start[b.nm];
         size_t columns = 0;
         for (int j = 0; j < b.nm; j++) columns += (size_t)b.m[j].iend;
-        P->dense[c] = dense_call(*d, columns) && batch_has_dense(P->prec, P->cls_id[c]);
+        P->limit[c] = short_list(*d, columns, P->prec, ncnst, false);
     }
     *plan = P;
     return UWSHCU_OK;

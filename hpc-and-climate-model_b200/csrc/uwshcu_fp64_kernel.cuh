@@ -616,8 +616,8 @@ __device__ __forceinline__ void uw_column(const UwArgs& A, const double* __restr
     // Code size bounds the worklist passes: with the loops unrolled by the compiler and exp, log and pow
     // inlined at each use their kernels were 833 kB (LIST1) and 631 kB (RESUME), far beyond the
     // instruction caches that 16 warps at different places share, and at full occupancy a warp waited 4.4
-    // to 6.5 cycles per instruction for its next one.  So no loop here is unrolled and the
-    // transcendentals are calls.
+    // to 6.5 cycles per instruction for its next one.  So the loops here are not unrolled (but for the resumed
+    // slopes, by tracer, and the state copies of uw_state.cuh) and the transcendentals are calls.
 #define CONDEN(...) conden_call<FAST>(__VA_ARGS__)
 // qsat_qs(t, p) right after a CONDEN call at that temperature and pressure: its first lookup
 #define UW_QSAT_OF_CONDEN(t, p) rvj

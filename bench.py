@@ -143,6 +143,12 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
+def both_caps(torch, columns):
+    """Whether the FP64 worklist pass over `columns` is launched at both register caps: four kernels more,
+    two of one thread that hand each launch its count and the two launches whose count is 0."""
+    return columns > 4 * 128 * torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+
+
 def shard_seed(rank):
     """Seed of rank `rank`'s columns: every rank generates and computes its own columns (the
     columns are independent, so there is no exchange step and no collective on the data path)."""
@@ -637,7 +643,7 @@ def run_batched(args):
                                "5 tracers, dt=1800 s", "pver": [m[1] for m in BATCH_MEMBERS],
                    "trigger_fraction": trig, "l2": "inputs larger than L2",
                    "launch": ("CUDA graph: per level class one trigger launch, a persistent first "
-                              "worklist launch (4 blocks/SM, 7 for a class of more than 166,707 columns) and a "
+                              "worklist launch (4 blocks/SM, 7 where the class's worklists hold more than that) and a "
                               "persistent resume launch (5 or 7 blocks/SM), 2 ordering kernels per member; autotuned block %d, %d column(s) per lane per "
                               "task" % (tuned[0], tuned[2])
                               if sorted_plan else
@@ -645,7 +651,9 @@ def run_batched(args):
                               "launch; autotuned block %d, register cap %d blocks/SM, %d column(s) "
                               "per lane per task" % tuned),
                    "schedule": args.schedule},
-        "gpu_launches": args.steps * ((3 * nclass + 2 * len(BATCH_MEMBERS)) if sorted_plan else
+        "gpu_launches": args.steps * (sum(3 + 4 * both_caps(torch, sum(m[0] for m in BATCH_MEMBERS if (m[1] + 1 <= 32) == c))
+                                          for c in {m[1] + 1 <= 32 for m in BATCH_MEMBERS}) + 2 * len(BATCH_MEMBERS)
+                                         if sorted_plan else
                                          2 * nclass + len(BATCH_MEMBERS)),
         "status": st,
         "roofline": {"fp64_algorithmic": fp64_alg},
@@ -983,7 +991,8 @@ def main():
         "precision": args.precision,
         "phases": phases,
         # trigger, worklist order, worklist; sorted: first worklist launch, hand-off order, second launch
-        "gpu_launches": args.steps * ((5 if sorted_pass else 3) if two_phase else 1),
+        "gpu_launches": args.steps * ((5 + 4 * (args.precision == "fp64" and both_caps(torch, n)) if sorted_pass else 3)
+                                      if two_phase else 1),
         "status": st,
     }
     if e2e is not None:

@@ -26,9 +26,9 @@
 #define UW_HD static inline
 #define UW_HD_SLOW static
 #endif
-// exp, log, pow and erfc are calls on the device: inlined at each of their ~25 uses they made up 110 kB
-// of the 510 to 620 kB worklist kernels, which wait for their instructions (the step at 1,048,576
-// columns: 150 ms with calls against 158 ms inlined, loops not unrolled in both).
+// exp, log, pow and erfc are calls on the device: inlined at each of their ~25 uses they lengthen the worklist
+// kernels, which wait for their instructions (1,048,576 columns 103.7 ms with calls, 106.8 ms inlined; up to
+// 65,536 columns the same).
 // The adjoint's kernels (UW_MATH_INLINE) run few warps and wait on each one's chain: they keep them inlined.
 #if !defined(__CUDACC__)
 #define UW_HD_CALL static inline

@@ -10,8 +10,10 @@
 
 // The worklist entry of thread tid, -1 for none: 32 per warp, or as few (a power of two) as spread the n
 // entries over at most `spread` warps (0: full warps).  The fewer columns a warp holds, the fewer branches
-// it runs for the others': with one warp per scheduler (592) against full warps, 64 columns take 6.5 and
-// 6.9 ms, 256 columns 6.8 and 7.5, 1,024 columns 7.7 and 8.1.
+// it runs for the others', and the more warps wait for their instructions.  16 / 64 / 256 / 1,024 / 4,096 / 16,384
+// columns, ms, with full warps 6.6 / 7.7 / 8.1 / 8.2 / 8.4 / 9.5, at two warps per multiprocessor 6.0 / 6.5 / 6.9 / 7.9 /
+// 8.4 / 9.6, at one per scheduler (592 in all, as here) 6.0 / 6.5 / 6.9 / 7.7 / 8.7 / 9.5, at four per scheduler 6.0 /
+// 6.5 / 6.9 / 7.7 / 10.4 / 11.9.
 UW_RULE int uw_spread(int n, int spread, int tid)
 {
     int lanes = 32;

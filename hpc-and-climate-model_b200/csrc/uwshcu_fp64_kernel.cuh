@@ -196,8 +196,8 @@ __device__ __forceinline__ int conden_fast(double p, double ex, double thl, doub
 // between 2^-100 and 2^100; a test per divisor finds the others, and the call is then repeated with conden.
 // The kernels spend most of their time in these Newton steps, a chain of dependent FP64 operations with
 // three divisions.  Here a division has no slow path to branch around, and the table position needs no
-// conversion: a 16-column call takes 6.3 instead of 7.2 ms, 4,096 columns 8.6 instead of 9.7 ms, 1,048,576
-// columns (which wait for memory and instructions) 113.6 instead of 116.1 ms.
+// conversion: a 16-column call takes 6.0 ms, with conden in its place 6.8, 4,096 columns 8.7 and 9.7, 65,536
+// columns 11.4 and 12.4, 1,048,576 columns (which wait for memory and instructions) 103.7 and 108.5.
 
 // qsat_qs; ok is cleared where the divisor is out of range.
 __device__ __forceinline__ double qsat_qs_f64(double t, double p, bool& ok, const double* __restrict__ tbl)

@@ -419,10 +419,11 @@ int stream_ctx(DeviceState& d, cudaStream_t st, StreamCtx** out)
 // ---- split worklist pass -----------------------------------------------------------------------
 // The worklist and the hand-off slots are ordered by key in tiles of 8,192: a warp's columns then start
 // their updraft at the same level and climb about as far, and still lie close together in the caller's
-// arrays.  (Ordered over the whole call, the scattered reads and writes of those arrays cost what the
-// order gains: 1,048,576 columns FP64 119.4 ms as without order, MIXED at 259,200 columns 27.7 against 17.4
-// ms; in tiles FP64 119.6 -> 116.2 ms, 262,144 columns 29.5 -> 28.0 ms, MIXED 17.8 -> 16.9 ms.)  The order
-// within a key is that of the atomics: a column's result does not depend on which columns share its warp.
+// arrays.  A tile is one block's work.  Column kernels of 65,536 / 262,144 / 1,048,576 columns in FP64 and of 259,200 in
+// MIXED, ms: without order 11.9 / 24.4 / 105.3 / 17.0, in tiles of 2,048 11.6 / 24.4 / 105.6 / 17.2, of 8,192 11.3 / 23.9 /
+// 103.3 / 16.8, of 32,768 11.2 / 23.4 / 102.1 / 16.6; as one tile 11.4 / 22.1 / 101.7 / 15.7, of which its one block gives
+// 0.1 / 0.5 / 1.6 / 0.5 back.  The order within a key is that of the atomics: a column's result does not depend
+// on which columns share its warp.
 constexpr int kTile = 8192, kTileThreads = 1024;
 unsigned tiles(size_t n) { return (unsigned)((n + kTile - 1) / kTile); }
 unsigned tile_threads(size_t n) { return n >= (size_t)kTileThreads ? kTileThreads : (unsigned)((n + 31) / 32 * 32); }

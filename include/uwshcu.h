@@ -43,14 +43,17 @@ extern "C" {
 #define UWSHCU_PREC_FP64 0               /* FP64 throughout, Fortran evaluation order, no FMA      */
 #define UWSHCU_PREC_MIXED 1              /* FP32 bulk, FP64 conden/roots/qsinvert/implicit CIN/
                                             positive_moisture, Kahan vertical sums (ncnst <= 5).
-                                            1.7x the FP64 path; column heating/moistening/precip
+                                            1.48x the FP64 path; column heating/moistening/precip
                                             ~0.9 % relative RMS (cloud tops of ~0.6 % of the
                                             convecting columns move)                            */
 #define UWSHCU_PREC_FAST 2               /* FP64 throughout with a Newton conden that stops each
                                             lane after its first step below 1e-10 T and divides
                                             twice per step; FMA contraction allowed.  Not
-                                            bit-exact (~1e-12 relative per conden call); about
-                                            the FP64 path's speed                              */
+                                            bit-exact (~1e-12 relative per conden call).  3 to
+                                            11 % less time than FP64 while the convecting columns
+                                            of a call fit four blocks per SM (75,776 on a B200),
+                                            6 to 8 % more above, where FP64 has launches for long
+                                            worklists: FP64 is the better choice there        */
 
 /* ---- set-up -------------------------------------------------------------------------------- */
 

@@ -144,8 +144,8 @@ class ClockSampler:
 
 
 def both_caps(torch, columns):
-    """Whether the FP64 worklist pass over `columns` is launched at both register caps: four kernels more,
-    two of one thread that hand each launch its count and the two launches whose count is 0."""
+    """Whether the FP64 worklist pass over `columns` (a plan's class: twice as many) is launched at both register
+    caps: four kernels more, two of one thread that hand each launch its count and the two launches whose count is 0."""
     return columns > 4 * 128 * torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
 
 
@@ -651,7 +651,7 @@ def run_batched(args):
                               "launch; autotuned block %d, register cap %d blocks/SM, %d column(s) "
                               "per lane per task" % tuned),
                    "schedule": args.schedule},
-        "gpu_launches": args.steps * (sum(3 + 4 * both_caps(torch, sum(m[0] for m in BATCH_MEMBERS if (m[1] + 1 <= 32) == c))
+        "gpu_launches": args.steps * (sum(3 + 4 * both_caps(torch, sum(m[0] for m in BATCH_MEMBERS if (m[1] + 1 <= 32) == c) // 2)
                                           for c in {m[1] + 1 <= 32 for m in BATCH_MEMBERS}) + 2 * len(BATCH_MEMBERS)
                                          if sorted_plan else
                                          2 * nclass + len(BATCH_MEMBERS)),
